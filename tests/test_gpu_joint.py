@@ -101,3 +101,36 @@ def test_joint3_on_simulated_three_population_state():
     np.testing.assert_allclose(J3.sum(axis=1), J02, rtol=1e-5, atol=1e-3)
     assert abs(J3.sum() - L) <= 1e-5 * L
     assert J3[1:, 1:, 1:].sum() > 0     # variants shared by all three populations
+
+
+def _structured_rows(rng, M, Nc, P):
+    """Shared, private (lost in the other populations) and fixed mutations, in no order."""
+    j = np.exp(rng.uniform(0, np.log(Nc), (P, M))).astype(np.int64)
+    j[:, rng.random(M) < 0.05] = Nc
+    owner = rng.integers(0, P, M)
+    private = rng.random(M) < 0.5
+    for p in range(P):
+        j[p, private & (owner != p)] = 0
+    return [(r / Nc).astype(np.float32) for r in np.minimum(j, Nc)]
+
+
+# fragment (8), warp (32), block-tile (128) edges of the plane; chunk (16) and sort (512) edges of M
+@pytest.mark.parametrize("M,na,nb", [(15, 7, 8), (16, 8, 7), (17, 31, 32), (511, 32, 31), (513, 127, 128),
+                                     (1500, 128, 127), (2049, 129, 300), (700, 1023, 5), (700, 5, 1023)])
+def test_joint_fragment_edges(M, na, nb):
+    rng = np.random.default_rng(7 * M + na)
+    fa, fb = _structured_rows(rng, M, 1000, 2)
+    with Engine() as e:
+        got = e.joint_site_frequency_spectrum(fa, fb, na, nb, 1e6).astype(np.float64)
+    # fp32 output of double sums (relative 6e-8; subnormal floats flush)
+    np.testing.assert_allclose(got, joint_sfs(fa, fb, na, nb, 1e6), rtol=2e-7, atol=1.2e-38)
+
+
+@pytest.mark.parametrize("M,na,nb,nc", [(513, 20, 16, 12), (100, 7, 7, 7), (300, 1, 1, 255), (300, 1, 2, 256),
+                                        (300, 2, 1, 300), (65, 40, 3, 130), (33, 130, 5, 40), (40, 2, 200, 1)])
+def test_joint3_fragment_edges(M, na, nb, nc):
+    rng = np.random.default_rng(7 * M + nc)
+    rows = _structured_rows(rng, M, 1000, 3)
+    with Engine() as e:
+        got = e.joint3_site_frequency_spectrum(*rows, na, nb, nc, 1e6).astype(np.float64)
+    np.testing.assert_allclose(got, joint3_sfs(*rows, na, nb, nc, 1e6), rtol=2e-7, atol=1.2e-38)
