@@ -26,6 +26,7 @@
 #include "gf_internal.h"
 #include "gf_mse.cuh"
 #include "gf_plan.h"
+#include "gf_project.h"
 
 #ifdef GF_TRACE
 #include <chrono>
@@ -52,6 +53,7 @@ static double gf_trace_elapsed_ms() {
 namespace gf {
 
 constexpr int kBatchTile = 1024;
+constexpr int kBatchMaxSample = 1023;   // batched spectra
 
 static long long align_tiles(long long v) { return (v + kBatchTile - 1) / kBatchTile * kBatchTile; }
 
@@ -197,90 +199,6 @@ __global__ void batch_mse_fill_kernel(float* __restrict__ freq, int* __restrict_
     freq[f.base + k] = (a + 1.f) / f.Nc0;
     id_gp[f.base + k] = 0;
     id_tid[f.base + k] = k + 1;
-  }
-}
-
-// ------------------------------------------------------------------------------------------------
-// batched SFS: one block per replicate, direct projection of its frequencies in double
-// ------------------------------------------------------------------------------------------------
-struct SfsRep {
-  long long base;
-  int M;
-  float L;
-};
-
-constexpr int kBatchSfsThreads = 128;
-
-__global__ void __launch_bounds__(kBatchSfsThreads)
-    batch_sfs_kernel(const float* __restrict__ freq, const SfsRep* __restrict__ reps, int n,
-                     const double* __restrict__ lgc, float* __restrict__ out) {
-  const SfsRep R = reps[blockIdx.x];
-  __shared__ double s_lp[kBatchSfsThreads];
-  __shared__ double s_lq[kBatchSfsThreads];
-  __shared__ unsigned s_seg[kBatchSfsThreads];
-  __shared__ double s_acc0[kBatchSfsThreads];
-  const int levels = n + 1;
-  double acc[8];
-#pragma unroll
-  for (int u = 0; u < 8; ++u) acc[u] = 0.0;
-  unsigned nonseg = 0;
-  for (int c0 = 0; c0 < R.M; c0 += kBatchSfsThreads) {
-    const int i = c0 + threadIdx.x;
-    double lp = 0.0, lq = 0.0;
-    unsigned seg = 0;
-    if (i < R.M) {
-      const float p = freq[R.base + i];
-      if (p > 0.f && p < 1.f) {
-        seg = 1;
-        lp = log(static_cast<double>(p));
-        lq = log1p(-static_cast<double>(p));
-      } else {
-        ++nonseg;
-      }
-    }
-    s_lp[threadIdx.x] = lp;
-    s_lq[threadIdx.x] = lq;
-    s_seg[threadIdx.x] = seg;
-    __syncthreads();
-    const int cend = min(kBatchSfsThreads, R.M - c0);
-    for (int t = 0; t < cend; ++t) {
-      if (!s_seg[t]) continue;
-#pragma unroll
-      for (int u = 0; u < 8; ++u) {
-        const int k = threadIdx.x + u * kBatchSfsThreads;
-        if (k < levels) acc[u] += exp(lgc[k] + k * s_lp[t] + (n - k) * s_lq[t]);
-      }
-    }
-    __syncthreads();
-  }
-  // non-segregating count of the block
-  s_acc0[threadIdx.x] = static_cast<double>(nonseg);
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    double ns = 0;
-    for (int t = 0; t < kBatchSfsThreads; ++t) ns += s_acc0[t];
-    s_acc0[0] = ns;
-  }
-  __syncthreads();
-  const double ns = s_acc0[0];
-  __syncthreads();
-  // bin n folds into bin 0: park it in shared memory
-  double top = 0.0;
-#pragma unroll
-  for (int u = 0; u < 8; ++u) {
-    const int k = threadIdx.x + u * kBatchSfsThreads;
-    if (k == n) top = acc[u];
-  }
-  if (threadIdx.x == n % kBatchSfsThreads) s_acc0[1] = top;
-  __syncthreads();
-#pragma unroll
-  for (int u = 0; u < 8; ++u) {
-    const int k = threadIdx.x + u * kBatchSfsThreads;
-    if (k < n) {
-      double v = acc[u];
-      if (k == 0) v += s_acc0[1] + ns + static_cast<double>(R.L - R.M);
-      out[static_cast<long long>(blockIdx.x) * n + k] = static_cast<float>(v);
-    }
   }
 }
 
@@ -1242,7 +1160,7 @@ gf_status gf_batch_sfs(gf_engine* g, int32_t n, float* out) {
     Engine* e = &g->impl;
     Batch* b = e->batch;
     if (!b) return fail(e, GF_ERR_STATE, "no batch");
-    if (n < 1 || n + 1 > 8 * kBatchSfsThreads) return fail(e, GF_ERR_CAPACITY, "sample size %d outside [1, %d)", n, 8 * kBatchSfsThreads);
+    if (n < 1 || n > kBatchMaxSample) return fail(e, GF_ERR_CAPACITY, "sample size %d outside [1, %d)", n, kBatchMaxSample + 1);
     for (int r = 0; r < b->R; ++r) {
       const int Nc = rep_nchrom(b->reps[r].p, b->reps[r].generation);   // Nchrom_e at its current generation
       if (n >= Nc) return fail(e, GF_ERR_INVALID_ARGUMENT, "replicate %d: sample size %d >= Nchrom_e %d", r, n, Nc);
@@ -1252,29 +1170,55 @@ gf_status gf_batch_sfs(gf_engine* g, int32_t n, float* out) {
       gf_status st = sync_counts(e);
       if (st != GF_OK) return st;
     }
-    std::vector<SfsRep> sr(b->R);
-    for (int r = 0; r < b->R; ++r) sr[r] = {b->reps[r].base, b->reps[r].M, b->reps[r].p.num_sites};
-    std::vector<double> lgc(n + 1);
-    const double ln = std::lgamma(n + 1.0);
-    for (int k = 0; k <= n; ++k) lgc[k] = ln - std::lgamma(k + 1.0) - std::lgamma(n - k + 1.0);
-    SfsRep* d_sr = nullptr;
-    double* d_lgc = nullptr;
-    float* d_out = nullptr;
-    {
-      gf_status ast = pool_alloc(e, reinterpret_cast<void**>(&d_sr), sizeof(SfsRep) * b->R);
-      if (ast == GF_OK) ast = pool_alloc(e, reinterpret_cast<void**>(&d_lgc), sizeof(double) * (n + 1));
-      if (ast == GF_OK) ast = pool_alloc(e, reinterpret_cast<void**>(&d_out), sizeof(float) * b->R * n);
-      if (ast != GF_OK) return ast;
+    // every replicate's mutations projected (a row per replicate), its base, count and sites in one upload
+    const int R = b->R;
+    long long most = 0;
+    struct Row {
+      std::vector<long long> base;
+      std::vector<int> M;
+      std::vector<float> L;
+    } rows{std::vector<long long>(R), std::vector<int>(R), std::vector<float>(R)};
+    for (int r = 0; r < R; ++r) {
+      rows.base[r] = b->reps[r].base;
+      rows.M[r] = b->reps[r].M;
+      rows.L[r] = b->reps[r].p.num_sites;
+      most = std::max<long long>(most, rows.M[r]);
     }
-    GF_CUDA(e, cudaMemcpyAsync(d_sr, sr.data(), sizeof(SfsRep) * b->R, cudaMemcpyHostToDevice, e->stream));
-    GF_CUDA(e, cudaMemcpyAsync(d_lgc, lgc.data(), sizeof(double) * (n + 1), cudaMemcpyHostToDevice, e->stream));
-    batch_sfs_kernel<<<b->R, kBatchSfsThreads, 0, e->stream>>>(b->freq[0], d_sr, n, d_lgc, d_out);
-    GF_CUDA(e, cudaGetLastError());
-    e->kernel_launches += 1;
-    GF_CUDA(e, cudaMemcpyAsync(out, d_out, sizeof(float) * b->R * n, cudaMemcpyDeviceToHost, e->stream));
-    cudaFreeAsync(d_sr, e->stream);
-    cudaFreeAsync(d_lgc, e->stream);
-    cudaFreeAsync(d_out, e->stream);
+    const int parts = project_parts(n, most, R, e->num_sms);
+    char* d_rows = nullptr;
+    double* d_scratch = nullptr;
+    float* d_out = nullptr;
+    gf_status ast = pool_alloc(e, reinterpret_cast<void**>(&d_rows), 16 * static_cast<size_t>(R));
+    if (ast == GF_OK) ast = pool_alloc(e, reinterpret_cast<void**>(&d_scratch), sizeof(double) * project_scratch(n, parts, R));
+    if (ast == GF_OK) ast = pool_alloc(e, reinterpret_cast<void**>(&d_out), sizeof(float) * static_cast<size_t>(R) * n);
+    cudaError_t err = cudaSuccess;
+    if (ast == GF_OK) {
+      long long* d_base = reinterpret_cast<long long*>(d_rows);
+      int* d_M = reinterpret_cast<int*>(d_base + R);
+      float* d_L = reinterpret_cast<float*>(d_M + R);
+      err = cudaMemcpyAsync(d_base, rows.base.data(), sizeof(long long) * R, cudaMemcpyHostToDevice, e->stream);
+      if (err == cudaSuccess) err = cudaMemcpyAsync(d_M, rows.M.data(), sizeof(int) * R, cudaMemcpyHostToDevice, e->stream);
+      if (err == cudaSuccess) err = cudaMemcpyAsync(d_L, rows.L.data(), sizeof(float) * R, cudaMemcpyHostToDevice, e->stream);
+      ProjSource src;
+      src.freq = b->freq[0];
+      src.rep_base = d_base;
+      src.rep_M = d_M;
+      // gridDim.y is limited to 65,535: more replicates in several launches
+      for (int r0 = 0; r0 < R && err == cudaSuccess; r0 += 65535) {
+        const int rn = std::min(R - r0, 65535);
+        err = project_rows(src, n, rn, parts, 0.0, d_L + r0, d_scratch + project_scratch(n, parts, r0),
+                           d_out + static_cast<size_t>(r0) * n, e->stream);
+        src.rep_base += rn;
+        src.rep_M += rn;
+        e->kernel_launches += 2;
+      }
+      if (err == cudaSuccess)
+        err = cudaMemcpyAsync(out, d_out, sizeof(float) * static_cast<size_t>(R) * n, cudaMemcpyDeviceToHost, e->stream);
+    }
+    for (void* q : {static_cast<void*>(d_rows), static_cast<void*>(d_scratch), static_cast<void*>(d_out)})
+      if (q) cudaFreeAsync(q, e->stream);
+    if (ast != GF_OK) return ast;
+    if (err != cudaSuccess) return cuda_fail(e, err, "batched SFS");
     GF_CUDA(e, cudaStreamSynchronize(e->stream));
     return GF_OK;
   });

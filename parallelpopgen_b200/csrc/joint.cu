@@ -57,35 +57,6 @@ struct JointTable {
   int n;
 };
 
-// x = m 2^e with m in (1/2, 1] (x > 0 and normal).
-__device__ __forceinline__ double split_exponent(double x, int& e) {
-  const int hi = __double2hiint(x);
-  double m = __hiloint2double((hi & 0x000FFFFF) | 0x3FE00000, __double2loint(x));   // [1/2, 1)
-  e = (hi >> 20) - 1022;
-  if (m == 0.5) {
-    m = 1.0;
-    e -= 1;
-  }
-  return m;
-}
-
-// C(n, k) p^k q^(n-k) by repeated squaring of the mantissas, the exponents apart: m_p^k m_q^(n-k) >= 2^-1023 and
-// C <= 2^1020 for n <= 1023 stay in range.  About n * 1e-16 relative error, as k log p + (n - k) log q has, in
-// a third of the dependent operations of two logarithms and an exp.
-__device__ __forceinline__ double binomial_pmf(double c, int k, int n, double p, double q) {
-  int ep, eq;
-  double bp = split_exponent(p, ep), bq = split_exponent(q, eq);
-  const int kq = n - k;
-  double vp = 1.0, vq = 1.0;
-  for (int bit = 1; bit <= n; bit <<= 1) {   // uniform
-    vp = (k & bit) ? vp * bp : vp;
-    vq = (kq & bit) ? vq * bq : vq;
-    bp *= bp;
-    bq *= bq;
-  }
-  return ldexp(c * vp * vq, ep * k + eq * kq);
-}
-
 // One mutation's values for the runs r0 .. r0 + runs - 1 of population t: start(r) gets pmf(8r), pow[u] the
 // power (p / q)^u.  The run nearest the mode is computed, the others follow from it run by run, up and down,
 // by C(n, 8r +- 8) / C(n, 8r) * (p / q)^+-8: away from the mode the pmf only falls, so what underflows is below
