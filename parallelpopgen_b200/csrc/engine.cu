@@ -502,7 +502,8 @@ static void release_sim(Engine* e) {
   e->flags = nullptr;
   e->tile_count = nullptr;
   e->tile_offset = nullptr;
-  for (auto& pc : e->pending) e->free_events.push_back(pc.event);
+  for (auto& pc : e->pending)
+    if (pc.event) e->free_events.push_back(pc.event);
   e->pending.clear();
   e->capacity = 0;
   e->active = false;
@@ -612,6 +613,7 @@ static gf_status begin_common(Engine* e, const gf_sim_config* c, long long initi
   GF_CUDA(e, cudaMemsetAsync(e->d_stats, 0, sizeof(unsigned long long) * 2, e->stream));
   e->compactions = 0;
   e->M_upper = initial_mutations;
+  e->M_recent = initial_mutations;
   e->M_exact = true;
   e->active = true;
   return GF_OK;
@@ -621,18 +623,34 @@ static gf_status begin_common(Engine* e, const gf_sim_config* c, long long initi
 static void poll_pending(Engine* e, bool wait_all) {
   while (!e->pending.empty()) {
     PendingCount& pc = e->pending.front();
-    if (wait_all) {
-      cudaEventSynchronize(pc.event);
-    } else if (cudaEventQuery(pc.event) != cudaSuccess) {
-      cudaGetLastError();
-      break;
+    long long count;
+    if (pc.event) {
+      if (wait_all) {
+        cudaEventSynchronize(pc.event);
+      } else if (cudaEventQuery(pc.event) != cudaSuccess) {
+        cudaGetLastError();
+        break;
+      }
+      count = e->h_pinned[pc.slot];
+      e->free_events.push_back(pc.event);
+    } else {
+      const volatile unsigned long long* mail = e->h_mail + pc.slot;
+      unsigned long long v = *mail;
+      if (static_cast<unsigned>(v >> 32) != pc.tag) {
+        if (!wait_all) break;
+        cudaStreamSynchronize(e->stream);
+        v = *mail;
+      }
+      // after a failed stream the mail may not have come: the bound stays as it is
+      count = static_cast<unsigned>(v >> 32) == pc.tag ? static_cast<long long>(v & 0xFFFFFFFFu) : e->M_upper;
     }
-    const long long exact = e->h_pinned[pc.slot] + pc.added;
-    if (e->pending.size() == 1 && exact <= e->M_upper) {
-      e->M_upper = exact;
-      e->M_exact = true;
+    // a bound whatever came after (later compactions only lower the count), exact if nothing did
+    const long long bound = count + pc.added;
+    e->M_recent = count;
+    if (bound <= e->M_upper) {
+      e->M_upper = bound;
+      if (e->pending.size() == 1) e->M_exact = true;
     }
-    e->free_events.push_back(pc.event);
     e->pending.pop_front();
   }
 }
@@ -948,7 +966,8 @@ static int drift_bits(const gf_generation& g, int P) { return drifted_population
 
 // Run generations [first, first + count) of the batch as one window launch.
 static gf_status launch_window(Engine* e, int b, int first, int count, const GenHost* gh) {
-  WinRep& R = e->h_wrep[b][first];
+  WindowLaunch w;
+  WinRep& R = w.one;
   long long news = 0;
   for (int k = 0; k < count; ++k) news += e->h_wgen[b][first + k].new_count;
   long long need = 0;
@@ -968,9 +987,7 @@ static gf_status launch_window(Engine* e, int b, int first, int count, const Gen
   R.preserve = (last.flag && gh[first + count - 1].preserve) ? 1 : 0;
   R.rep = 0;
   R.births = news;
-  GF_CUDA(e, cudaMemcpyAsync(e->d_wrep[b] + first, &R, sizeof(WinRep), cudaMemcpyHostToDevice, e->stream));
   const int slot = e->count_slot;
-  WindowLaunch w;
   w.A = e->freq[e->cur];
   w.B = e->freq[e->cur ^ 1];
   w.id_gp_cur = e->id_gp[e->id_cur];
@@ -984,17 +1001,26 @@ static gf_status launch_window(Engine* e, int b, int first, int count, const Gen
   w.M_end = e->d_count + 3;
   w.M_next = e->d_count + (slot ^ 1);
   w.M_out = e->d_count + (slot ^ 1);
-  w.reps = e->d_wrep[b] + first;
+  w.reps = nullptr;
   w.nreps = 1;
   w.recs = e->d_wgen[b];
   w.total_tiles = R.ntiles;
+  w.expected_slots = std::min(need, e->M_recent + news);
   w.any_compact = R.compact != 0;
   w.stats = e->d_stats;
   w.fault = e->d_count + 2;
   w.sched = e->d_count + kSchedWord;
-  w.uniform_key = true;
-  w.seed1 = e->seed1;
-  w.seed2 = e->seed2;
+  PendingCount pc;
+  if (w.any_compact) {
+    poll_pending(e, false);
+    if (static_cast<int>(e->pending.size()) >= e->pinned_slots - 1) poll_pending(e, true);
+    pc.slot = e->next_slot;
+    e->next_slot = (e->next_slot + 1) % e->pinned_slots;
+    pc.tag = ++e->mail_tag;
+    if (pc.tag == 0) pc.tag = ++e->mail_tag;   // fresh slots hold tag 0
+    w.mail = e->h_mail + pc.slot;
+    w.mail_tag = pc.tag;
+  }
   // profiling: the window kernel's time counts as drift, its segmented scan and scatter as compaction
   cudaEvent_t ev0 = nullptr, evw = nullptr, evc = nullptr, ev1 = nullptr;
   if (e->profiling) {
@@ -1017,15 +1043,15 @@ static gf_status launch_window(Engine* e, int b, int first, int count, const Gen
     }
   }
   e->M_upper = need;
-  for (auto& pc : e->pending) pc.added += news;
+  for (auto& earlier : e->pending) earlier.added += news;
   e->count_slot ^= 1;
   e->step_index += count;
   if (R.compact) {
     if (R.preserve) e->any_preserved = true;
     e->id_cur ^= 1;
     e->compactions += 1;
-    st = push_readback(e, e->count_slot);
-    if (st != GF_OK) return st;
+    e->pending.push_back(pc);
+    e->M_exact = false;
   } else {
     e->cur ^= 1;
   }
@@ -1120,17 +1146,11 @@ static gf_status run_batch(Engine* e, const gf_generation* gens, int n) {
     const size_t cap = std::max<size_t>(n, 256);
     if (e->d_wgen[b]) GF_CUDA(e, cudaFree(e->d_wgen[b]));
     if (e->h_wgen[b]) GF_CUDA(e, cudaFreeHost(e->h_wgen[b]));
-    if (e->d_wrep[b]) GF_CUDA(e, cudaFree(e->d_wrep[b]));
-    if (e->h_wrep[b]) GF_CUDA(e, cudaFreeHost(e->h_wrep[b]));
     e->d_wgen[b] = nullptr;
     e->h_wgen[b] = nullptr;
-    e->d_wrep[b] = nullptr;
-    e->h_wrep[b] = nullptr;
     e->wtable_cap[b] = 0;
     GF_CUDA(e, cudaMalloc(&e->d_wgen[b], sizeof(WinGen) * cap));
     GF_CUDA(e, cudaMallocHost(&e->h_wgen[b], sizeof(WinGen) * cap));
-    GF_CUDA(e, cudaMalloc(&e->d_wrep[b], sizeof(WinRep) * cap));
-    GF_CUDA(e, cudaMallocHost(&e->h_wrep[b], sizeof(WinRep) * cap));
     e->wtable_cap[b] = cap;
   }
   std::vector<GenHost> gh(n);
@@ -1196,6 +1216,7 @@ static gf_status current_count(Engine* e, int* M) {
   if (st != GF_OK) return st;
   poll_pending(e, true);
   e->M_upper = *M;
+  e->M_recent = *M;
   e->M_exact = true;
   return GF_OK;
 }
@@ -1258,12 +1279,15 @@ gf_status gf_engine_create(int device, void* cuda_stream, gf_engine** out) {
   }
   if (cudaMalloc(&e->d_count, sizeof(int) * kCountWords) != cudaSuccess ||
       cudaMalloc(&e->d_stats, sizeof(unsigned long long) * 2) != cudaSuccess ||
-      cudaMallocHost(&e->h_pinned, sizeof(int) * e->pinned_slots) != cudaSuccess) {
+      cudaMallocHost(&e->h_pinned, (sizeof(unsigned long long) + sizeof(int)) * e->pinned_slots) != cudaSuccess) {
     if (e->d_count) cudaFree(e->d_count);
     if (e->own_stream) cudaStreamDestroy(e->stream);
     delete g;
     return GF_ERR_OUT_OF_MEMORY;
   }
+  e->h_mail = reinterpret_cast<unsigned long long*>(e->h_pinned);   // the 64-bit slots first
+  e->h_pinned = reinterpret_cast<int*>(e->h_mail + e->pinned_slots);
+  std::memset(e->h_mail, 0, sizeof(unsigned long long) * e->pinned_slots);
   cudaMemsetAsync(e->d_count, 0, sizeof(int) * kCountWords, e->stream);
   cudaMemsetAsync(e->d_stats, 0, sizeof(unsigned long long) * 2, e->stream);
   {
@@ -1321,13 +1345,11 @@ void gf_engine_destroy(gf_engine* g) {
     if (e->table_done[b]) cudaEventDestroy(e->table_done[b]);
     if (e->d_wgen[b]) cudaFree(e->d_wgen[b]);
     if (e->h_wgen[b]) cudaFreeHost(e->h_wgen[b]);
-    if (e->d_wrep[b]) cudaFree(e->d_wrep[b]);
-    if (e->h_wrep[b]) cudaFreeHost(e->h_wrep[b]);
   }
   for (auto& pr : e->prof_drift) e->prof_pool.insert(e->prof_pool.end(), {pr.first, pr.second});
   for (auto& pr : e->prof_compact) e->prof_pool.insert(e->prof_pool.end(), {pr.first, pr.second});
   for (auto ev : e->prof_pool) cudaEventDestroy(ev);
-  if (e->h_pinned) cudaFreeHost(e->h_pinned);
+  if (e->h_mail) cudaFreeHost(e->h_mail);
   if (e->own_stream) cudaStreamDestroy(e->stream);
   delete g;
 }

@@ -22,10 +22,6 @@
 #ifndef GF_WINDOW_MIN_BLOCKS_KEYS
 #define GF_WINDOW_MIN_BLOCKS_KEYS 5
 #endif
-// 1: a single-replicate window launch takes its Philox round keys from the kernel parameters.
-#ifndef GF_WINDOW_UNIFORM_KEYS
-#define GF_WINDOW_UNIFORM_KEYS 1
-#endif
 // 1: the lane-order draw schedule walks a quad's lanes in a rolled loop (one inlined copy of the
 // sampler instead of four); 0: the loop is unrolled.
 #ifndef GF_LANES_ROLLED

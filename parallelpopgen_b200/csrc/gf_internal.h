@@ -118,10 +118,13 @@ struct WindowLaunch {
   int* fault;
   int* sched = nullptr;    // two zeroed device words: next tile to hand out, blocks finished (the
                            // launch's last block sets both back to zero)
-  // one replicate (the plain engine): its seeds, from which the launch passes the Philox round keys
-  // as kernel parameters
-  bool uniform_key = false;
-  int seed1 = 0, seed2 = 0;
+  // one replicate (the plain engine, nreps == 1 and reps null): its window by value and its Philox round
+  // keys from its seeds, as kernel parameters
+  WinRep one{};
+  long long expected_slots = 0;   // about how many slots it ends with (which kernels run it, not what they do)
+  // where the compaction also stores the survivor count (tagged), in page-locked host memory; null: nowhere
+  unsigned long long* mail = nullptr;
+  unsigned mail_tag = 0;
   RepList list{};
 };
 
@@ -260,10 +263,13 @@ struct Batch {
   long long steps_enqueued = 0, slabs_enqueued = 0;
 };
 
+// A compaction's survivor count on its way to the host: copied behind an event into h_pinned[slot], or
+// (event null) stored by the compaction itself into h_mail[slot] with the tag above it.
 struct PendingCount {
-  cudaEvent_t event;
-  int slot;           // index into the pinned readback array
-  long long added;    // new mutations appended after this compaction
+  cudaEvent_t event = nullptr;
+  int slot = 0;
+  long long added = 0;   // new mutations appended after this compaction
+  unsigned tag = 0;
 };
 
 struct Engine {
@@ -304,11 +310,15 @@ struct Engine {
                                             // [3]: slots at the end of a launch; [4],[5]: window tile
                                             // scheduler (kSchedWord); kCountWords words in all
   int* h_pinned = nullptr;                  // pinned readback slots
+  unsigned long long* h_mail = nullptr;     // the same, written by the device: tag << 32 | count
+  unsigned mail_tag = 0;
   int pinned_slots = 64;
   int next_slot = 0;
 
   // host tracking of the mutation count
   long long M_upper = 0;   // upper bound on the current count (exact when nothing is pending)
+  long long M_recent = 0;  // the last count read back: what a window's size is expected from (the bound
+                           // grows by the births of every window enqueued ahead of the read-backs)
   bool M_exact = true;
   // an asynchronous time sample (gf_sim_sample_begin / _wait): the state packed into device scratch on
   // the engine's stream, copied to the caller's arrays on a second stream
@@ -337,8 +347,6 @@ struct Engine {
   // window records of the single-population path (same double-buffering as the tables above)
   WinGen* d_wgen[2] = {nullptr, nullptr};
   WinGen* h_wgen[2] = {nullptr, nullptr};
-  WinRep* d_wrep[2] = {nullptr, nullptr};
-  WinRep* h_wrep[2] = {nullptr, nullptr};
   size_t wtable_cap[2] = {0, 0};
   bool use_windows = true;   // single-population runs use the window kernel
   // per-slot selection table of generations whose selection model is evaluated by the caller on the

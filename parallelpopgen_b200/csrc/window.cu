@@ -233,9 +233,9 @@ __global__ void __launch_bounds__(1024) batch_step_kernel(WinRep* __restrict__ r
   }
 }
 
-// DRAW: how a warp schedules its sampler draws (DrawStrategy).  KEYS: every replicate of the launch
-// has the seeds whose round keys `keys` holds (a plain-engine launch), so the quads' Philox blocks take
-// their round keys from the kernel parameters instead of deriving them from the replicate's seeds.
+// DRAW: how a warp schedules its sampler draws (DrawStrategy).  KEYS: a launch of one replicate (the plain
+// engine), whose window `one` and Philox round keys `keys` are kernel parameters: no table to read or
+// search, and a round's key costs no instruction.
 template <int DRAW, bool KEYS>
 __global__ void __launch_bounds__(kWinThreads, KEYS ? GF_WINDOW_MIN_BLOCKS_KEYS : GF_WINDOW_MIN_BLOCKS)
     window_kernel(const float* __restrict__ A, float* __restrict__ B, int* __restrict__ id_gp,
@@ -243,17 +243,18 @@ __global__ void __launch_bounds__(kWinThreads, KEYS ? GF_WINDOW_MIN_BLOCKS_KEYS 
                   const int* __restrict__ M_in, int* __restrict__ M_end, int* __restrict__ M_next,
                   const WinRep* __restrict__ reps, int nreps, const WinGen* __restrict__ recs, int total_tiles,
                   const int* __restrict__ total_dev, unsigned long long* __restrict__ stats,
-                  int* __restrict__ fault, const PhiloxKeys keys, int* __restrict__ sched, const RepList list) {
+                  int* __restrict__ fault, const PhiloxKeys keys, int* __restrict__ sched, const RepList list,
+                  const WinRep one) {
   __shared__ int s_rep;
   __shared__ int s_tile;
   __shared__ unsigned s_warp[kWinThreads / 32];
-  __shared__ int s_tile0[kRepCache];
+  __shared__ int s_tile0[KEYS ? 1 : kRepCache];
   __shared__ WarpDraws s_draws[(DRAW == kDrawWarp || DRAW == kDrawPooledSearch) ? kWinThreads / 32 : 1];
   const int lane = threadIdx.x & 31;
   WarpDraws* wd = &s_draws[(DRAW == kDrawWarp || DRAW == kDrawPooledSearch) ? (threadIdx.x >> 5) : 0];
   const int ntiles_all = total_dev ? *total_dev : total_tiles;
-  const int nlist = list_count(list, nreps);
-  load_tile0(s_tile0, list, reps, nlist);
+  const int nlist = KEYS ? 1 : list_count(list, nreps);
+  if (!KEYS) load_tile0(s_tile0, list, reps, nlist);
   // Tiles are handed out in order by an atomic counter, so a block that drew cheap tiles (slots born
   // late in the window) takes more of them: the launch does not wait on the blocks that a fixed
   // assignment would have given the most expensive tiles.
@@ -261,12 +262,12 @@ __global__ void __launch_bounds__(kWinThreads, KEYS ? GF_WINDOW_MIN_BLOCKS_KEYS 
     if (threadIdx.x == 0) {
       const int t = atomicAdd(sched, 1);
       s_tile = t;
-      if (t < ntiles_all) s_rep = list_rep(list, find_rep_cached(s_tile0, list, reps, nlist, t));
+      if (!KEYS && t < ntiles_all) s_rep = list_rep(list, find_rep_cached(s_tile0, list, reps, nlist, t));
     }
     __syncthreads();
     const int gt = s_tile;
     if (gt >= ntiles_all) break;   // block-uniform
-    const WinRep R = reps[s_rep];
+    const WinRep R = KEYS ? one : reps[s_rep];
     __syncthreads();
     const int t = gt - R.tile0;
     const int q = t * kWinThreads + threadIdx.x;  // quad within the replicate
@@ -431,16 +432,220 @@ __global__ void __launch_bounds__(kWinThreads, KEYS ? GF_WINDOW_MIN_BLOCKS_KEYS 
   }
 }
 
+// A compaction's survivor count to the host (PendingCount).
+__device__ __forceinline__ void post_count(unsigned long long* mail, unsigned tag, int count) {
+  if (!mail) return;
+  *reinterpret_cast<volatile unsigned long long*>(mail) =
+      static_cast<unsigned long long>(tag) << 32 | static_cast<unsigned>(count);
+  __threadfence_system();
+}
+
+// ------------------------------------------------------------------------------------------------
+// Small windows: a slot per thread
+// ------------------------------------------------------------------------------------------------
+// Between compactions a slot depends on nothing but its own frequency and the generations' records, so a
+// thread can carry one slot through the window with no barrier.  Every slot then evaluates its quad's
+// Philox block alone (four times the work, about 118 thread instructions a draw against 73), but the four
+// draws of a quad are no longer one thread's chain: a generation takes the latency of one draw, not of
+// four with both sampler branches each.  That is what a state of few mutations waits for: 0.7 us a
+// generation against 1.9 at 12,000 slots; see kSlotWindowSlots for where the line lies.
+struct SlotGen {
+  int generation, Nc;
+  int M;            // mutations at the generation's start
+  int new_count;
+  float sel_a, sel_b, F, h;
+};
+
+// Slot e's frequency after the generation (e < G.M): the arithmetic and counters of the window kernel.
+template <bool KEYS>
+__device__ __forceinline__ float slot_generation(float x, int e, const SlotGen& G, const PhiloxKeys& keys, int seed1,
+                                                 int seed2) {
+  const int N = G.Nc, g = G.generation;
+  if (N <= 0) return 0.f;   // extinction generation: the population's row is cleared
+  const bool neutral = G.sel_a == 0.f && G.sel_b == 0.f;
+  const float xs = neutral ? selected_freq<true>(x, 0.f, 0.f, 0.f, 0.f)
+                           : selected_freq<false>(x, G.sel_a, G.sel_b, G.F, G.h);
+  int res = (xs == 1.f && N > 6) ? N : 0;
+  if (e < (G.M & ~3)) {
+    if (!(xs == 0.f || (xs == 1.f && N > 6))) {
+      const int q = e >> 2, j = e & 3;
+      uint4 r;
+      if (KEYS) r = philox4x32_10_keys(make_uint4(static_cast<uint32_t>(q + 2), static_cast<uint32_t>(g), 0u, 0u), keys);
+      else r = philox(seed1, seed2, q + 2, g, 0, 0);
+      const uint32_t bits = j == 0 ? r.x : j == 1 ? r.y : j == 2 ? r.z : r.w;
+      res = GF_LANE_DRAW(bits, xs * N, (1.0f - xs) * (xs * N), static_cast<float>(N));
+    }
+  } else {
+    res = drift_tail(seed1, seed2, e, g, 0, xs, N);   // scalar tail: counter (slot + 2), variance in double
+  }
+  return static_cast<float>(clampi(res, 0, N)) / static_cast<float>(N);
+}
+
+constexpr int kSlotThreads = 128;   // one SM takes several blocks, and a small state spreads over many SMs
+
+// The records of a window in shared memory: s_gen, the frequencies of new mutations, and whether a lost slot
+// stays lost through every generation (its selected frequency is 0; not so if a coefficient is infinite).
+// All threads of the block.
+__device__ __forceinline__ void load_slot_generations(SlotGen* s_gen, float* s_new, int* s_scan, int* s_lost_stays,
+                                                      const WinGen* __restrict__ recs, int ngen, int M0) {
+  const int t = threadIdx.x, lane = t & 31, warp = t >> 5;
+  static_assert(kSlotThreads >= kMaxWindowGenerations, "a thread per record");
+  if (t == 0) *s_lost_stays = 1;
+  __syncthreads();
+  int births = 0;
+  if (t < ngen) {
+    const WinGen G = recs[t];
+    births = G.new_count;
+    s_gen[t] = {G.generation, G.Nc, 0, G.new_count, G.sel_a, G.sel_b, G.F, G.h};
+    s_new[t] = G.new_freq;
+    if (!(G.sel_a == 0.f && G.sel_b == 0.f) && !(selected_freq<false>(0.f, G.sel_a, G.sel_b, G.F, G.h) == 0.f))
+      *s_lost_stays = 0;
+  }
+  int incl = births;
+#pragma unroll
+  for (int o = 1; o < 32; o <<= 1) {
+    const int y = __shfl_up_sync(0xFFFFFFFFu, incl, o);
+    if (lane >= o) incl += y;
+  }
+  if (lane == 31) s_scan[warp] = incl;
+  __syncthreads();
+  int before = M0 + incl - births;
+  for (int w = 0; w < warp; ++w) before += s_scan[w];
+  if (t < ngen) s_gen[t].M = before;
+  __syncthreads();
+}
+
+// One replicate's window, kSlotThreads slots a block; writes the rows, the births' IDs and, before a
+// compaction, the flag words.
+__global__ void __launch_bounds__(kSlotThreads)
+    window_slots_kernel(const float* __restrict__ A, float* __restrict__ B, int* __restrict__ id_gp,
+                        int* __restrict__ id_tid, unsigned* __restrict__ flags, const int* __restrict__ M_in,
+                        int* __restrict__ M_end, int* __restrict__ M_next, const WinGen* __restrict__ recs,
+                        unsigned long long* __restrict__ stats, int* __restrict__ fault, const PhiloxKeys keys,
+                        const WinRep R) {
+  __shared__ SlotGen s_gen[kMaxWindowGenerations];
+  __shared__ float s_new[kMaxWindowGenerations];
+  __shared__ int s_scan[kSlotThreads / 32];
+  __shared__ int s_lost_stays;
+  const int cap = static_cast<int>(R.capacity);
+  const int M0 = M_in[R.rep];
+  const int Mw = static_cast<int>(min(static_cast<long long>(M0) + R.births, R.capacity));
+  const int first = static_cast<int>(blockIdx.x) * kSlotThreads;
+  if (first >= Mw && blockIdx.x > 0) return;   // block 0 keeps the books
+  load_slot_generations(s_gen, s_new, s_scan, &s_lost_stays, recs + R.rec, R.ngen, M0);
+  const bool lost_stays = s_lost_stays != 0;
+  const int alive = recs[R.rec + R.ngen - 1].alive;
+  for (int s0 = first; s0 < Mw; s0 += static_cast<int>(gridDim.x) * kSlotThreads) {
+    const int e = s0 + threadIdx.x;
+    bool keep = false;
+    if (e < Mw) {
+      int k = 0;
+      float x;
+      if (e < M0) {
+        x = A[R.base + e];
+      } else {   // born in the last generation k whose births start at or below e
+        int hi = R.ngen - 1;
+        while (k < hi) {
+          const int mid = (k + hi + 1) >> 1;
+          if (s_gen[mid].M <= e) k = mid;
+          else hi = mid - 1;
+        }
+        x = s_new[k];
+        id_gp[R.base + e] = s_gen[k].generation;
+        id_tid[R.base + e] = e - s_gen[k].M + 1;
+        ++k;
+      }
+#pragma unroll 1
+      for (; k < R.ngen; ++k) {
+        if (lost_stays && __float_as_uint(x) == 0u) break;
+        x = slot_generation<true>(x, e, s_gen[k], keys, R.seed1, R.seed2);
+      }
+      B[R.base + e] = x;
+      keep = alive && !(x <= 0.f || x >= 1.f);
+      if (R.check_preserved && e < M0 && id_tid[R.base + e] < 0) keep = true;
+    }
+    if (R.compact) {
+      const unsigned word = __ballot_sync(0xFFFFFFFFu, keep);
+      if ((threadIdx.x & 31) == 0) flags[(R.base + e) >> 5] = word;
+    }
+  }
+  if (blockIdx.x == 0 && threadIdx.x == 0) {
+    unsigned long long mg = 0;
+    for (int k = 0; k < R.ngen; ++k) mg += static_cast<unsigned long long>(s_gen[k].M);
+    atomicAdd(stats, mg);
+    atomicAdd(stats + 1, static_cast<unsigned long long>(R.ngen));
+    if (static_cast<long long>(M0) + R.births > cap) atomicExch(fault, kFaultCapacity);
+    M_end[R.rep] = Mw;
+    if (M_next && !R.compact) M_next[R.rep] = Mw;
+  }
+}
+
+// The compaction of a small window in one launch: a block counts the survivors before its tile from the
+// flag words themselves (a few hundred words from L2), then scatters its tile as seg_scatter_kernel does.
+__global__ void __launch_bounds__(kWinThreads)
+    compact_slots_kernel(const float* __restrict__ src, float* __restrict__ dst, const int* __restrict__ gp_src,
+                         const int* __restrict__ tid_src, int* __restrict__ gp_dst, int* __restrict__ tid_dst,
+                         const unsigned* __restrict__ flags, const int* __restrict__ M_end, int* __restrict__ M_out,
+                         const WinRep R, unsigned long long* mail, unsigned tag) {
+  __shared__ int s_sum[kWinThreads / 32];
+  const int Mw = M_end[R.rep];
+  const int ntiles = max(1, (Mw + kWinTile - 1) / kWinTile), nwords = (Mw + 31) / 32;
+  const unsigned* const word0 = flags + (R.base >> 5);
+  const int t = threadIdx.x, lane = t & 31, warp = t >> 5;
+  for (int tile = blockIdx.x; tile < ntiles; tile += gridDim.x) {
+    const int w0 = tile * (kWinTile / 32);
+    int sum = 0;
+    for (int w = t; w < w0; w += kWinThreads) sum += __popc(word0[w]);
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) sum += __shfl_xor_sync(0xFFFFFFFFu, sum, o);
+    if (lane == 0) s_sum[warp] = sum;
+    __syncthreads();
+    int before = 0;
+#pragma unroll
+    for (int w = 0; w < kWinThreads / 32; ++w) before += s_sum[w];
+    __syncthreads();
+    // a warp's four words, one after the other: lane l of word w holds slot 32 w + l, and the words of the
+    // tile before them are counted by the warp itself
+    const unsigned mine = w0 + lane < nwords ? word0[w0 + lane] : 0u;
+    int incl = __popc(mine);
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const int y = __shfl_up_sync(0xFFFFFFFFu, incl, o);
+      if (lane >= o) incl += y;
+    }
+#pragma unroll
+    for (int i = 0; i < kWinTile / 32 / (kWinThreads / 32); ++i) {
+      const int w = i * (kWinThreads / 32) + warp;
+      const unsigned word = __shfl_sync(0xFFFFFFFFu, mine, w);
+      const int upto = __shfl_sync(0xFFFFFFFFu, incl, w) - __popc(word);
+      if ((word >> lane) & 1u) {
+        const long long from = R.base + static_cast<long long>(w0 + w) * 32 + lane;
+        const long long to = R.base + before + upto + __popc(word & ((1u << lane) - 1u));
+        const int id = tid_src[from];
+        dst[to] = src[from];
+        gp_dst[to] = gp_src[from];
+        tid_dst[to] = R.preserve ? -abs(id) : id;
+      }
+    }
+    if (tile == ntiles - 1 && t == kWinThreads - 1) {   // lane 31 holds the tile's survivors
+      M_out[R.rep] = before + incl;
+      post_count(mail, tag, before + incl);
+    }
+  }
+}
+
 // One block per replicate: exclusive scan of its tile survivor counts, compacted count.  Each thread
-// takes kSegScanItems consecutive tiles, so one pass covers 8,192 tiles (8.4 M slots).
+// takes kSegScanItems consecutive tiles, so one pass covers 8,192 tiles (8.4 M slots).  SINGLE: one
+// replicate, `one`, whose count also goes to the host.
 constexpr int kSegScanThreads = 1024;
 constexpr int kSegScanItems = 8;
+template <bool SINGLE>
 __global__ void __launch_bounds__(kSegScanThreads)
     seg_scan_kernel(const unsigned* __restrict__ tile_count, unsigned* __restrict__ tile_offset,
                     const WinRep* __restrict__ reps, const int* __restrict__ M_end, int* __restrict__ M_out,
-                    const RepList list) {
-  if (list.count && static_cast<int>(blockIdx.x) >= *list.count) return;
-  const WinRep R = reps[list_rep(list, blockIdx.x)];
+                    const RepList list, const WinRep one, unsigned long long* mail, unsigned tag) {
+  if (!SINGLE && list.count && static_cast<int>(blockIdx.x) >= *list.count) return;
+  const WinRep R = SINGLE ? one : reps[list_rep(list, blockIdx.x)];
   if (!R.compact) return;
   __shared__ unsigned s_warp[kSegScanThreads / 32];
   __shared__ unsigned s_carry;
@@ -487,13 +692,16 @@ __global__ void __launch_bounds__(kSegScanThreads)
     if (threadIdx.x == kSegScanThreads - 1) s_carry = run;
     __syncthreads();
   }
-  if (threadIdx.x == 0) M_out[R.rep] = static_cast<int>(s_carry);
+  if (threadIdx.x == 0) {
+    M_out[R.rep] = static_cast<int>(s_carry);
+    if (SINGLE) post_count(mail, tag, static_cast<int>(s_carry));
+  }
 }
 
 // Stable scatter of every compacting replicate's survivors (scatter_arrays, go_fish_impl.cu:147-189),
 // staged through shared memory into one contiguous run per tile.  FUSED stages the frequency and
 // both ID words of a tile together (one barrier, the three loads in flight at once, 12 KB of staging)
-// -- faster for one large replicate; otherwise the arrays go one after the other through one 4 KB
+// -- faster for one large replicate, passed by value as `one`; otherwise the arrays go one after the other through one 4 KB
 // buffer, which keeps more blocks resident for the many small tiles of a batch.
 template <bool FUSED>
 __global__ void __launch_bounds__(kWinThreads)
@@ -501,21 +709,23 @@ __global__ void __launch_bounds__(kWinThreads)
                        const int* __restrict__ tid_src, int* __restrict__ gp_dst, int* __restrict__ tid_dst,
                        const unsigned* __restrict__ flags, const unsigned* __restrict__ tile_offset,
                        const WinRep* __restrict__ reps, int nreps, const int* __restrict__ M_end, int total_tiles,
-                       const int* __restrict__ total_dev, const RepList list) {
+                       const int* __restrict__ total_dev, const RepList list, const WinRep one) {
   __shared__ int s_rep;
-  __shared__ int s_tile0[kRepCache];
+  __shared__ int s_tile0[FUSED ? 1 : kRepCache];
   const int ntiles_all = total_dev ? *total_dev : total_tiles;
-  const int nlist = list_count(list, nreps);
-  load_tile0(s_tile0, list, reps, nlist);
+  const int nlist = FUSED ? 1 : list_count(list, nreps);
+  if (!FUSED) load_tile0(s_tile0, list, reps, nlist);
   __shared__ unsigned s_words[32];
   __shared__ unsigned s_prefix[32];
   __shared__ float s_stage[FUSED ? 3 * kWinTile : kWinTile];
   const int t = threadIdx.x;
   for (int gt = blockIdx.x; gt < ntiles_all; gt += gridDim.x) {
-    if (t == 0) s_rep = list_rep(list, find_rep_cached(s_tile0, list, reps, nlist, gt));
-    __syncthreads();
-    const WinRep R = reps[s_rep];
-    __syncthreads();
+    if (!FUSED) {
+      if (t == 0) s_rep = list_rep(list, find_rep_cached(s_tile0, list, reps, nlist, gt));
+      __syncthreads();
+    }
+    const WinRep R = FUSED ? one : reps[s_rep];
+    if (!FUSED) __syncthreads();
     const int tile = gt - R.tile0;
     const int ntiles = (M_end[R.rep] + kWinTile - 1) / kWinTile;
     if (!R.compact || tile >= ntiles) continue;  // block-uniform
@@ -631,46 +841,80 @@ static void launch_window_kernel(Engine* e, const WindowLaunch& w) {
   }();
   const int per_sm = e->blocks_per_sm > 0 ? std::min(e->blocks_per_sm, occupancy) : occupancy;
   const int blocks = std::max(1, std::min(w.total_tiles, e->num_sms * per_sm));
-  const PhiloxKeys keys = philox_round_keys(w.seed1, w.seed2);
+  const PhiloxKeys keys = philox_round_keys(w.one.seed1, w.one.seed2);
   window_kernel<DRAW, KEYS><<<blocks, kWinThreads, 0, e->stream>>>(
       w.A, w.B, w.id_gp_cur, w.id_tid_cur, w.flags, w.tile_count, w.M_in, w.M_end, w.M_next, w.reps, w.nreps,
-      w.recs, w.total_tiles, w.total_tiles_dev, w.stats, w.fault, keys, w.sched, w.list);
+      w.recs, w.total_tiles, w.total_tiles_dev, w.stats, w.fault, keys, w.sched, w.list, w.one);
 }
 
-// Launch a window over w.nreps replicates and, for the replicates that compact, the segmented scan
-// and scatter into `compact_dst` (the other state buffer).
+// Expected slots (at the window's end) up to which one replicate's window runs a slot per thread.  Window
+// kernels of 25 generations on a B200, a slot per thread against a quad per thread: 23 / 51 us at 12,000
+// slots, 28 / 53 at 92,000, 54 / 70 at 368,000, 92 / 104 at 648,000, 96 / 96 at 736,000, 109 / 106 at 833,000 and
+// 178 / 130 at 1,470,000 (N = 1e4 and 2e5, neutral and gamma = -10).
+#ifndef GF_SLOT_WINDOW_SLOTS
+#define GF_SLOT_WINDOW_SLOTS 600000
+#endif
+constexpr long long kSlotWindowSlots = GF_SLOT_WINDOW_SLOTS;
+
+// Launch a window over w.nreps replicates (one passed by value) and, for the replicates that compact, the
+// segmented scan and scatter into `compact_dst` (the other state buffer).
 gf_status window_run(Engine* e, const WindowLaunch& w, float* compact_dst, cudaEvent_t after_window,
                      cudaEvent_t before_compaction) {
-  const bool keys = GF_WINDOW_UNIFORM_KEYS && w.uniform_key && w.nreps == 1;
-  switch (e->draw_strategy) {
-    case kDrawWarp: launch_window_kernel<kDrawWarp, false>(e, w); break;
-    case kDrawGrouped: launch_window_kernel<kDrawGrouped, false>(e, w); break;
-    case kDrawNormalAll: launch_window_kernel<kDrawNormalAll, false>(e, w); break;
-    case kDrawPooledSearch:
-      if (keys) launch_window_kernel<kDrawPooledSearch, true>(e, w);
-      else launch_window_kernel<kDrawPooledSearch, false>(e, w);
-      break;
-    default:
-      if (keys) launch_window_kernel<kDrawLanes, true>(e, w);
-      else launch_window_kernel<kDrawLanes, false>(e, w);
-      break;
+  const bool single = w.reps == nullptr;
+  const bool slots = single && w.expected_slots <= kSlotWindowSlots && e->draw_strategy == kDrawLanes;
+  if (slots) {
+    const long long blocks = (w.one.ntiles * static_cast<long long>(kWinTile) + kSlotThreads - 1) / kSlotThreads;
+    window_slots_kernel<<<static_cast<int>(std::max(1ll, std::min(blocks, 16ll * e->num_sms))), kSlotThreads, 0,
+                          e->stream>>>(w.A, w.B, w.id_gp_cur, w.id_tid_cur, w.flags, w.M_in, w.M_end, w.M_next, w.recs,
+                                       w.stats, w.fault, philox_round_keys(w.one.seed1, w.one.seed2), w.one);
+  } else {
+    switch (e->draw_strategy) {
+      case kDrawWarp:
+        if (single) launch_window_kernel<kDrawWarp, true>(e, w);
+        else launch_window_kernel<kDrawWarp, false>(e, w);
+        break;
+      case kDrawGrouped:
+        if (single) launch_window_kernel<kDrawGrouped, true>(e, w);
+        else launch_window_kernel<kDrawGrouped, false>(e, w);
+        break;
+      case kDrawNormalAll:
+        if (single) launch_window_kernel<kDrawNormalAll, true>(e, w);
+        else launch_window_kernel<kDrawNormalAll, false>(e, w);
+        break;
+      case kDrawPooledSearch:
+        if (single) launch_window_kernel<kDrawPooledSearch, true>(e, w);
+        else launch_window_kernel<kDrawPooledSearch, false>(e, w);
+        break;
+      default:
+        if (single) launch_window_kernel<kDrawLanes, true>(e, w);
+        else launch_window_kernel<kDrawLanes, false>(e, w);
+        break;
+    }
   }
   GF_CUDA(e, cudaGetLastError());
   e->kernel_launches += 1;
   if (after_window) GF_CUDA(e, cudaEventRecord(after_window, e->stream));
   if (before_compaction) GF_CUDA(e, cudaEventRecord(before_compaction, e->stream));
-  if (w.any_compact) {
-    seg_scan_kernel<<<w.nreps, kSegScanThreads, 0, e->stream>>>(w.tile_count, w.tile_offset, w.reps, w.M_end,
-                                                                w.M_out, w.list);
+  if (!w.any_compact) return GF_OK;
+  const int sblocks = std::max(1, std::min(w.total_tiles, e->num_sms * 8));
+  if (slots) {
+    compact_slots_kernel<<<sblocks, kWinThreads, 0, e->stream>>>(w.B, compact_dst, w.id_gp_cur, w.id_tid_cur,
+                                                                 w.id_gp_next, w.id_tid_next, w.flags, w.M_end, w.M_out,
+                                                                 w.one, w.mail, w.mail_tag);
     GF_CUDA(e, cudaGetLastError());
-    const int sblocks = std::max(1, std::min(w.total_tiles, e->num_sms * 8));
-    auto scatter = w.nreps == 1 ? seg_scatter_kernel<true> : seg_scatter_kernel<false>;
-    scatter<<<sblocks, kWinThreads, 0, e->stream>>>(w.B, compact_dst, w.id_gp_cur, w.id_tid_cur, w.id_gp_next,
-                                                    w.id_tid_next, w.flags, w.tile_offset, w.reps, w.nreps,
-                                                    w.M_end, w.total_tiles, w.total_tiles_dev, w.list);
-    GF_CUDA(e, cudaGetLastError());
-    e->kernel_launches += 2;
+    e->kernel_launches += 1;
+    return GF_OK;
   }
+  auto scan = single ? seg_scan_kernel<true> : seg_scan_kernel<false>;
+  scan<<<w.nreps, kSegScanThreads, 0, e->stream>>>(w.tile_count, w.tile_offset, w.reps, w.M_end, w.M_out, w.list, w.one,
+                                                   w.mail, w.mail_tag);
+  GF_CUDA(e, cudaGetLastError());
+  auto scatter = single ? seg_scatter_kernel<true> : seg_scatter_kernel<false>;
+  scatter<<<sblocks, kWinThreads, 0, e->stream>>>(w.B, compact_dst, w.id_gp_cur, w.id_tid_cur, w.id_gp_next,
+                                                  w.id_tid_next, w.flags, w.tile_offset, w.reps, w.nreps, w.M_end,
+                                                  w.total_tiles, w.total_tiles_dev, w.list, w.one);
+  GF_CUDA(e, cudaGetLastError());
+  e->kernel_launches += 2;
   return GF_OK;
 }
 
