@@ -79,6 +79,28 @@ __device__ __forceinline__ int clampi(int v, int lo, int hi) { return max(lo, mi
 #endif
 
 
+// Drift of one quad lane as the window kernels evaluate it: the count drawn from frequency x, clamped to
+// [0, N], as a float (every count below 2^24 is one, and above that the draw itself is).  The same value as
+// clampi(binom_draw_body(...), 0, N), in fewer instructions:
+//   * the two ends share one search: N - search(N - mean) at the upper one;
+//   * the normal approximation is rounded half away from zero by adding 1/2 toward zero and truncating (the
+//     sum never reaches the next integer from below; what is negative clamps to 0 either way), and stays a
+//     float, clamped there (a draw that is not a number gives 0, as its conversion to an integer does);
+//   * a fixed slot needs no case of its own: its mean is N, and the search at the upper end returns 0 at
+//     once for N - mean = 0.
+__device__ __forceinline__ float binom_draw_count(uint32_t bits, float x, int N, float Nf) {
+  const float mean = x * N;
+  const float var = (1.0f - x) * (x * N);
+  const bool low = mean <= kMeanBoundary;
+  if (low || mean >= Nf - kMeanBoundary) {
+    const float m = low ? mean : Nf - mean;
+    const int j = Nf < kBinomNBoundary ? binom_search(u01(bits), m, m / Nf, Nf) : pois_search(u01(bits), m);
+    return static_cast<float>(clampi(low ? j : N - j, 0, N));
+  }
+  const float r = truncf(__fadd_rz(normcdfinv(u01(bits)) * sqrtf(var) + mean, 0.5f));
+  return fminf(fmaxf(r, 0.f), Nf);
+}
+
 // How the draws of a warp's quads are scheduled.  All three give identical results: every lane
 // calls the same sampler on the same (bits, mean, var, N); only the order of the calls differs.
 enum DrawStrategy : int {

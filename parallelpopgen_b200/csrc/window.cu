@@ -449,14 +449,14 @@ __device__ __forceinline__ void post_count(unsigned long long* mail, unsigned ta
 // draws of a quad are no longer one thread's chain: a generation takes the latency of one draw, not of
 // four with both sampler branches each.  That is what a state of few mutations waits for: 0.7 us a
 // generation against 1.9 at 12,000 slots; see kSlotWindowSlots for where the line lies.
-struct SlotGen {
+struct __align__(16) SlotGen {   // two 16-byte loads
   int generation, Nc;
   int M;            // mutations at the generation's start
-  int new_count;
+  float Nf;         // Nc
   float sel_a, sel_b, F, h;
 };
 
-// Slot e's frequency after the generation (e < G.M): the arithmetic and counters of the window kernel.
+// Slot e's frequency after the generation (e < G.M): the arithmetic and counters of the generation kernel.
 template <bool KEYS>
 __device__ __forceinline__ float slot_generation(float x, int e, const SlotGen& G, const PhiloxKeys& keys, int seed1,
                                                  int seed2) {
@@ -465,23 +465,24 @@ __device__ __forceinline__ float slot_generation(float x, int e, const SlotGen& 
   const bool neutral = G.sel_a == 0.f && G.sel_b == 0.f;
   const float xs = neutral ? selected_freq<true>(x, 0.f, 0.f, 0.f, 0.f)
                            : selected_freq<false>(x, G.sel_a, G.sel_b, G.F, G.h);
-  int res = (xs == 1.f && N > 6) ? N : 0;
+  const float Nf = G.Nf;
+  float count = 0.f;
   if (e < (G.M & ~3)) {
-    if (!(xs == 0.f || (xs == 1.f && N > 6))) {
+    if (xs != 0.f) {
       const int q = e >> 2, j = e & 3;
       uint4 r;
       if (KEYS) r = philox4x32_10_keys(make_uint4(static_cast<uint32_t>(q + 2), static_cast<uint32_t>(g), 0u, 0u), keys);
       else r = philox(seed1, seed2, q + 2, g, 0, 0);
-      const uint32_t bits = j == 0 ? r.x : j == 1 ? r.y : j == 2 ? r.z : r.w;
-      res = GF_LANE_DRAW(bits, xs * N, (1.0f - xs) * (xs * N), static_cast<float>(N));
+      count = binom_draw_count(j == 0 ? r.x : j == 1 ? r.y : j == 2 ? r.z : r.w, xs, N, Nf);
     }
-  } else {
-    res = drift_tail(seed1, seed2, e, g, 0, xs, N);   // scalar tail: counter (slot + 2), variance in double
+  } else {   // scalar tail: counter (slot + 2), variance in double
+    count = static_cast<float>(clampi(drift_tail(seed1, seed2, e, g, 0, xs, N), 0, N));
   }
-  return static_cast<float>(clampi(res, 0, N)) / static_cast<float>(N);
+  return count / Nf;
 }
 
 constexpr int kSlotThreads = 128;   // one SM takes several blocks, and a small state spreads over many SMs
+static_assert(kSlotThreads >= kMaxWindowGenerations, "a thread per record");
 
 // The records of a window in shared memory: s_gen, the frequencies of new mutations, and whether a lost slot
 // stays lost through every generation (its selected frequency is 0; not so if a coefficient is infinite).
@@ -489,14 +490,13 @@ constexpr int kSlotThreads = 128;   // one SM takes several blocks, and a small 
 __device__ __forceinline__ void load_slot_generations(SlotGen* s_gen, float* s_new, int* s_scan, int* s_lost_stays,
                                                       const WinGen* __restrict__ recs, int ngen, int M0) {
   const int t = threadIdx.x, lane = t & 31, warp = t >> 5;
-  static_assert(kSlotThreads >= kMaxWindowGenerations, "a thread per record");
   if (t == 0) *s_lost_stays = 1;
   __syncthreads();
   int births = 0;
   if (t < ngen) {
     const WinGen G = recs[t];
     births = G.new_count;
-    s_gen[t] = {G.generation, G.Nc, 0, G.new_count, G.sel_a, G.sel_b, G.F, G.h};
+    s_gen[t] = {G.generation, G.Nc, 0, static_cast<float>(G.Nc), G.sel_a, G.sel_b, G.F, G.h};
     s_new[t] = G.new_freq;
     if (!(G.sel_a == 0.f && G.sel_b == 0.f) && !(selected_freq<false>(0.f, G.sel_a, G.sel_b, G.F, G.h) == 0.f))
       *s_lost_stays = 0;
@@ -630,6 +630,314 @@ __global__ void __launch_bounds__(kWinThreads)
     if (tile == ntiles - 1 && t == kWinThreads - 1) {   // lane 31 holds the tile's survivors
       M_out[R.rep] = before + incl;
       post_count(mail, tag, before + incl);
+    }
+  }
+}
+
+// ------------------------------------------------------------------------------------------------
+// Large windows: a quad per thread while most of its slots live, then the living slots packed
+// ------------------------------------------------------------------------------------------------
+// A quad per thread shares one Philox block over four draws, but a warp walks all four lane positions, with
+// both sampler branches where its lanes differ, as long as one of its 128 slots lives -- and new mutations
+// die fast: of a tile of births half the slots are lost after two generations, four fifths after eight.
+// Once fewer than kPackPairs of a tile's 256 threads have two living slots or more, the block therefore moves
+// the frequencies to shared memory and hands out the living slots one per thread, densely (each evaluating
+// its quad's Philox block alone), repacking every few generations.  A slot's counters depend on its position
+// only, so who computes it does not matter.  Lost slots cost nothing from then on.
+//
+// Issue-bound (78 % of issue slots, 25 of 32 lanes).  Windows of 25 generations on a B200, against a quad per
+// thread throughout (window_kernel): N = 2e5, L = 2.5e8, neutral 354 -> 293 us, gamma = -10 357 -> 293; N = 1e4 with 4
+// million slots 201 -> 157; the batched windows of 256 replicates (N0 in [1e3, 1e4]) 400 -> 310 ms in all.
+// A third of that is the shorter draw (binom_draw_count) and generation loop: 20 % fewer warp instructions.
+//
+// kPackPairs: 100 and 190 measured 1 % slower (the neutral half below).  The threads are counted after two
+// generations of a full tile of births and then after each, after four of a tile the window began with and
+// then after every fifth (one barrier: counting the slots themselves every third generation cost 8 % of the
+// instructions); the first packed stage lasts three generations, each later one a generation longer (2 or 4
+// at first: the same within 1 %).
+constexpr int kPackPairs = 150;
+
+// A whole quad's generation: Philox (q + 2, g, 0, 0), lanes x, y, z, w.
+template <bool KEYS>
+__device__ __forceinline__ void quad_generation(float (&x)[4], int q, const SlotGen& G, const PhiloxKeys& keys,
+                                                int seed1, int seed2) {
+  const int N = G.Nc, g = G.generation;
+  if (N <= 0) {   // extinction generation: the population's row is cleared
+#pragma unroll
+    for (int j = 0; j < 4; ++j) x[j] = 0.f;
+    return;
+  }
+  if (!(G.sel_a == 0.f && G.sel_b == 0.f)) {
+#pragma unroll
+    for (int j = 0; j < 4; ++j) x[j] = selected_freq<false>(x[j], G.sel_a, G.sel_b, G.F, G.h);
+  }
+  const float Nf = G.Nf;
+  if (x[0] != 0.f || x[1] != 0.f || x[2] != 0.f || x[3] != 0.f) {
+    uint4 r;
+    if (KEYS) r = philox4x32_10_keys(make_uint4(static_cast<uint32_t>(q + 2), static_cast<uint32_t>(g), 0u, 0u), keys);
+    else r = philox(seed1, seed2, q + 2, g, 0, 0);
+    const uint32_t bits[4] = {r.x, r.y, r.z, r.w};
+#pragma unroll
+    for (int j = 0; j < 4; ++j)
+      if (x[j] != 0.f) x[j] = binom_draw_count(bits[j], x[j], N, Nf) / Nf;
+  }
+#pragma unroll
+  for (int j = 0; j < 4; ++j)
+    if (x[j] == 0.f) x[j] = 0.f;   // a negative zero of the caller's becomes a positive one, as a draw gives
+}
+
+// Exclusive position of this thread's `c` items in the block's order of (round, thread), and their total.
+// s_part: [kWinThreads / 32] words.  Ends with the block past a barrier; s_part is free again after the next one.
+__device__ __forceinline__ int pack_position(int c, int* s_part, int& total) {
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  int incl = c;
+#pragma unroll
+  for (int o = 1; o < 32; o <<= 1) {
+    const int y = __shfl_up_sync(0xFFFFFFFFu, incl, o);
+    if (lane >= o) incl += y;
+  }
+  if (lane == 31) s_part[warp] = incl;
+  __syncthreads();
+  int before = 0;
+  total = 0;
+#pragma unroll
+  for (int w = 0; w < kWinThreads / 32; ++w) {
+    const int v = s_part[w];
+    before += w < warp ? v : 0;
+    total += v;
+  }
+  return before + incl - c;
+}
+
+template <bool KEYS>
+__global__ void __launch_bounds__(kWinThreads, KEYS ? GF_WINDOW_MIN_BLOCKS_KEYS : GF_WINDOW_MIN_BLOCKS)
+    window_pack_kernel(const float* __restrict__ A, float* __restrict__ B, int* __restrict__ id_gp,
+                       int* __restrict__ id_tid, unsigned* __restrict__ flags, unsigned* __restrict__ tile_count,
+                       const int* __restrict__ M_in, int* __restrict__ M_end, int* __restrict__ M_next,
+                       const WinRep* __restrict__ reps, int nreps, const WinGen* __restrict__ recs, int total_tiles,
+                       const int* __restrict__ total_dev, unsigned long long* __restrict__ stats,
+                       int* __restrict__ fault, const PhiloxKeys keys, int* __restrict__ sched, const RepList list,
+                       const WinRep one) {
+  __shared__ int s_rep;
+  __shared__ int s_tile;
+  __shared__ int s_part[2][kWinThreads / 32];
+  __shared__ int s_tile0[KEYS ? 1 : kRepCache];
+  __shared__ SlotGen s_gen[kMaxWindowGenerations];
+  __shared__ float s_new[kMaxWindowGenerations];
+  __shared__ int s_scan[kWinThreads / 32];
+  __shared__ int s_lost_stays;
+  __shared__ float4 s_x[kWinThreads];
+  __shared__ unsigned short s_list[2][kWinTile];
+  const int lane = threadIdx.x & 31;
+  const int ntiles_all = total_dev ? *total_dev : total_tiles;
+  const int nlist = KEYS ? 1 : list_count(list, nreps);
+  if (!KEYS) load_tile0(s_tile0, list, reps, nlist);
+  int loaded = -1;   // the replicate whose records s_gen holds
+  // tiles are handed out in order by an atomic counter, as in window_kernel
+  for (;;) {
+    if (threadIdx.x == 0) {
+      const int t = atomicAdd(sched, 1);
+      s_tile = t;
+      s_rep = KEYS ? 0 : t < ntiles_all ? list_rep(list, find_rep_cached(s_tile0, list, reps, nlist, t)) : -1;
+    }
+    __syncthreads();
+    const int gt = s_tile, rep = s_rep;
+    if (gt >= ntiles_all) break;   // block-uniform
+    const WinRep R = KEYS ? one : reps[rep];
+    __syncthreads();
+    const int t = gt - R.tile0;
+    const int q = t * kWinThreads + threadIdx.x;  // quad within the replicate
+    const int s0 = 4 * q;
+    const int cap = static_cast<int>(R.capacity);
+    const int M0 = M_in[R.rep];
+    const long long end = M0 + R.births;
+    // a tile past the replicate's end-of-window count has nothing to do (tile 0 keeps the bookkeeping)
+    if (t > 0 && static_cast<long long>(t) * kWinTile >= end) continue;   // block-uniform
+    if (rep != loaded) {
+      load_slot_generations(s_gen, s_new, s_scan, &s_lost_stays, recs + R.rec, R.ngen, M0);
+      loaded = rep;
+    }
+    float* const rowB = B + R.base;
+    const float* const rowA = A + R.base;
+    int* const gp = id_gp + R.base;
+    int* const tid = id_tid + R.base;
+
+    float x[4];
+    if (s0 + 3 < M0) {
+      const float4 v = __ldg(reinterpret_cast<const float4*>(rowA + s0));
+      x[0] = v.x; x[1] = v.y; x[2] = v.z; x[3] = v.w;
+    } else {
+#pragma unroll
+      for (int j = 0; j < 4; ++j) x[j] = (s0 + j < M0) ? rowA[s0 + j] : 0.f;
+    }
+
+    // a tile of births starts with the generation that appends its first one
+    const int tile_first = t * kWinTile;
+    int k = 0;
+    if (tile_first >= M0) {
+      int hi = R.ngen - 1;
+      while (k < hi) {
+        const int mid = (k + hi + 1) >> 1;
+        if (s_gen[mid].M <= tile_first) k = mid;
+        else hi = mid - 1;
+      }
+    }
+    // ---- until every slot of the tile is born: whole quads, the scalar tail and births ----
+#pragma unroll 1
+    for (; k < R.ngen && s_gen[k].M < tile_first + kWinTile; ++k) {
+      const SlotGen& G = s_gen[k];
+      const int M = G.M;
+      if (s0 + 3 < (M & ~3)) {
+        quad_generation<KEYS>(x, q, G, keys, R.seed1, R.seed2);
+      } else if (s0 < M) {
+#pragma unroll 1
+        for (int j = 0; j < 4; ++j) {
+          if (s0 + j >= M) break;
+          const float v = slot_generation<KEYS>(j == 0 ? x[0] : j == 1 ? x[1] : j == 2 ? x[2] : x[3], s0 + j, G, keys,
+                                                R.seed1, R.seed2);
+          x[0] = j == 0 ? v : x[0];
+          x[1] = j == 1 ? v : x[1];
+          x[2] = j == 2 ? v : x[2];
+          x[3] = j == 3 ? v : x[3];
+        }
+      }
+      // births: slots [M, M + new_count) start at 1/Nc with ID (g, 0, slot - M + 1)
+      const int Mn = k + 1 < R.ngen ? s_gen[k + 1].M : static_cast<int>(end);
+      if (s0 + 3 >= M && s0 < Mn) {
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+          const int e = s0 + j;
+          if (e >= M && e < Mn && e < cap) {
+            x[j] = s_new[k];
+            gp[e] = G.generation;
+            tid[e] = e - M + 1;
+          }
+        }
+      }
+    }
+    // ---- a full tile: whole quads only, and now and then a count of the threads with two living slots ----
+    bool packed = false;
+    int check = tile_first >= M0 ? 2 : 4;
+#pragma unroll 1
+    while (k < R.ngen) {
+      quad_generation<KEYS>(x, q, s_gen[k], keys, R.seed1, R.seed2);
+      ++k;
+      if (--check > 0) continue;
+      check = tile_first >= M0 ? 1 : 5;
+      if (k + 2 > R.ngen || !s_lost_stays) continue;
+      int c = 0;
+#pragma unroll
+      for (int j = 0; j < 4; ++j) c += __float_as_uint(x[j]) != 0u ? 1 : 0;
+      if (__syncthreads_count(c >= 2) <= kPackPairs) {
+        packed = true;
+        break;
+      }
+    }
+    if (packed) {   // block-uniform
+      int living;
+      {
+        s_x[threadIdx.x] = make_float4(x[0], x[1], x[2], x[3]);
+        int c = 0;
+#pragma unroll
+        for (int j = 0; j < 4; ++j) c += __float_as_uint(x[j]) != 0u ? 1 : 0;
+        int living_at = pack_position(c, s_part[0], living);
+#pragma unroll
+        for (int j = 0; j < 4; ++j)
+          if (__float_as_uint(x[j]) != 0u) s_list[0][living_at++] = static_cast<unsigned short>(4 * threadIdx.x + j);
+        __syncthreads();
+      }
+      float* const s_xs = reinterpret_cast<float*>(s_x);
+      int cur = 0, stage = 3;
+      while (living > 0) {
+        const int k1 = min(R.ngen, k + stage);
+        int stays = 0;   // of this thread's slots, at positions t, t + 256, ...: how many still live
+#pragma unroll 1
+        for (int at = threadIdx.x; at < living; at += kWinThreads) {
+          const int local = s_list[cur][at];
+          float v = s_xs[local];
+#pragma unroll 1
+          for (int kk = k; kk < k1; ++kk) {
+            v = slot_generation<KEYS>(v, tile_first + local, s_gen[kk], keys, R.seed1, R.seed2);
+            if (__float_as_uint(v) == 0u) break;
+          }
+          s_xs[local] = v;
+          stays += __float_as_uint(v) != 0u ? 1 : 0;
+        }
+        k = k1;
+        if (k >= R.ngen) break;   // block-uniform
+        const int had = living;
+        int to = pack_position(stays, s_part[cur ^ 1], living);
+#pragma unroll 1
+        for (int at = threadIdx.x; at < had; at += kWinThreads) {
+          const int local = s_list[cur][at];
+          if (__float_as_uint(s_xs[local]) != 0u) s_list[cur ^ 1][to++] = static_cast<unsigned short>(local);
+        }
+        __syncthreads();
+        cur ^= 1;
+        stage += 1;
+      }
+      __syncthreads();
+      const float4 v = s_x[threadIdx.x];
+      x[0] = v.x; x[1] = v.y; x[2] = v.z; x[3] = v.w;
+    }
+    const int Mw = static_cast<int>(min(end, static_cast<long long>(cap)));
+    if (s0 + 3 < Mw) {
+      *reinterpret_cast<float4*>(rowB + s0) = make_float4(x[0], x[1], x[2], x[3]);
+    } else {
+#pragma unroll
+      for (int j = 0; j < 4; ++j)
+        if (s0 + j < Mw) rowB[s0 + j] = x[j];
+    }
+
+    if (R.compact) {
+      // flag_segregating_mutations for one population: keep unless lost or fixed (when alive), or
+      // if preserved
+      const int alive = R.ngen > 0 ? recs[R.rec + R.ngen - 1].alive : 1;
+      unsigned keep = 0;
+#pragma unroll
+      for (int j = 0; j < 4; ++j) {
+        const int e = s0 + j;
+        if (e >= Mw) continue;
+        // lost or fixed in the (only) population -- or the population is not alive -- removes it
+        bool kp = alive && !(x[j] <= 0.f || x[j] >= 1.f);
+        if (R.check_preserved && e < M0 && tid[e] < 0) kp = true;
+        if (kp) keep |= 1u << j;
+      }
+      unsigned word = keep << ((lane & 7) * 4);
+      word |= __shfl_xor_sync(0xFFFFFFFFu, word, 1);
+      word |= __shfl_xor_sync(0xFFFFFFFFu, word, 2);
+      word |= __shfl_xor_sync(0xFFFFFFFFu, word, 4);
+      if ((lane & 7) == 0) flags[(R.base + s0) >> 5] = word;
+      const int c = __reduce_add_sync(0xFFFFFFFFu, __popc(keep));
+      if (lane == 0) s_scan[threadIdx.x >> 5] = c;
+      __syncthreads();
+      if (threadIdx.x == 0) {
+        unsigned tot = 0;
+#pragma unroll
+        for (int w = 0; w < kWinThreads / 32; ++w) tot += s_scan[w];
+        tile_count[R.base / kWinTile + t] = tot;
+      }
+      __syncthreads();
+    }
+
+    if (t == 0 && threadIdx.x == 0) {
+      // window bookkeeping, once per replicate
+      unsigned long long mg = 0;
+      for (int kk = 0; kk < R.ngen; ++kk) mg += static_cast<unsigned long long>(s_gen[kk].M);
+      atomicAdd(stats, mg);
+      atomicAdd(stats + 1, static_cast<unsigned long long>(R.ngen));
+      if (end > cap) atomicExch(fault, kFaultCapacity);
+      M_end[R.rep] = Mw;
+      if (M_next && !R.compact) M_next[R.rep] = Mw;
+    }
+  }
+  // the launch's last block sets the scheduler back to zero, as in window_kernel
+  if (threadIdx.x == 0) {
+    __threadfence();
+    const int finished = atomicAdd(sched + 1, 1);
+    if (finished == static_cast<int>(gridDim.x) - 1) {
+      sched[0] = 0;
+      sched[1] = 0;
     }
   }
 }
@@ -825,32 +1133,43 @@ void batch_step_tiles(Engine* e, WinRep* d_table, int R, const int* M_in, const 
   e->kernel_launches += 1;
 }
 
-template <int DRAW, bool KEYS>
-static void launch_window_kernel(Engine* e, const WindowLaunch& w) {
-  // resident blocks per SM, queried once per instantiation (thread-safe initialisation; the same on
-  // every B200)
-  static const int occupancy = [] {
-    int o = 0;
-    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&o, window_kernel<DRAW, KEYS>, kWinThreads, 0) !=
-            cudaSuccess ||
-        o < 1) {
-      cudaGetLastError();
-      o = 1;
-    }
-    return o;
-  }();
+template <bool KEYS, typename Kernel>
+static void launch_window_tiles(Engine* e, const WindowLaunch& w, Kernel kernel, int occupancy) {
   const int per_sm = e->blocks_per_sm > 0 ? std::min(e->blocks_per_sm, occupancy) : occupancy;
   const int blocks = std::max(1, std::min(w.total_tiles, e->num_sms * per_sm));
   const PhiloxKeys keys = philox_round_keys(w.one.seed1, w.one.seed2);
-  window_kernel<DRAW, KEYS><<<blocks, kWinThreads, 0, e->stream>>>(
-      w.A, w.B, w.id_gp_cur, w.id_tid_cur, w.flags, w.tile_count, w.M_in, w.M_end, w.M_next, w.reps, w.nreps,
-      w.recs, w.total_tiles, w.total_tiles_dev, w.stats, w.fault, keys, w.sched, w.list, w.one);
+  kernel<<<blocks, kWinThreads, 0, e->stream>>>(w.A, w.B, w.id_gp_cur, w.id_tid_cur, w.flags, w.tile_count, w.M_in,
+                                                w.M_end, w.M_next, w.reps, w.nreps, w.recs, w.total_tiles,
+                                                w.total_tiles_dev, w.stats, w.fault, keys, w.sched, w.list, w.one);
+}
+
+// Resident blocks per SM of a kernel (the same on every B200).
+template <typename Kernel>
+static int resident_blocks(Kernel kernel) {
+  int o = 0;
+  if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&o, kernel, kWinThreads, 0) != cudaSuccess || o < 1) {
+    cudaGetLastError();
+    o = 1;
+  }
+  return o;
+}
+
+// One large or several replicates: lane order on the packing kernel, the other draw schedules on window_kernel.
+template <int DRAW, bool KEYS>
+static void launch_window_kernel(Engine* e, const WindowLaunch& w) {
+  if constexpr (DRAW == kDrawLanes) {
+    static const int occupancy = resident_blocks(window_pack_kernel<KEYS>);   // thread-safe, once
+    launch_window_tiles<KEYS>(e, w, window_pack_kernel<KEYS>, occupancy);
+  } else {
+    static const int occupancy = resident_blocks(window_kernel<DRAW, KEYS>);
+    launch_window_tiles<KEYS>(e, w, window_kernel<DRAW, KEYS>, occupancy);
+  }
 }
 
 // Expected slots (at the window's end) up to which one replicate's window runs a slot per thread.  Window
-// kernels of 25 generations on a B200, a slot per thread against a quad per thread: 23 / 51 us at 12,000
-// slots, 28 / 53 at 92,000, 54 / 70 at 368,000, 92 / 104 at 648,000, 96 / 96 at 736,000, 109 / 106 at 833,000 and
-// 178 / 130 at 1,470,000 (N = 1e4 and 2e5, neutral and gamma = -10).
+// kernels of 25 generations on a B200, a slot per thread against the packing kernel: 23 / 53 us at 12,000
+// slots, 27 / 55 at 92,000, 50 / 70 at 368,000, 74 / 80 at 552,000 (N = 1e4, neutral), 92 / 104 at 648,000 (gamma = -10),
+// 86 / 86 at 625,000, 98 / 90 at 736,000 and 111 / 94 at 833,000 (neutral, N = 1e4 and 2e5).
 #ifndef GF_SLOT_WINDOW_SLOTS
 #define GF_SLOT_WINDOW_SLOTS 600000
 #endif

@@ -1,5 +1,6 @@
-"""Windows of small states (a slot per thread, compaction in one launch) against one launch per generation:
-the same state bit for bit, at the sizes where the two differ in how they reach it."""
+"""Windows of small states (a slot per thread, compaction in one launch) and of large ones (a quad per thread
+until few slots live, then the living packed) against one launch per generation: the same state bit for
+bit, at the sizes where they differ in how they reach it."""
 from __future__ import annotations
 
 import numpy as np
@@ -33,11 +34,12 @@ def _same(model, L, gens, ci, start=None):
 
 
 # windows of one generation, of the longest kind (128) and past it; states of a few slots (tails of every
-# length), of several blocks, and just past the line to the quad kernel (about 600,000 slots)
+# length), of several blocks, and past the line to the packing kernel (about 600,000 slots), there also with
+# every draw on the binomial search (Nchrom_e below 100)
 @pytest.mark.parametrize("N,L,ngen,ci,gamma,F,h", [
     (40, 2e5, 37, 1, 0.0, 0.0, 0.5), (500, 3e5, 60, 7, -20.0, 0.3, 0.1), (2000, 1e6, 300, 130, 5.0, 0.0, 1.0),
     (1000, 1e4, 100, 25, 0.0, 0.0, 0.5), (10_000, 2e7, 130, 25, -10.0, 0.2, 0.5), (10_000, 7e8, 40, 20, 0.0, 0.0, 0.5),
-    (10_000, 1.1e9, 30, 15, -3.0, 0.0, 0.2)])
+    (10_000, 1.1e9, 30, 15, -3.0, 0.0, 0.2), (10_000, 3e9, 57, 27, 4.0, 0.1, 0.9), (40, 6e10, 45, 20, 0.0, 0.0, 0.5)])
 def test_slot_windows_equal_generations(N, L, ngen, ci, gamma, F, h):
     s = ConstantModel.s_from_gamma(gamma, N, F) if gamma else 0.0
     model = ConstantModel(N=N, mu=1e-8 if N < 5000 else 1e-9, s=s, F=F, h=h)
