@@ -323,6 +323,61 @@ __global__ void __launch_bounds__(kScanThreads)
   if (threadIdx.x == 0 && total_out) *total_out = static_cast<int>(s_carry);
 }
 
+// The same over many counts, kScanTile to a block: the tiles' sums, their scan by the kernel above, then each
+// tile's own.  The equilibrium start's 400,000 classes take 10 us in the three launches, and took 281 in one
+// block.
+constexpr int kScanTileThreads = 256;
+constexpr int kScanTile = 4 * kScanTileThreads;
+constexpr int kScanOneBlock = kScanThreads * kScanItems;   // counts that one pass of one block covers
+
+// Exclusive prefix of this thread's v over the block, and the block's total.
+__device__ __forceinline__ unsigned block_exclusive(unsigned v, unsigned* s_part, unsigned& total) {
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  unsigned incl = v;
+#pragma unroll
+  for (int o = 1; o < 32; o <<= 1) {
+    const unsigned y = __shfl_up_sync(0xFFFFFFFFu, incl, o);
+    if (lane >= o) incl += y;
+  }
+  if (lane == 31) s_part[warp] = incl;
+  __syncthreads();
+  unsigned before = 0;
+  total = 0;
+#pragma unroll
+  for (int w = 0; w < kScanTileThreads / 32; ++w) {
+    before += w < warp ? s_part[w] : 0u;
+    total += s_part[w];
+  }
+  return before + incl - v;
+}
+
+// offset null: sums[tile] = the tile's total; else out = offset[tile] + exclusive prefix within the tile.
+__global__ void __launch_bounds__(kScanTileThreads)
+    scan_tile_kernel(const unsigned* __restrict__ in, int n, unsigned* __restrict__ sums,
+                     const unsigned* __restrict__ offset, unsigned* __restrict__ out) {
+  __shared__ unsigned s_part[kScanTileThreads / 32];
+  const int first = blockIdx.x * kScanTile + 4 * threadIdx.x;
+  unsigned v[4];
+  unsigned sum = 0;
+#pragma unroll
+  for (int j = 0; j < 4; ++j) {
+    v[j] = first + j < n ? in[first + j] : 0u;
+    sum += v[j];
+  }
+  unsigned total;
+  unsigned run = block_exclusive(sum, s_part, total);
+  if (!offset) {
+    if (threadIdx.x == 0) sums[blockIdx.x] = total;
+    return;
+  }
+  run += offset[blockIdx.x];
+#pragma unroll
+  for (int j = 0; j < 4; ++j) {
+    if (first + j < n) out[first + j] = run;
+    run += v[j];
+  }
+}
+
 // ------------------------------------------------------------------------------------------------
 // stable scatter of surviving slots (scatter_arrays, go_fish_impl.cu:147-189), staged through
 // shared memory so that every tile writes its survivors as one contiguous, coalesced run
@@ -409,9 +464,46 @@ __global__ void mse_area_kernel(float* __restrict__ area, int num_freq, float st
     area[id] = mse_area(id, step, N_ind, F, h, sa, sb);
 }
 
+// The integral over many frequencies (mse_integral_block's sums in the same order, so the same values): the
+// tiles' last sums, the carry through them, then every tile from its carry.  400,000 frequencies take 20 us in
+// the three launches, and took 304 in one block.
+struct MseTileSum {
+  double before_last_warp, last;   // the two terms that thread 1023 adds to the carry, in this order
+};
+
+__global__ void __launch_bounds__(1024) mse_tile_sums_kernel(const float* __restrict__ area, int num_freq,
+                                                             MseTileSum* __restrict__ sums) {
+  double before, incl;
+  mse_tile_scan(area, blockIdx.x * 1024, num_freq, before, incl);
+  if (threadIdx.x == 1023) sums[blockIdx.x] = {before, incl};
+}
+
+// carry[t] = the running total before tile t: one thread's chain, the sums staged by the others.
+__global__ void __launch_bounds__(1024) mse_carry_kernel(const MseTileSum* __restrict__ sums, int tiles,
+                                                         double* __restrict__ carry) {
+  __shared__ MseTileSum s_sum[1024];
+  double c = 0.0;
+  for (int base = 0; base < tiles; base += 1024) {
+    if (base + static_cast<int>(threadIdx.x) < tiles) s_sum[threadIdx.x] = sums[base + threadIdx.x];
+    __syncthreads();
+    if (threadIdx.x == 0) {
+      const int n = min(1024, tiles - base);
+      for (int t = 0; t < n; ++t) {
+        carry[base + t] = c;
+        c = c + s_sum[t].before_last_warp + s_sum[t].last;
+      }
+    }
+    __syncthreads();
+  }
+}
+
 __global__ void __launch_bounds__(1024) mse_integral_kernel(const float* __restrict__ area, float* __restrict__ integral,
-                                                            int num_freq) {
-  mse_integral_block(area, integral, num_freq);
+                                                            int num_freq, const double* __restrict__ carry) {
+  double before, incl;
+  const int idx = blockIdx.x * 1024 + threadIdx.x;
+  mse_tile_scan(area, blockIdx.x * 1024, num_freq, before, incl);
+  const double total = carry[blockIdx.x] + before + incl;
+  if (idx < num_freq) integral[num_freq - 1 - idx] = static_cast<float>(total);
 }
 
 __global__ void mse_count_kernel(unsigned* __restrict__ counts, const float* __restrict__ integral, int offset,
@@ -485,10 +577,9 @@ __global__ void pack_sample_kernel(const float* __restrict__ freq, long long cap
 
 static void release_sim(Engine* e) {
   // stream-ordered frees: the memory returns to the engine's pool for the next simulation
+  if (e->sim_mem) cudaFreeAsync(e->sim_mem, e->stream);
+  e->sim_mem = nullptr;
   for (int b = 0; b < 2; ++b) {
-    if (e->freq[b]) cudaFreeAsync(e->freq[b], e->stream);
-    if (e->id_gp[b]) cudaFreeAsync(e->id_gp[b], e->stream);
-    if (e->id_tid[b]) cudaFreeAsync(e->id_tid[b], e->stream);
     e->freq[b] = nullptr;
     e->id_gp[b] = nullptr;
     e->id_tid[b] = nullptr;
@@ -496,9 +587,6 @@ static void release_sim(Engine* e) {
   if (e->sel_table) cudaFreeAsync(e->sel_table, e->stream);
   e->sel_table = nullptr;
   e->sel_table_stride = 0;
-  if (e->flags) cudaFreeAsync(e->flags, e->stream);
-  if (e->tile_count) cudaFreeAsync(e->tile_count, e->stream);
-  if (e->tile_offset) cudaFreeAsync(e->tile_offset, e->stream);
   e->flags = nullptr;
   e->tile_count = nullptr;
   e->tile_offset = nullptr;
@@ -509,64 +597,57 @@ static void release_sim(Engine* e) {
   e->active = false;
 }
 
-// Allocate (zeroed) arrays of `cap` slots.  When `keep` > 0, the first `keep` slots of the current
-// buffers are carried over.
-static gf_status set_capacity(Engine* e, long long cap, long long keep) {
+// Lays (zeroed) arrays of `cap` slots out in one allocation: `mem`, if not null, of that capacity already, else
+// a new one.  When `keep` > 0, the first `keep` slots of the current buffers are carried over.
+static gf_status set_capacity(Engine* e, long long cap, long long keep, char* mem = nullptr) {
   cap = align_up(std::max<long long>(cap, kSlotAlign), kSlotAlign);
   if (cap > (1LL << 31) - kSlotAlign) return fail(e, GF_ERR_CAPACITY, "mutation capacity %lld exceeds 2^31 slots", cap);
   const int P = e->P;
-  float* nf[2] = {nullptr, nullptr};
-  int* ngp[2] = {nullptr, nullptr};
-  int* ntid[2] = {nullptr, nullptr};
-  unsigned *nflags = nullptr, *ncount = nullptr, *noffset = nullptr;
-  const long long ntiles = cap / kTileSlots;
-  cudaError_t err = cudaSuccess;
-  auto palloc = [e](void** p, size_t bytes) {
-    return e->pool ? cudaMallocFromPoolAsync(p, bytes, e->pool, e->stream) : cudaMallocAsync(p, bytes, e->stream);
+  const long long ntiles = cap / kTileSlots;   // cap is a multiple of 1,024: every slice is 128-byte aligned but the last
+  const size_t state = (2 * sizeof(float) * P + 4 * sizeof(int)) * static_cast<size_t>(cap);
+  const size_t flag_bytes = sizeof(unsigned) * static_cast<size_t>(cap / 32);
+  if (!mem) {
+    gf_status st = pool_alloc(e, reinterpret_cast<void**>(&mem), state + flag_bytes + 2 * sizeof(unsigned) * ntiles);
+    if (st != GF_OK) return st;
+  }
+  char* at = mem;
+  auto slice = [&at](size_t bytes) {
+    char* p = at;
+    at += bytes;
+    return p;
   };
-  for (int b = 0; b < 2 && err == cudaSuccess; ++b) {
-    err = palloc(reinterpret_cast<void**>(&nf[b]), sizeof(float) * P * cap);
-    if (err == cudaSuccess) err = palloc(reinterpret_cast<void**>(&ngp[b]), sizeof(int) * cap);
-    if (err == cudaSuccess) err = palloc(reinterpret_cast<void**>(&ntid[b]), sizeof(int) * cap);
-  }
-  if (err == cudaSuccess) err = palloc(reinterpret_cast<void**>(&nflags), sizeof(unsigned) * (cap / 32));
-  if (err == cudaSuccess) err = palloc(reinterpret_cast<void**>(&ncount), sizeof(unsigned) * ntiles);
-  if (err == cudaSuccess) err = palloc(reinterpret_cast<void**>(&noffset), sizeof(unsigned) * ntiles);
-  if (err != cudaSuccess) {
-    for (int b = 0; b < 2; ++b) {
-      if (nf[b]) cudaFreeAsync(nf[b], e->stream);
-      if (ngp[b]) cudaFreeAsync(ngp[b], e->stream);
-      if (ntid[b]) cudaFreeAsync(ntid[b], e->stream);
-    }
-    if (nflags) cudaFreeAsync(nflags, e->stream);
-    if (ncount) cudaFreeAsync(ncount, e->stream);
-    cudaGetLastError();
-    return cuda_fail(e, err, "allocating the mutation arrays");
-  }
+  float* nf[2];
+  int *ngp[2], *ntid[2];
   for (int b = 0; b < 2; ++b) {
-    GF_CUDA(e, cudaMemsetAsync(nf[b], 0, sizeof(float) * P * cap, e->stream));
-    GF_CUDA(e, cudaMemsetAsync(ngp[b], 0, sizeof(int) * cap, e->stream));
-    GF_CUDA(e, cudaMemsetAsync(ntid[b], 0, sizeof(int) * cap, e->stream));
+    nf[b] = reinterpret_cast<float*>(slice(sizeof(float) * P * cap));
+    ngp[b] = reinterpret_cast<int*>(slice(sizeof(int) * cap));
+    ntid[b] = reinterpret_cast<int*>(slice(sizeof(int) * cap));
   }
+  unsigned* nflags = reinterpret_cast<unsigned*>(slice(flag_bytes));
+  unsigned* ncount = reinterpret_cast<unsigned*>(slice(sizeof(unsigned) * ntiles));
+  unsigned* noffset = reinterpret_cast<unsigned*>(slice(sizeof(unsigned) * ntiles));
+  cudaError_t err = cudaMemsetAsync(mem, 0, state, e->stream);
   if (keep > 0 && e->capacity > 0) {
-    GF_CUDA(e, cudaMemcpy2DAsync(nf[e->cur], sizeof(float) * cap, e->freq[e->cur], sizeof(float) * e->capacity,
-                                 sizeof(float) * keep, P, cudaMemcpyDeviceToDevice, e->stream));
-    GF_CUDA(e, cudaMemcpyAsync(ngp[e->id_cur], e->id_gp[e->id_cur], sizeof(int) * keep, cudaMemcpyDeviceToDevice,
-                               e->stream));
-    GF_CUDA(e, cudaMemcpyAsync(ntid[e->id_cur], e->id_tid[e->id_cur], sizeof(int) * keep, cudaMemcpyDeviceToDevice,
-                               e->stream));
+    if (err == cudaSuccess)
+      err = cudaMemcpy2DAsync(nf[e->cur], sizeof(float) * cap, e->freq[e->cur], sizeof(float) * e->capacity,
+                              sizeof(float) * keep, P, cudaMemcpyDeviceToDevice, e->stream);
+    if (err == cudaSuccess)
+      err = cudaMemcpyAsync(ngp[e->id_cur], e->id_gp[e->id_cur], sizeof(int) * keep, cudaMemcpyDeviceToDevice, e->stream);
+    if (err == cudaSuccess)
+      err = cudaMemcpyAsync(ntid[e->id_cur], e->id_tid[e->id_cur], sizeof(int) * keep, cudaMemcpyDeviceToDevice,
+                            e->stream);
   }
+  if (err != cudaSuccess) {
+    cudaFreeAsync(mem, e->stream);
+    return cuda_fail(e, err, "setting up the mutation arrays");
+  }
+  if (e->sim_mem) cudaFreeAsync(e->sim_mem, e->stream);
+  e->sim_mem = mem;
   for (int b = 0; b < 2; ++b) {
-    if (e->freq[b]) cudaFreeAsync(e->freq[b], e->stream);
-    if (e->id_gp[b]) cudaFreeAsync(e->id_gp[b], e->stream);
-    if (e->id_tid[b]) cudaFreeAsync(e->id_tid[b], e->stream);
     e->freq[b] = nf[b];
     e->id_gp[b] = ngp[b];
     e->id_tid[b] = ntid[b];
   }
-  if (e->flags) cudaFreeAsync(e->flags, e->stream);
-  if (e->tile_count) cudaFreeAsync(e->tile_count, e->stream);
-  if (e->tile_offset) cudaFreeAsync(e->tile_offset, e->stream);
   e->flags = nflags;
   e->tile_count = ncount;
   e->tile_offset = noffset;
@@ -593,6 +674,14 @@ static gf_status begin_common(Engine* e, const gf_sim_config* c, long long initi
   if (c->compact_interval < 0) return fail(e, GF_ERR_INVALID_ARGUMENT, "compact_interval must be >= 0");
   GF_CUDA(e, cudaSetDevice(e->device));
   GF_CUDA(e, cudaStreamSynchronize(e->stream));
+  const long long want = std::max<long long>({static_cast<long long>(c->reserve_mutations),
+                                               2 * initial_mutations + 65536, 65536});
+  // the previous simulation's arrays serve again where they hold this one without being much larger: a
+  // repeated run then starts with what the first one grew to
+  const bool reuse = e->sim_mem && e->P == c->num_populations && e->capacity >= want && e->capacity <= 4 * want + 65536;
+  void* const mem = reuse ? e->sim_mem : nullptr;
+  const long long cap = e->capacity;
+  if (reuse) e->sim_mem = nullptr;   // kept
   release_sim(e);
   e->P = c->num_populations;
   e->seed1 = c->seed1;
@@ -605,9 +694,7 @@ static gf_status begin_common(Engine* e, const gf_sim_config* c, long long initi
   e->count_slot = 0;
   e->cur = 0;
   e->id_cur = 0;
-  const long long want = std::max<long long>({static_cast<long long>(c->reserve_mutations),
-                                               2 * initial_mutations + 65536, 65536});
-  gf_status st = set_capacity(e, want, 0);
+  gf_status st = set_capacity(e, reuse ? cap : want, 0, static_cast<char*>(mem));
   if (st != GF_OK) return st;
   GF_CUDA(e, cudaMemsetAsync(e->d_count, 0, sizeof(int) * kCountWords, e->stream));
   GF_CUDA(e, cudaMemsetAsync(e->d_stats, 0, sizeof(unsigned long long) * 2, e->stream));
@@ -1444,28 +1531,37 @@ gf_status gf_sim_begin_mse(gf_engine* g, const gf_sim_config* c, const gf_mse_po
     }
     for (int p = P; p <= kMaxPops; ++p) cr.first_class[p] = static_cast<int>(num_classes);
     GF_CUDA(e, cudaSetDevice(e->device));
-    // class counts, then their exclusive scan; the total is read back once (as the reference does)
-    unsigned* d_counts = nullptr;
-    unsigned* d_starts = nullptr;
-    float* d_area = nullptr;
-    float* d_integral = nullptr;
-    int* d_total = nullptr;
+    // class counts, then their exclusive scan; the total is read back once (as the reference does).  The
+    // scratch is one allocation.
     const long long ncls = std::max<long long>(num_classes, 1);
     long long max_nc = 1;
     for (int p = 0; p < P; ++p) max_nc = std::max<long long>(max_nc, pops[p].Nchrom_e);
+    const long long scan_tiles = (ncls + kScanTile - 1) / kScanTile, mse_tiles = (max_nc + 1023) / 1024;
+    char* d_scratch = nullptr;
+    size_t used = 0;
+    auto slice = [&used](size_t bytes) {
+      const size_t at = used;
+      used += (bytes + 255) / 256 * 256;
+      return at;
+    };
+    const size_t at_counts = slice(sizeof(unsigned) * ncls), at_starts = slice(sizeof(unsigned) * ncls);
+    const size_t at_area = slice(sizeof(float) * max_nc), at_integral = slice(sizeof(float) * max_nc);
+    const size_t at_sums = slice(sizeof(MseTileSum) * mse_tiles), at_carry = slice(sizeof(double) * mse_tiles);
+    const size_t at_tiles = slice(sizeof(unsigned) * scan_tiles), at_offsets = slice(sizeof(unsigned) * scan_tiles);
+    const size_t at_total = slice(sizeof(int));
     {
-      gf_status ast = pool_alloc(e, reinterpret_cast<void**>(&d_counts), sizeof(unsigned) * ncls);
-      if (ast == GF_OK) ast = pool_alloc(e, reinterpret_cast<void**>(&d_starts), sizeof(unsigned) * ncls);
-      if (ast == GF_OK) ast = pool_alloc(e, reinterpret_cast<void**>(&d_area), sizeof(float) * max_nc);
-      if (ast == GF_OK) ast = pool_alloc(e, reinterpret_cast<void**>(&d_integral), sizeof(float) * max_nc);
-      if (ast == GF_OK) ast = pool_alloc(e, reinterpret_cast<void**>(&d_total), sizeof(int));
-      if (ast != GF_OK) {
-        for (void* q : {static_cast<void*>(d_counts), static_cast<void*>(d_starts), static_cast<void*>(d_area),
-                        static_cast<void*>(d_integral), static_cast<void*>(d_total)})
-          if (q) cudaFreeAsync(q, e->stream);
-        return ast;
-      }
+      gf_status ast = pool_alloc(e, reinterpret_cast<void**>(&d_scratch), used);
+      if (ast != GF_OK) return ast;
     }
+    unsigned* d_counts = reinterpret_cast<unsigned*>(d_scratch + at_counts);
+    unsigned* d_starts = reinterpret_cast<unsigned*>(d_scratch + at_starts);
+    float* d_area = reinterpret_cast<float*>(d_scratch + at_area);
+    float* d_integral = reinterpret_cast<float*>(d_scratch + at_integral);
+    MseTileSum* d_sums = reinterpret_cast<MseTileSum*>(d_scratch + at_sums);
+    double* d_carry = reinterpret_cast<double*>(d_scratch + at_carry);
+    unsigned* d_tiles = reinterpret_cast<unsigned*>(d_scratch + at_tiles);
+    unsigned* d_offsets = reinterpret_cast<unsigned*>(d_scratch + at_offsets);
+    int* d_total = reinterpret_cast<int*>(d_scratch + at_total);
     GF_CUDA(e, cudaMemsetAsync(d_counts, 0, sizeof(unsigned) * ncls, e->stream));
     for (int p = 0; p < P; ++p) {
       const gf_mse_population& mp = pops[p];
@@ -1475,17 +1571,30 @@ gf_status gf_sim_begin_mse(gf_engine* g, const gf_sim_config* c, const gf_mse_po
       if (selected) {
         mse_area_kernel<<<148, 1024, 0, e->stream>>>(d_area, Nc, 1.0f / Nc, mp.N_ind, mp.F, mp.h, mp.sel_slope,
                                                       mp.sel_intercept);
-        mse_integral_kernel<<<1, 1024, 0, e->stream>>>(d_area, d_integral, Nc);
+        const int tiles = (Nc + 1023) / 1024;
+        mse_tile_sums_kernel<<<tiles, 1024, 0, e->stream>>>(d_area, Nc, d_sums);
+        mse_carry_kernel<<<1, 1024, 0, e->stream>>>(d_sums, tiles, d_carry);
+        mse_integral_kernel<<<tiles, 1024, 0, e->stream>>>(d_area, d_integral, Nc, d_carry);
       }
       mse_count_kernel<<<std::max(1, std::min(1184, (Nc + 255) / 256)), 256, 0, e->stream>>>(
           d_counts, d_integral, cr.first_class[p], mp.mu, mp.N_ind, Nc, c->num_sites, mp.sel_slope, mp.sel_intercept,
           mp.F, mp.h, c->seed1, c->seed2, p, selected ? 1 : 0);
       GF_CUDA(e, cudaGetLastError());
-      e->kernel_launches += selected ? 3 : 1;
+      e->kernel_launches += selected ? 5 : 1;
     }
     e->kernel_launches += 2;  // class scan + slot fill
-    scan_exclusive_kernel<<<1, kScanThreads, 0, e->stream>>>(d_counts, d_starts, static_cast<int>(num_classes), d_total,
-                                                              nullptr);
+    const int classes = static_cast<int>(num_classes);
+    if (classes > kScanOneBlock) {
+      scan_tile_kernel<<<static_cast<unsigned>(scan_tiles), kScanTileThreads, 0, e->stream>>>(d_counts, classes, d_tiles,
+                                                                                              nullptr, nullptr);
+      scan_exclusive_kernel<<<1, kScanThreads, 0, e->stream>>>(d_tiles, d_offsets, static_cast<int>(scan_tiles), d_total,
+                                                                nullptr);
+      scan_tile_kernel<<<static_cast<unsigned>(scan_tiles), kScanTileThreads, 0, e->stream>>>(d_counts, classes, nullptr,
+                                                                                              d_offsets, d_starts);
+      e->kernel_launches += 2;
+    } else {
+      scan_exclusive_kernel<<<1, kScanThreads, 0, e->stream>>>(d_counts, d_starts, classes, d_total, nullptr);
+    }
     GF_CUDA(e, cudaGetLastError());
     int M0 = 0;
     GF_CUDA(e, cudaMemcpyAsync(&M0, d_total, sizeof(int), cudaMemcpyDeviceToHost, e->stream));
@@ -1505,11 +1614,7 @@ gf_status gf_sim_begin_mse(gf_engine* g, const gf_sim_config* c, const gf_mse_po
       for (int p = 0; p < P; ++p)  // populations with equilibrium mutations (the others' rows stay zero)
         if (pops[p].Nchrom_e > 1) e->live_rows |= 1 << p;
     }
-    cudaFreeAsync(d_counts, e->stream);
-    cudaFreeAsync(d_starts, e->stream);
-    cudaFreeAsync(d_area, e->stream);
-    cudaFreeAsync(d_integral, e->stream);
-    cudaFreeAsync(d_total, e->stream);
+    cudaFreeAsync(d_scratch, e->stream);
     return st;
   });
 }

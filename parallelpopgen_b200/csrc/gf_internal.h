@@ -296,7 +296,8 @@ struct Engine {
   long long step_index = 0;  // generations run since begin
   int count_slot = 0;        // d_count slot holding the current mutation count
 
-  // device arrays; capacity = row stride in slots
+  // device arrays, slices of one allocation; capacity = row stride in slots
+  void* sim_mem = nullptr;
   long long capacity = 0;
   float* freq[2] = {nullptr, nullptr};      // [P][capacity]
   int* id_gp[2] = {nullptr, nullptr};       // origin generation | origin population << 24

@@ -23,39 +23,49 @@ __device__ __forceinline__ float mse_area(int id, float step, int N_ind, float F
   return step * (f1 + f2) / 2;
 }
 
-// Deterministic inclusive scan of the slices in double precision by one 1024-thread block, stored
-// reversed as float: integral[id] = sum_{k <= num_freq-1-id} area[k] (the reference scans in float
-// with CUB and then reverses, go_fish_impl.cuh:213-221; its float summation order is not fixed).
+// One tile (1,024 slices from `base` on) of the deterministic inclusive scan of the slices in double precision,
+// by one 1024-thread block: thread t's inclusive sum is carry + before + incl, added in this order, where
+// `before` is the sum of the warps before its own and the carry that of the tiles before.
+__device__ __forceinline__ void mse_tile_scan(const float* __restrict__ area, int base, int num_freq, double& before,
+                                              double& incl) {
+  __shared__ double s_warp[32];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int idx = base + threadIdx.x;
+  incl = idx < num_freq ? static_cast<double>(area[idx]) : 0.0;
+#pragma unroll
+  for (int o = 1; o < 32; o <<= 1) {
+    const double y = __shfl_up_sync(0xFFFFFFFFu, incl, o);
+    if (lane >= o) incl += y;
+  }
+  if (lane == 31) s_warp[warp] = incl;
+  __syncthreads();
+  if (warp == 0) {
+    const double w = s_warp[lane];
+    double wi = w;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const double y = __shfl_up_sync(0xFFFFFFFFu, wi, o);
+      if (lane >= o) wi += y;
+    }
+    s_warp[lane] = wi - w;
+  }
+  __syncthreads();
+  before = s_warp[warp];
+}
+
+// The whole scan by one block, stored reversed as float: integral[id] = sum_{k <= num_freq-1-id} area[k] (the
+// reference scans in float with CUB and then reverses, go_fish_impl.cuh:213-221; its float summation order is
+// not fixed).
 __device__ __forceinline__ void mse_integral_block(const float* __restrict__ area, float* __restrict__ integral,
                                                    int num_freq) {
-  __shared__ double s_warp[32];
   __shared__ double s_carry;
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   if (threadIdx.x == 0) s_carry = 0.0;
   __syncthreads();
   for (int base = 0; base < num_freq; base += 1024) {
     const int idx = base + threadIdx.x;
-    const double v = idx < num_freq ? static_cast<double>(area[idx]) : 0.0;
-    double incl = v;
-#pragma unroll
-    for (int o = 1; o < 32; o <<= 1) {
-      const double y = __shfl_up_sync(0xFFFFFFFFu, incl, o);
-      if (lane >= o) incl += y;
-    }
-    if (lane == 31) s_warp[warp] = incl;
-    __syncthreads();
-    if (warp == 0) {
-      const double w = s_warp[lane];
-      double wi = w;
-#pragma unroll
-      for (int o = 1; o < 32; o <<= 1) {
-        const double y = __shfl_up_sync(0xFFFFFFFFu, wi, o);
-        if (lane >= o) wi += y;
-      }
-      s_warp[lane] = wi - w;
-    }
-    __syncthreads();
-    const double total = s_carry + s_warp[warp] + incl;
+    double before, incl;
+    mse_tile_scan(area, base, num_freq, before, incl);
+    const double total = s_carry + before + incl;
     if (idx < num_freq) integral[num_freq - 1 - idx] = static_cast<float>(total);
     __syncthreads();
     if (threadIdx.x == 1023) s_carry = total;
