@@ -72,6 +72,11 @@ gf_status gf_mlp_gradients(gf_mlp* mlp, const float* d_inputs, const float* d_ta
 gf_status gf_mlp_train_step(gf_mlp* mlp, const float* d_inputs, const float* d_targets, int32_t batch,
                             float* d_loss);
 
+/* The same on rows d_rows[0 .. batch) (device, int64) of d_inputs and d_targets: a minibatch without a copy
+ * of it. */
+gf_status gf_mlp_train_step_rows(gf_mlp* mlp, const float* d_inputs, const float* d_targets, const int64_t* d_rows,
+                                 int32_t batch, float* d_loss);
+
 /* Kernel-fault word of the network's kernels (bounded waits that ran out); synchronous.  Returns
  * GF_ERR_DEVICE once per fault and clears the word; the network stays usable. */
 gf_status gf_mlp_check(gf_mlp* mlp);

@@ -1,6 +1,6 @@
 // SFS surrogate network on sm_100a tensor cores: a bf16 GEMM built on TMA + tcgen05 with the
-// accumulator in tensor memory, fused epilogues (bias + GELU forward, GELU' backward with bias
-// gradients, split-K weight-gradient partials), the loss, the gradient reduction and Adam.
+// accumulator in tensor memory, fused epilogues (bias + GELU forward, the loss and its gradient, GELU'
+// backward with bias gradients), and one kernel for the weight gradients of all layers and Adam.
 //
 // Every GEMM is C[M][N] = A[M][K] * B[N][K]^T with both operands K-contiguous:
 //   forward   Z_l  = Y_{l-1} W_l^T          A = Y_{l-1} [batch][in]      B = W_l   [out][in]
@@ -17,6 +17,7 @@
 #include <cuda_runtime.h>
 #include <cudaTypedefs.h>
 
+#include <algorithm>
 #include <atomic>
 #include <cmath>
 #include <cstdarg>
@@ -25,6 +26,7 @@
 #include <mutex>
 #include <new>
 #include <string>
+#include <utility>
 #include <vector>
 
 #include "gf_surrogate.h"
@@ -44,11 +46,11 @@ constexpr int MAX_SPLITS = 16;
 enum Epi : int {
   EPI_STORE_F32 = 0,     // C (fp32)
   EPI_FWD_GELU = 1,      // Z = acc + bias (fp32), Y = GELU(Z) (bf16) and Y^T (bf16)
-  EPI_FWD_LINEAR = 2,    // out = acc + bias (fp32)
   EPI_BWD_GELU = 3,      // dZ = acc * GELU'(Z) (bf16) and dZ^T (bf16), bias partials
-  EPI_PARTIAL = 4,       // split-K partial slice of C (fp32)
   EPI_FWD_GELU_INFER = 5,// Y = GELU(acc + bias) (bf16) only
-  EPI_FWD_OUT = 6        // out = acc + bias written straight to the caller's [rows][99] array
+  EPI_FWD_OUT = 6,       // out = acc + bias written straight to the caller's [rows][99] array
+  EPI_FWD_LOSS = 7       // dOut = 2 (acc + bias - target) / (rows * 99) (bf16) and dOut^T, the tile's column sums
+                         // of it (layer 5's bias gradient) and its loss
 };
 
 struct EpiArgs {
@@ -57,46 +59,67 @@ struct EpiArgs {
   long long ldz;
   float* bias_part;          // [M / 128][ld_bias_part] column sums of the backward output
   long long ld_bias_part;
-  int rows_per_split;        // row offset of split s in the partial-slice map (EPI_PARTIAL)
   float* out;                // caller's output [rows][out_cols] (EPI_FWD_OUT)
   int out_cols;
+  const float* target;       // [rows][99], row idx[i] for output row i where idx is given (EPI_FWD_LOSS)
+  const long long* idx;
+  float* loss_part;          // [M / 128] (EPI_FWD_LOSS)
+  int batch;
   int* fault;                // set when a bounded wait ran out
 };
 
-constexpr int EPI_WARPS = 8;                        // two per tensor-memory lane quarter
-constexpr int GEMM_THREADS = 64 + 32 * EPI_WARPS;   // TMA warp, MMA warp, 8 epilogue warps
+// Epilogue warps of an N tile: two per tensor-memory lane quarter, one where a quarter has a single 32-column
+// chunk.
+__host__ __device__ constexpr int epi_warps(int BN) { return BN >= 64 ? 8 : 4; }
+__host__ __device__ constexpr int gemm_threads(int BN) { return 64 + 32 * epi_warps(BN); }   // TMA warp, MMA warp, epilogue warps
+
+// Programmatic dependent launch: a training step's kernels follow one another on one stream, and each may set
+// up its barriers and tensor memory while the one before it still runs, then waits here for its results.
+// (Without the launch attribute both are no-ops.)
+__device__ __forceinline__ void grid_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+__device__ __forceinline__ void grid_launch_next() { asm volatile("griddepcontrol.launch_dependents;"); }
 constexpr int SMEM_LIMIT = 232448;                  // dynamic shared memory per CTA on sm_100
 
 // Per-epilogue-warp staging of one 32 x 32 output chunk, double-buffered: fp32 rows with the 128-byte
 // swizzle, bf16 rows with the 64-byte swizzle, bf16 transposed rows unswizzled -- the layouts the
 // output tensor maps expect, and conflict-free for the row-per-lane writes.  Only the outputs the
 // epilogue writes get space.
-template <int EPI>
+template <int BN, int EPI>
 struct Stage {
-  static constexpr bool F32 = EPI == EPI_STORE_F32 || EPI == EPI_PARTIAL || EPI == EPI_FWD_LINEAR || EPI == EPI_FWD_GELU;
-  static constexpr bool BF16 = EPI == EPI_FWD_GELU || EPI == EPI_FWD_GELU_INFER || EPI == EPI_BWD_GELU;
-  static constexpr bool T = EPI == EPI_FWD_GELU || EPI == EPI_BWD_GELU;
+  static constexpr bool F32 = EPI == EPI_STORE_F32 || EPI == EPI_FWD_GELU;
+  static constexpr bool BF16 = EPI == EPI_FWD_GELU || EPI == EPI_FWD_GELU_INFER || EPI == EPI_BWD_GELU ||
+                               EPI == EPI_FWD_LOSS;
+  static constexpr bool T = EPI == EPI_FWD_GELU || EPI == EPI_BWD_GELU || EPI == EPI_FWD_LOSS;
+  static constexpr int BUFFERS = BN >= 128 ? 2 : 1;   // a warp has one chunk per tile below that
   static constexpr int F32_OFF = 0;
   static constexpr int BF16_OFF = F32 ? 4096 : 0;
   static constexpr int T_OFF = BF16_OFF + (BF16 ? 2048 : 0);
   static constexpr int BUF = ((T_OFF + (T ? 2048 : 0)) + 1023) / 1024 * 1024;
-  static constexpr int WARP = 2 * BUF;
+  static constexpr int WARP = BUFFERS * BUF;
 };
 
 template <int BN, int EPI>
 struct Smem {
+  // narrow training tiles load two K blocks with one TMA box (a 3-D map of K blocks): half the loads, which is
+  // what their short K loops wait for (128-wide tiles have no room for it beside their staging)
+  static constexpr int KS = BN < 128 && (EPI == EPI_FWD_GELU || EPI == EPI_BWD_GELU) ? 2 : 1;
   static constexpr int A_BYTES = BM * BK * 2;
   static constexpr int B_BYTES = BN * BK * 2;
-  static constexpr int STAGE_BYTES = A_BYTES + B_BYTES;
+  static constexpr int STAGE_BYTES = KS * (A_BYTES + B_BYTES);
   static constexpr int BIAS_FLOATS = 512;   // the bias vector of the whole output width
   // EPI_FWD_OUT stages a whole 128-row tile of the caller's [rows][99] output (one contiguous span)
-  static constexpr int OUT_TILE = EPI == EPI_FWD_OUT ? (BM * GF_MLP_OUTPUTS * 4 + 1023) / 1024 * 1024 : 0;
-  static constexpr int EXTRA = EPI_WARPS * Stage<EPI>::WARP + OUT_TILE + 256 + 2 * 4 * 32 * 4 + 4 * BIAS_FLOATS + 1024;
-  static constexpr int STAGES = (4 * STAGE_BYTES + EXTRA <= SMEM_LIMIT)   ? 4
+  // EPI_FWD_LOSS keeps a tile's targets, then its residuals, in rows of 99 floats
+  static constexpr int OUT_TILE =
+      EPI == EPI_FWD_OUT || EPI == EPI_FWD_LOSS ? (BM * GF_MLP_OUTPUTS * 4 + 1023) / 1024 * 1024 : 0;
+  static constexpr int STAGING = epi_warps(BN) * Stage<BN, EPI>::WARP;
+  static constexpr int EXTRA = STAGING + OUT_TILE + 256 + 2 * 4 * 32 * 4 + 4 * BIAS_FLOATS + 1024;
+  // narrow tiles: two stages of two blocks, so that the next kernel's CTA fits beside this one's
+  static constexpr int STAGES = BN == 32                                  ? 2
+                                : (4 * STAGE_BYTES + EXTRA <= SMEM_LIMIT) ? 4
                                 : (3 * STAGE_BYTES + EXTRA <= SMEM_LIMIT) ? 3
                                                                           : 2;
   static constexpr int STG_OFFSET = STAGES * STAGE_BYTES;
-  static constexpr int BAR_OFFSET = STG_OFFSET + EPI_WARPS * Stage<EPI>::WARP + OUT_TILE;
+  static constexpr int BAR_OFFSET = STG_OFFSET + STAGING + OUT_TILE;
   static constexpr int OUT_OFFSET = BAR_OFFSET - OUT_TILE;
   static constexpr int BIAS_OFFSET = BAR_OFFSET + 256 + 2 * 4 * 32 * 4;
   static constexpr int BYTES = BIAS_OFFSET + 4 * BIAS_FLOATS + 1024;   // + barriers, reductions, bias, alignment
@@ -156,20 +179,20 @@ __device__ __forceinline__ void stage_bf16_col(uint8_t* buf, int r, const float*
   for (int j = 0; j < 32; ++j) *reinterpret_cast<__nv_bfloat16*>(buf + j * 64 + 2 * r) = __float2bfloat16_rn(v[j]);
 }
 
-// Persistent tensor-core GEMM: CTAs stride over 128 x BN output tiles (N fastest, then M, then the
-// K split).  Warp 0 streams A/B K-blocks with TMA into a 4-stage ring, warp 1 issues tcgen05 MMAs
+// Persistent tensor-core GEMM: CTAs stride over 128 x BN output tiles (N fastest, then M).  Warp 0 streams A/B K-blocks with TMA into a 4-stage ring, warp 1 issues tcgen05 MMAs
 // into one of two tensor-memory accumulators, warps 2-5 drain the other accumulator through the
 // epilogue (tcgen05.ld -> registers -> swizzled shared staging -> TMA store), so a tile's epilogue
 // overlaps the next tile's MMAs.
 template <int BN, int EPI>
-__global__ void __launch_bounds__(GEMM_THREADS, 1)
+__global__ void __launch_bounds__(gemm_threads(BN), BN == 32 ? 2 : 1)   // 2: the next kernel's CTA beside it
 umma_gemm_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constant__ CUtensorMap tma_b,
                  const __grid_constant__ CUtensorMap tma_c, const __grid_constant__ CUtensorMap tma_y,
-                 const __grid_constant__ CUtensorMap tma_yt, int m_tiles, int n_tiles, int splits, int k_blocks,
-                 EpiArgs ep, long long wait_limit, int inject) {
+                 const __grid_constant__ CUtensorMap tma_yt, int m_tiles, int n_tiles, int k_blocks, EpiArgs ep,
+                 long long wait_limit, int inject) {
   using L = Smem<BN, EPI>;
-  using SG = Stage<EPI>;
+  using SG = Stage<BN, EPI>;
   constexpr int STAGES = L::STAGES;
+  constexpr int EPI_WARPS = epi_warps(BN);
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
   uint64_t* full = reinterpret_cast<uint64_t*>(smem + L::BAR_OFFSET);
@@ -184,11 +207,11 @@ umma_gemm_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constan
   float* red = reinterpret_cast<float*>(smem + L::BAR_OFFSET + 256);   // [2 halves][4 quarters][32]
   float* s_bias = reinterpret_cast<float*>(smem + L::BIAS_OFFSET);
   volatile int* abort_flag = timed_out;
-  constexpr bool HAS_BIAS = EPI == EPI_FWD_GELU || EPI == EPI_FWD_GELU_INFER || EPI == EPI_FWD_LINEAR ||
-                            EPI == EPI_FWD_OUT;
+  constexpr bool HAS_BIAS = EPI == EPI_FWD_GELU || EPI == EPI_FWD_GELU_INFER || EPI == EPI_FWD_OUT ||
+                            EPI == EPI_FWD_LOSS;
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int tiles = m_tiles * n_tiles * splits;
+  const int tiles = m_tiles * n_tiles;
   // Bounded waits.  The producer and MMA threads stop issuing work as soon as any wait of the CTA has
   // run out (`wait`); the epilogue warps wait on the barrier alone and then agree on the outcome, so
   // all of them leave the tile loop together.  An aborted CTA never touches unsynchronised data: it
@@ -224,11 +247,13 @@ umma_gemm_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constan
     *consumed_s = 0;
     mbar_fence_init();
   }
+  __syncwarp();
+  if (warp == 1) tmem_alloc(tmem_slot, 2 * BN);
+  grid_launch_next();
+  grid_wait();   // from here on: what the kernels before this one wrote
   if constexpr (HAS_BIAS) {
     for (int i = threadIdx.x; i < n_tiles * BN && i < L::BIAS_FLOATS; i += blockDim.x) s_bias[i] = ep.bias[i];
   }
-  __syncwarp();
-  if (warp == 1) tmem_alloc(tmem_slot, 2 * BN);
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
@@ -240,11 +265,8 @@ umma_gemm_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constan
     if (lane == 0) {
       int it = 0;
       for (int tile = blockIdx.x; tile < tiles; tile += gridDim.x) {
-        const int nt = tile % n_tiles;
-        const int rest = tile / n_tiles;
-        const int mt = rest % m_tiles;
-        const int sp = rest / m_tiles;
-        for (int kb = 0; kb < k_blocks; ++kb, ++it) {
+        const int nt = tile % n_tiles, mt = tile / n_tiles;
+        for (int kb = 0; kb < k_blocks; kb += L::KS, ++it) {
           const int s = it % STAGES;
           const uint32_t ph = (it / STAGES) & 1;
           if (!wait(&empty[s], ph ^ 1)) {
@@ -252,10 +274,15 @@ umma_gemm_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constan
             goto producer_done;
           }
           uint8_t* a = smem + s * L::STAGE_BYTES;
-          mbar_arrive_expect_tx(&full[s], L::STAGE_BYTES);
-          const int kx = (sp * k_blocks + kb) * BK;
-          tma_load_2d(a, &tma_a, kx, mt * BM, &full[s]);
-          tma_load_2d(a + L::A_BYTES, &tma_b, kx, nt * BN, &full[s]);
+          if constexpr (L::KS == 1) {
+            mbar_arrive_expect_tx(&full[s], L::STAGE_BYTES);
+            tma_load_2d(a, &tma_a, kb * BK, mt * BM, &full[s]);
+            tma_load_2d(a + L::A_BYTES, &tma_b, kb * BK, nt * BN, &full[s]);
+          } else {   // the maps' boxes hold min(KS, k_blocks) K blocks
+            mbar_arrive_expect_tx(&full[s], min(L::KS, k_blocks) * (L::A_BYTES + L::B_BYTES));
+            tma_load_3d(a, &tma_a, 0, mt * BM, kb, &full[s]);
+            tma_load_3d(a + L::KS * L::A_BYTES, &tma_b, 0, nt * BN, kb, &full[s]);
+          }
         }
       }
     producer_done:
@@ -276,7 +303,7 @@ umma_gemm_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constan
         tc_fence_after();
         const uint32_t d = tmem + static_cast<uint32_t>(acc * BN);
         bool stop = false;
-        for (int kb = 0; kb < k_blocks; ++kb, ++it) {
+        for (int kb = 0; kb < k_blocks; kb += L::KS, ++it) {
           const int s = it % STAGES;
           const uint32_t ph = (it / STAGES) & 1;
           if (!wait(&full[s], ph)) {
@@ -285,12 +312,16 @@ umma_gemm_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constan
             break;
           }
           tc_fence_after();
-          const uint32_t a_addr = smem_u32(smem + s * L::STAGE_BYTES);
-          const uint32_t b_addr = a_addr + L::A_BYTES;
+          const uint32_t stage = smem_u32(smem + s * L::STAGE_BYTES);
 #pragma unroll
-          for (int kk = 0; kk < BK / 16; ++kk)
-            umma_bf16(d, sw128_kmajor_desc(a_addr + kk * 32), sw128_kmajor_desc(b_addr + kk * 32), idesc,
-                      (kb | kk) != 0);
+          for (int h = 0; h < L::KS; ++h) {
+            if (kb + h >= k_blocks) break;
+            const uint32_t a_addr = stage + h * L::A_BYTES, b_addr = stage + L::KS * L::A_BYTES + h * L::B_BYTES;
+#pragma unroll
+            for (int kk = 0; kk < BK / 16; ++kk)
+              umma_bf16(d, sw128_kmajor_desc(a_addr + kk * 32), sw128_kmajor_desc(b_addr + kk * 32), idesc,
+                        (kb | h | kk) != 0);
+          }
           umma_commit(&empty[s]);
         }
         if (stop) break;
@@ -307,14 +338,35 @@ umma_gemm_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constan
     const int ew = warp - 2;
     const int half = ew >> 2;
     uint8_t* stg = smem + L::STG_OFFSET + ew * SG::WARP;
+    // the forward pre-activations of 32 columns of a row (EPI_BWD_GELU), read while the MMAs run where the warp
+    // has a single chunk per tile
+    float4 z[EPI == EPI_BWD_GELU ? 8 : 1];
+    auto load_z = [&](float4* to, int r, int n) {
+      const float4* zp = reinterpret_cast<const float4*>(ep.z + static_cast<long long>(r) * ep.ldz + n);
+#pragma unroll
+      for (int q = 0; q < 8; ++q) to[q] = __ldg(zp + q);
+    };
     int chunk = 0, local = 0;
     for (int tile = blockIdx.x; tile < tiles; tile += gridDim.x, ++local) {
-      const int nt = tile % n_tiles;
-      const int rest = tile / n_tiles;
-      const int mt = rest % m_tiles;
-      const int sp = rest / m_tiles;
+      const int nt = tile % n_tiles, mt = tile / n_tiles;
       const int acc = local & 1;
       const uint32_t use = static_cast<uint32_t>(local >> 1);
+      if constexpr (EPI == EPI_BWD_GELU && SG::BUFFERS == 1) load_z(z, mt * BM + qd * 32 + lane, nt * BN + 32 * half);
+      if constexpr (EPI == EPI_FWD_LOSS) {
+        // the tile's targets, coalesced row by row, while its MMAs run (the barrier below orders them); a lane
+        // holds one of the warp's row indices, so that the rows' loads do not wait for one another
+        constexpr int ROWS = BM / EPI_WARPS;
+        float* s_t = reinterpret_cast<float*>(smem + L::OUT_OFFSET) + ew * ROWS * GF_MLP_OUTPUTS;
+        const long long r0 = static_cast<long long>(mt) * BM + ew * ROWS;
+        const long long mine = lane < ROWS ? (ep.idx ? ep.idx[r0 + lane] : r0 + lane) : 0;
+#pragma unroll 8
+        for (int r = 0; r < ROWS; ++r) {
+          const float* from = ep.target + __shfl_sync(0xffffffffu, mine, r) * GF_MLP_OUTPUTS;
+#pragma unroll
+          for (int j = 0; j < 4; ++j)
+            if (32 * j + lane < GF_MLP_OUTPUTS) s_t[r * GF_MLP_OUTPUTS + 32 * j + lane] = __ldg(from + 32 * j + lane);
+        }
+      }
       if (lane == 0 && !mbar_wait(&tfull[acc], use & 1, wait_limit)) atomicOr(epi_fail, 1);
       named_barrier_sync(4, 32 * EPI_WARPS);     // every epilogue warp has its verdict in epi_fail
       if (*reinterpret_cast<volatile int*>(epi_fail)) {
@@ -335,16 +387,12 @@ umma_gemm_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constan
 #pragma unroll 1
       for (int c0 = 32 * half; c0 < BN; c0 += 64, ++chunk) {
         const int n = nt * BN + c0;
-        uint8_t* buf = stg + (chunk & 1) * SG::BUF;
-        if (lane == 0) bulk_wait_read<1>();     // the store that last used this buffer has read it
+        uint8_t* buf = stg + (chunk % SG::BUFFERS) * SG::BUF;
+        if (lane == 0) bulk_wait_read<SG::BUFFERS - 1>();     // the store that last used this buffer has read it
         __syncwarp();
         float v[32];
         tmem_ld_32cols(tbase + c0, v);
-        if constexpr (EPI == EPI_STORE_F32 || EPI == EPI_PARTIAL) {
-          stage_f32_row(buf + SG::F32_OFF, lane, v);
-        } else if constexpr (EPI == EPI_FWD_LINEAR) {
-#pragma unroll
-          for (int j = 0; j < 32; ++j) v[j] += s_bias[n + j];
+        if constexpr (EPI == EPI_STORE_F32) {
           stage_f32_row(buf + SG::F32_OFF, lane, v);
         } else if constexpr (EPI == EPI_FWD_OUT) {
           // row stride 99 words: lanes (rows) hit distinct banks
@@ -360,28 +408,48 @@ umma_gemm_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constan
           for (int j = 0; j < 32; ++j) v[j] = gelu(v[j]);
           stage_bf16_row(buf + SG::BF16_OFF, lane, v);
           if constexpr (EPI == EPI_FWD_GELU) stage_bf16_col(buf + SG::T_OFF, lane, v);
+        } else if constexpr (EPI == EPI_FWD_LOSS) {
+          const float scale = 2.f / (static_cast<float>(ep.batch) * GF_MLP_OUTPUTS);
+          float* d = s_out + (qd * 32 + lane) * GF_MLP_OUTPUTS;   // targets in, residuals out
+#pragma unroll
+          for (int j = 0; j < 32; ++j) {
+            if (n + j < GF_MLP_OUTPUTS) {
+              const float r = v[j] + s_bias[n + j] - d[n + j];
+              d[n + j] = r;
+              v[j] = scale * r;
+            } else {
+              v[j] = 0.f;
+            }
+          }
+          stage_bf16_row(buf + SG::BF16_OFF, lane, v);
+          stage_bf16_col(buf + SG::T_OFF, lane, v);
         } else if constexpr (EPI == EPI_BWD_GELU) {
-          const float4* zp = reinterpret_cast<const float4*>(ep.z + static_cast<long long>(row) * ep.ldz + n);
+          if constexpr (SG::BUFFERS > 1) load_z(z, row, n);
 #pragma unroll
           for (int q = 0; q < 8; ++q) {
-            const float4 z = __ldg(zp + q);
-            v[4 * q] *= gelu_grad(z.x);
-            v[4 * q + 1] *= gelu_grad(z.y);
-            v[4 * q + 2] *= gelu_grad(z.z);
-            v[4 * q + 3] *= gelu_grad(z.w);
+            v[4 * q] *= gelu_grad(z[q].x);
+            v[4 * q + 1] *= gelu_grad(z[q].y);
+            v[4 * q + 2] *= gelu_grad(z[q].z);
+            v[4 * q + 3] *= gelu_grad(z[q].w);
           }
           stage_bf16_row(buf + SG::BF16_OFF, lane, v);
           stage_bf16_col(buf + SG::T_OFF, lane, v);
           // column sums over the tile's 128 rows (fixed order: lanes, then quarters 0..3); the four
           // warps of a half work on the same chunk and meet at their own named barrier
-          float mine = 0.f;
+          // lanes: the sums of a butterfly over all 32 columns, but each step keeps only the half of the columns
+          // that this lane's bit selects and sends the other (31 shuffles in place of 160), so lane j ends with
+          // column j
 #pragma unroll
-          for (int j = 0; j < 32; ++j) {
-            float t = v[j];
+          for (int o = 16; o > 0; o >>= 1) {
+            const bool upper = (lane & o) != 0;
 #pragma unroll
-            for (int o = 16; o > 0; o >>= 1) t += __shfl_xor_sync(0xffffffffu, t, o);
-            if (lane == j) mine = t;
+            for (int j = 0; j < 16; ++j) {
+              if (j >= o) break;
+              const float keep = upper ? v[j + o] : v[j], send = upper ? v[j] : v[j + o];
+              v[j] = keep + __shfl_xor_sync(0xffffffffu, send, o);
+            }
           }
+          const float mine = v[0];
           float* rh = red + half * 128;
           rh[qd * 32 + lane] = mine;
           named_barrier_sync(1 + half, 128);
@@ -395,11 +463,7 @@ umma_gemm_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constan
         fence_proxy_async_smem();
         __syncwarp();
         if (lane == 0) {
-          if constexpr (EPI == EPI_STORE_F32 || EPI == EPI_FWD_LINEAR || EPI == EPI_FWD_GELU) {
-            tma_store_2d(&tma_c, n, row0, buf + SG::F32_OFF);
-          } else if constexpr (EPI == EPI_PARTIAL) {
-            tma_store_2d(&tma_c, n, sp * ep.rows_per_split + row0, buf + SG::F32_OFF);
-          }
+          if constexpr (SG::F32) tma_store_2d(&tma_c, n, row0, buf + SG::F32_OFF);
           if constexpr (SG::BF16) tma_store_2d(&tma_y, n, row0, buf + SG::BF16_OFF);
           if constexpr (SG::T) tma_store_2d(&tma_yt, row0, n, buf + SG::T_OFF);
           bulk_commit();
@@ -413,6 +477,33 @@ umma_gemm_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constan
           bulk_store_1d(ep.out + static_cast<long long>(mt) * BM * GF_MLP_OUTPUTS, s_out, BM * GF_MLP_OUTPUTS * 4);
           bulk_commit();
         }
+      }
+      if constexpr (EPI == EPI_FWD_LOSS) {
+        // sums over the tile in a fixed order: a column's rows 0 .. 127, a row's columns, then the rows
+        named_barrier_sync(3, 32 * EPI_WARPS);   // every residual is in place
+        const int et = threadIdx.x - 64;
+        if (et < BM) {
+          float l = 0.f;
+          const float* d = s_out + et * GF_MLP_OUTPUTS;
+#pragma unroll 11
+          for (int j = 0; j < GF_MLP_OUTPUTS; ++j) l += d[j] * d[j];
+          red[et] = l;
+        } else if (et - BM < GF_MLP_OUTPUTS) {
+          const float scale = 2.f / (static_cast<float>(ep.batch) * GF_MLP_OUTPUTS);
+          const int j = et - BM;
+          float t = 0.f;
+#pragma unroll 16
+          for (int i = 0; i < BM; ++i) t += scale * s_out[i * GF_MLP_OUTPUTS + j];
+          ep.bias_part[mt * ep.ld_bias_part + j] = t;
+        }
+        named_barrier_sync(3, 32 * EPI_WARPS);
+        if (et == 0) {
+          float t = 0.f;
+#pragma unroll 16
+          for (int i = 0; i < BM; ++i) t += red[i];
+          ep.loss_part[mt] = t / (static_cast<float>(ep.batch) * GF_MLP_OUTPUTS);
+        }
+        named_barrier_sync(3, 32 * EPI_WARPS);   // before the next tile's targets
       }
       tc_fence_before();
       __syncwarp();
@@ -854,15 +945,19 @@ fused_forward_kernel(const __grid_constant__ CUtensorMap tma_x, const __grid_con
 // small kernels
 // ---------------------------------------------------------------------------------------------
 
-// Inputs [batch][6] fp32 -> X0 [cap][64] bf16 (one 16-byte store of columns 0..7 per row; columns
+// Inputs [batch][6] fp32 (row idx[i] for batch row i where idx is given) -> X0 [cap][64] bf16 (one 16-byte store of columns 0..7 per row; columns
 // 8..63 stay zero) and, for training, X0^T [64][cap].
-__global__ void encode_inputs_kernel(const float* __restrict__ x, int batch, __nv_bfloat16* __restrict__ x0,
-                                     __nv_bfloat16* __restrict__ x0t, long long cap, int transposed) {
+__global__ void encode_inputs_kernel(const float* __restrict__ x, const long long* __restrict__ idx, int batch,
+                                     __nv_bfloat16* __restrict__ x0, __nv_bfloat16* __restrict__ x0t, long long cap,
+                                     int transposed) {
   const int b = blockIdx.x * blockDim.x + threadIdx.x;
+  grid_launch_next();
+  grid_wait();   // the kernels before this one have read X0
   if (b >= batch) return;
+  const long long from = idx ? idx[b] : b;
   float v[8];
 #pragma unroll
-  for (int j = 0; j < GF_MLP_INPUTS; ++j) v[j] = x[b * GF_MLP_INPUTS + j];
+  for (int j = 0; j < GF_MLP_INPUTS; ++j) v[j] = x[from * GF_MLP_INPUTS + j];
   v[6] = 0.f;
   v[7] = 0.f;
   uint32_t w[4];
@@ -878,112 +973,326 @@ __global__ void encode_inputs_kernel(const float* __restrict__ x, int batch, __n
   }
 }
 
-// Squared-error loss of one 128-row tile and its gradient: dOut = 2 (out - target) / (batch * 99),
-// written row-major and transposed in bf16, with the tile's column sums (bias gradient of layer 5)
-// and loss sum.  One block of 128 threads per tile; thread = row for the gradient, thread = column
-// for the column sums (recomputed, same expression, fixed row order).
-__global__ void __launch_bounds__(128)
-loss_kernel(const float* __restrict__ out, const float* __restrict__ target, int batch,
-            __nv_bfloat16* __restrict__ dout, __nv_bfloat16* __restrict__ doutt, long long cap,
-            float* __restrict__ bias_part, float* __restrict__ loss_part) {
-  __shared__ float rl[BM];
-  const int r = threadIdx.x;
-  const int row0 = blockIdx.x * BM;
-  const int row = row0 + r;
-  const float scale = 2.f / (static_cast<float>(batch) * GF_MLP_OUTPUTS);
-  float l = 0.f;
-  for (int j = 0; j < GF_MLP_OUTPUTS; ++j) {
-    const float d = out[row * OUT_PAD + j] - target[row * GF_MLP_OUTPUTS + j];
-    l += d * d;
-    const __nv_bfloat16 b = __float2bfloat16_rn(scale * d);
-    dout[row * OUT_PAD + j] = b;
-    doutt[j * cap + row] = b;
+// ---------------------------------------------------------------------------------------------
+// The end of a training step: the weight gradients of all layers, then Adam, in one launch
+// ---------------------------------------------------------------------------------------------
+// dW_l = dZ_l^T Y_{l-1} has few output tiles (104 of 128 x 64 over the five layers) and the batch as its
+// reduction dimension.  A CTA owns one tile of one layer: the batch is cut into `splits` parts, each
+// accumulated on its own in one of two tensor-memory accumulators and added up in registers in order (the
+// sum, rounding included, of gradient slices reduced in a fixed order), and the tile's master weights,
+// moments and bf16 copies are updated from the registers.  The gradient itself is only written where the
+// caller asked for it.  Further blocks do the biases (partials summed in tile order) and the loss.
+//
+// At a batch of 1,024 the five GEMMs, their reduction over 27 MB of slices and Adam took 29 + 10 + 17 us in seven
+// launches; here they take 13 us.
+constexpr int DW_BN = 64;
+constexpr int DW_EPI_WARPS = 8;
+constexpr int DW_THREADS = 64 + 32 * DW_EPI_WARPS;
+constexpr int DW_KS = 2;   // K blocks a stage, one TMA box each for A and B (batches are a multiple of 128 rows)
+constexpr int DW_STAGES = 4;
+constexpr int DW_A_BYTES = BM * BK * 2, DW_B_BYTES = DW_BN * BK * 2;
+constexpr int DW_STAGE_BYTES = DW_KS * (DW_A_BYTES + DW_B_BYTES);
+constexpr int DW_BAR_OFFSET = DW_STAGES * DW_STAGE_BYTES;
+constexpr int DW_PIECE_ROW = 36;    // floats: rows 16 bytes apart modulo 128
+constexpr int DW_TPIECE_ROW = 34;   // bf16
+static_assert(DW_EPI_WARPS * 32 * (4 * DW_PIECE_ROW + 2 * DW_TPIECE_ROW) <= DW_BAR_OFFSET, "the pieces fit in the ring");
+constexpr int DW_SMEM = DW_BAR_OFFSET + 256 + 1024;   // + barriers and flags, alignment
+
+struct AdamArgs {
+  float lr, beta1, beta2, eps, bc1, bc2, decay;
+};
+
+// Adam (with optional decoupled weight decay) of one master value.
+__device__ __forceinline__ float adam_update(float w, float& m_io, float& v_io, float g, const AdamArgs& a) {
+  // the products contracted as one kernel over all parameters had them, spelled out
+  const float m = __fmaf_rn(1.f - a.beta1, g, __fmul_rn(a.beta1, m_io));
+  const float v = __fmaf_rn(__fmul_rn(1.f - a.beta2, g), g, __fmul_rn(a.beta2, v_io));
+  m_io = m;
+  v_io = v;
+  w -= a.lr * a.decay * w;
+  w -= a.lr * (m / a.bc1) / (sqrtf(v / a.bc2) + a.eps);
+  return w;
+}
+
+struct DwLayer {
+  CUtensorMap a, b;        // dZ^T [out][batch], Y^T [in][batch]
+  float *w, *m, *v, *g;    // [rows][cols]
+  __nv_bfloat16 *wb, *wt;  // [rows][cols], [cols][rows]
+  float *bias, *bm, *bv, *bg;
+  const float* bias_part;  // [batch / 128][rows]
+  int rows, cols, rows_true, cols_true;
+  int splits;              // of the batch's K blocks
+  int first;               // the layer's first tile in the grid
+};
+
+struct DwArgs {
+  DwLayer layer[GF_MLP_LAYERS];
+  AdamArgs adam;
+  int tiles, k_blocks;     // tiles of all layers; 64-row K blocks of the batch
+  int update;              // 1: Adam; 0: write the gradients
+  int batch_tiles;
+  const float* loss_part;
+  float *loss, *loss_out;  // loss_out: the caller's, may be null
+  int* fault;
+  long long wait_limit;
+};
+
+__global__ void __launch_bounds__(DW_THREADS, 1) weight_update_kernel(const __grid_constant__ DwArgs A) {
+  extern __shared__ uint8_t smem_raw[];
+  uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
+  if (static_cast<int>(blockIdx.x) >= A.tiles) {   // block-uniform: biases and loss
+    grid_launch_next();
+    grid_wait();
+    int i = (static_cast<int>(blockIdx.x) - A.tiles) * DW_THREADS + threadIdx.x;
+    if (i == 0) {
+      float s = 0.f;
+      for (int t = 0; t < A.batch_tiles; ++t) s += A.loss_part[t];
+      *A.loss = s;
+      if (A.loss_out) *A.loss_out = s;
+    }
+    int l = 0;
+    while (l < GF_MLP_LAYERS && i >= A.layer[l].rows) i -= A.layer[l++].rows;
+    if (l == GF_MLP_LAYERS || i >= A.layer[l].rows_true) return;
+    const DwLayer& L = A.layer[l];
+    float g = 0.f;
+    for (int t = 0; t < A.batch_tiles; ++t) g += L.bias_part[t * L.rows + i];
+    if (A.update) {
+      float m = L.bm[i], v = L.bv[i];
+      L.bias[i] = adam_update(L.bias[i], m, v, g, A.adam);
+      L.bm[i] = m;
+      L.bv[i] = v;
+    } else {
+      L.bg[i] = g;
+    }
+    return;
   }
-  rl[r] = l;
-  if (r < GF_MLP_OUTPUTS) {
-    float s = 0.f;
-    for (int i = 0; i < BM; ++i) s += scale * (out[(row0 + i) * OUT_PAD + r] - target[(row0 + i) * GF_MLP_OUTPUTS + r]);
-    bias_part[blockIdx.x * OUT_PAD + r] = s;
+  int l = 0;
+  while (l + 1 < GF_MLP_LAYERS && static_cast<int>(blockIdx.x) >= A.layer[l + 1].first) ++l;
+  const DwLayer& L = A.layer[l];
+  const int n_tiles = L.cols / DW_BN;
+  const int tile = static_cast<int>(blockIdx.x) - L.first;
+  const int nt = tile % n_tiles, mt = tile / n_tiles;
+  const int per_split = A.k_blocks / L.splits;
+
+  uint64_t* full = reinterpret_cast<uint64_t*>(smem + DW_BAR_OFFSET);
+  uint64_t* empty = full + DW_STAGES;
+  uint64_t* tfull = empty + DW_STAGES;
+  uint64_t* tempty = tfull + 2;
+  uint64_t* drain = tempty + 2;
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(drain + 1);
+  int* timed_out = reinterpret_cast<int*>(tmem_slot + 1);
+  int* epi_fail = timed_out + 1;
+  int* consumed_s = timed_out + 2;
+  volatile int* abort_flag = timed_out;
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  auto wait = [&](uint64_t* bar, uint32_t parity) -> bool {   // as in umma_gemm_kernel
+    if (*abort_flag) return false;
+    const uint32_t addr = smem_u32(bar);
+    const long long t0 = clock64();
+    while (!mbar_try_wait(addr, parity)) {
+      if (*abort_flag) return false;
+      if (clock64() - t0 > A.wait_limit) {
+        *abort_flag = 1;
+        return false;
+      }
+    }
+    return true;
+  };
+  if (threadIdx.x == 0) {
+    tma_prefetch_desc(&L.a);
+    tma_prefetch_desc(&L.b);
+    for (int s = 0; s < DW_STAGES; ++s) {
+      mbar_init(&full[s], 1);
+      mbar_init(&empty[s], 1);
+    }
+    for (int a = 0; a < 2; ++a) {
+      mbar_init(&tfull[a], 1);
+      mbar_init(&tempty[a], DW_EPI_WARPS);
+    }
+    mbar_init(drain, 1);
+    timed_out[0] = timed_out[1] = timed_out[2] = 0;
+    mbar_fence_init();
   }
+  __syncwarp();
+  if (warp == 1) tmem_alloc(tmem_slot, 2 * DW_BN);
+  grid_launch_next();
+  grid_wait();
+  tc_fence_before();
   __syncthreads();
-  if (r == 0) {
-    float s = 0.f;
-    for (int i = 0; i < BM; ++i) s += rl[i];
-    loss_part[blockIdx.x] = s / (static_cast<float>(batch) * GF_MLP_OUTPUTS);
+  tc_fence_after();
+  const uint32_t tmem = *tmem_slot;
+  bool late = false;
+  int issued = 0;
+
+  if (warp == 0) {
+    if (lane == 0) {
+      int it = 0;
+      for (; it < A.k_blocks / DW_KS; ++it) {
+        const int s = it % DW_STAGES;
+        if (!wait(&empty[s], ((it / DW_STAGES) & 1) ^ 1)) {
+          late = true;
+          break;
+        }
+        uint8_t* a = smem + s * DW_STAGE_BYTES;
+        mbar_arrive_expect_tx(&full[s], DW_STAGE_BYTES);
+        tma_load_3d(a, &L.a, 0, mt * BM, it * DW_KS, &full[s]);
+        tma_load_3d(a + DW_KS * DW_A_BYTES, &L.b, 0, nt * DW_BN, it * DW_KS, &full[s]);
+      }
+      issued = it;
+    }
+    __syncwarp();
+  } else if (warp == 1) {
+    if (lane == 0) {
+      constexpr uint32_t idesc = bf16_idesc(BM, DW_BN);
+      int blk = 0, received = 0;
+      for (int sp = 0; sp < L.splits && !late; ++sp) {
+        const int acc = sp & 1;
+        if (!wait(&tempty[acc], ((sp >> 1) & 1) ^ 1)) {
+          late = true;
+          break;
+        }
+        tc_fence_after();
+        for (int kb = 0; kb < per_split; ++kb, ++blk) {   // a split may end within a stage
+          const int it = blk / DW_KS, h = blk % DW_KS, s = it % DW_STAGES;
+          if (h == 0) {
+            if (!wait(&full[s], (it / DW_STAGES) & 1)) {
+              late = true;
+              break;
+            }
+            ++received;
+            tc_fence_after();
+          }
+          const uint32_t stage = smem_u32(smem + s * DW_STAGE_BYTES);
+          const uint32_t a_addr = stage + h * DW_A_BYTES, b_addr = stage + DW_KS * DW_A_BYTES + h * DW_B_BYTES;
+#pragma unroll
+          for (int kk = 0; kk < BK / 16; ++kk)
+            umma_bf16(tmem + acc * DW_BN, sw128_kmajor_desc(a_addr + kk * 32), sw128_kmajor_desc(b_addr + kk * 32), idesc,
+                      (kb | kk) != 0);
+          if (h == DW_KS - 1) umma_commit(&empty[s]);
+        }
+        if (!late) umma_commit(&tfull[acc]);
+      }
+      *consumed_s = received;
+    }
+    __syncwarp();
+  } else {
+    // epilogue warps: one 32 x 32 piece each (tensor-memory lane quarter, column half)
+    const int qd = warp & 3, half = (warp - 2) >> 2;
+    const int c0 = nt * DW_BN + 32 * half;
+    const uint32_t tbase = tmem + (static_cast<uint32_t>(qd * 32) << 16) + static_cast<uint32_t>(32 * half);
+    float g[32];
+#pragma unroll
+    for (int j = 0; j < 32; ++j) g[j] = 0.f;
+    for (int sp = 0; sp < L.splits; ++sp) {
+      const int acc = sp & 1;
+      if (lane == 0 && !mbar_wait(&tfull[acc], (sp >> 1) & 1, A.wait_limit)) atomicOr(epi_fail, 1);
+      named_barrier_sync(4, 32 * DW_EPI_WARPS);
+      if (*reinterpret_cast<volatile int*>(epi_fail)) {
+        late = true;
+        break;
+      }
+      __syncwarp();
+      tc_fence_after();
+      float v[32];
+      tmem_ld_32cols(tbase + acc * DW_BN, v);
+#pragma unroll
+      for (int j = 0; j < 32; ++j) g[j] += v[j];
+      tc_fence_before();
+      __syncwarp();
+      if (lane == 0) mbar_arrive(&tempty[acc]);
+    }
+    if (!late) {
+      // every MMA and load of the tile is done (the last hand-off), so the ring is free: the 32 x 32 piece goes
+      // through it, to be updated in rows of eight float4 (four rows a warp instruction, each 128 contiguous
+      // bytes of every array)
+      float* const piece = reinterpret_cast<float*>(smem) + (warp - 2) * 32 * DW_PIECE_ROW;
+      __nv_bfloat16* const tpiece = reinterpret_cast<__nv_bfloat16*>(smem + DW_EPI_WARPS * 32 * DW_PIECE_ROW * 4) +
+                                    (warp - 2) * 32 * DW_TPIECE_ROW;
+#pragma unroll
+      for (int q = 0; q < 8; ++q)
+        *reinterpret_cast<float4*>(piece + lane * DW_PIECE_ROW + 4 * q) =
+            make_float4(g[4 * q], g[4 * q + 1], g[4 * q + 2], g[4 * q + 3]);
+      __syncwarp();
+      const int row0 = mt * BM + qd * 32, c = 4 * (lane & 7);
+      const int valid = L.cols_true - c0 - c;   // of this lane's four columns
+      if (valid > 0) {
+#pragma unroll 4
+        for (int it = 0; it < 8; ++it) {
+          const int r = 4 * it + (lane >> 3);
+          if (row0 + r >= L.rows_true) continue;
+          const long long at = static_cast<long long>(row0 + r) * L.cols + c0 + c;
+          const float4 gv = *reinterpret_cast<const float4*>(piece + r * DW_PIECE_ROW + c);
+          if (!A.update) {   // columns past cols_true: their gradient is an exact zero
+            *reinterpret_cast<float4*>(L.g + at) = gv;
+            continue;
+          }
+          // columns past cols_true stay zero: zero weight, moments and gradient
+          float4 w = *reinterpret_cast<const float4*>(L.w + at);
+          float4 m = *reinterpret_cast<const float4*>(L.m + at);
+          float4 v = *reinterpret_cast<const float4*>(L.v + at);
+          w.x = adam_update(w.x, m.x, v.x, gv.x, A.adam);
+          w.y = adam_update(w.y, m.y, v.y, gv.y, A.adam);
+          w.z = adam_update(w.z, m.z, v.z, gv.z, A.adam);
+          w.w = adam_update(w.w, m.w, v.w, gv.w, A.adam);
+          *reinterpret_cast<float4*>(L.w + at) = w;
+          *reinterpret_cast<float4*>(L.m + at) = m;
+          *reinterpret_cast<float4*>(L.v + at) = v;
+          const __nv_bfloat16 b[4] = {__float2bfloat16_rn(w.x), __float2bfloat16_rn(w.y), __float2bfloat16_rn(w.z),
+                                      __float2bfloat16_rn(w.w)};
+          *reinterpret_cast<uint2*>(L.wb + at) =
+              make_uint2(static_cast<uint32_t>(__bfloat16_as_ushort(b[0])) | static_cast<uint32_t>(__bfloat16_as_ushort(b[1])) << 16,
+                         static_cast<uint32_t>(__bfloat16_as_ushort(b[2])) | static_cast<uint32_t>(__bfloat16_as_ushort(b[3])) << 16);
+#pragma unroll
+          for (int e = 0; e < 4; ++e) tpiece[(c + e) * DW_TPIECE_ROW + r] = b[e];
+        }
+      }
+      __syncwarp();
+      if (A.update) {   // the transposed copy: column c0 + j of the piece, a row a lane
+        const int rows = min(32, L.rows_true - row0), cols = min(32, L.cols_true - c0);
+        if (lane < rows) {
+#pragma unroll 8
+          for (int j = 0; j < cols; ++j)
+            L.wt[static_cast<long long>(c0 + j) * L.rows + row0 + lane] = tpiece[j * DW_TPIECE_ROW + lane];
+        }
+      }
+    }
   }
+
+  tc_fence_before();
+  if (late) *abort_flag = 1;
+  __syncthreads();
+  if (*abort_flag) {   // as in umma_gemm_kernel: what was issued lands before its memory is released
+    if (threadIdx.x == 0) {
+      for (int it = *consumed_s; it < issued; ++it) mbar_wait(&full[it % DW_STAGES], (it / DW_STAGES) & 1, A.wait_limit);
+      if (A.fault) atomicOr(A.fault, 1);
+    } else if (threadIdx.x == 32) {
+      umma_commit(drain);
+      mbar_wait(drain, 0, A.wait_limit);
+    }
+    __syncthreads();
+  }
+  if (warp == 1) tmem_dealloc(tmem, 2 * DW_BN);
 }
 
-__global__ void loss_finish_kernel(const float* __restrict__ loss_part, int tiles, float* __restrict__ loss) {
-  if (threadIdx.x == 0 && blockIdx.x == 0) {
-    float s = 0.f;
-    for (int i = 0; i < tiles; ++i) s += loss_part[i];
-    *loss = s;
-  }
-}
-
-// One parameter tensor (padded shape rows x cols) and where its gradient partials are.
+// One parameter tensor (padded shape rows x cols).
 struct ParamSlot {
   float* w;
-  float* m;
-  float* v;
-  float* g;
-  __nv_bfloat16* wb;     // bf16 copy [rows][cols] (weights only)
-  __nv_bfloat16* wt;     // bf16 transposed copy [cols][rows] (weights only)
-  const float* part;     // gradient partials
-  long long part_stride;
-  int nparts;
-  int rows, cols, rows_true, cols_true;
+  __nv_bfloat16* wb;     // bf16 copy [rows][cols]
+  __nv_bfloat16* wt;     // bf16 transposed copy [cols][rows]
+  int rows, cols;
   long long offset;      // first element in the concatenated index space
 };
 
 struct ParamTable {
-  ParamSlot s[2 * GF_MLP_LAYERS];
+  ParamSlot s[GF_MLP_LAYERS];
   long long total;
 };
 
 __device__ __forceinline__ int find_slot(const ParamTable& t, long long i) {
   int k = 0;
 #pragma unroll 1
-  while (k + 1 < 2 * GF_MLP_LAYERS && t.s[k + 1].offset <= i) ++k;
+  while (k + 1 < GF_MLP_LAYERS && t.s[k + 1].offset <= i) ++k;
   return k;
-}
-
-// g = sum of the partials in a fixed order.
-__global__ void reduce_grads_kernel(const __grid_constant__ ParamTable t) {
-  for (long long i = blockIdx.x * static_cast<long long>(blockDim.x) + threadIdx.x; i < t.total;
-       i += static_cast<long long>(gridDim.x) * blockDim.x) {
-    const ParamSlot& p = t.s[find_slot(t, i)];
-    const long long e = i - p.offset;
-    float acc = 0.f;
-    for (int k = 0; k < p.nparts; ++k) acc += p.part[k * p.part_stride + e];
-    p.g[e] = acc;
-  }
-}
-
-// Adam (with optional decoupled weight decay) on the master weights, then the bf16 copies.
-__global__ void adam_kernel(const __grid_constant__ ParamTable t, float lr, float beta1, float beta2, float eps,
-                            float bc1, float bc2, float decay) {
-  for (long long i = blockIdx.x * static_cast<long long>(blockDim.x) + threadIdx.x; i < t.total;
-       i += static_cast<long long>(gridDim.x) * blockDim.x) {
-    const ParamSlot& p = t.s[find_slot(t, i)];
-    const long long e = i - p.offset;
-    const int r = static_cast<int>(e / p.cols), c = static_cast<int>(e % p.cols);
-    if (r >= p.rows_true || c >= p.cols_true) continue;
-    const float g = p.g[e];
-    const float m = beta1 * p.m[e] + (1.f - beta1) * g;
-    const float v = beta2 * p.v[e] + (1.f - beta2) * g * g;
-    p.m[e] = m;
-    p.v[e] = v;
-    float w = p.w[e];
-    w -= lr * decay * w;
-    w -= lr * (m / bc1) / (sqrtf(v / bc2) + eps);
-    p.w[e] = w;
-    if (p.wb) {
-      const __nv_bfloat16 b = __float2bfloat16_rn(w);
-      p.wb[e] = b;
-      p.wt[static_cast<long long>(c) * p.rows + r] = b;
-    }
-  }
 }
 
 // bf16 copies of the master weights (after set_params).
@@ -991,7 +1300,6 @@ __global__ void refresh_bf16_kernel(const __grid_constant__ ParamTable t) {
   for (long long i = blockIdx.x * static_cast<long long>(blockDim.x) + threadIdx.x; i < t.total;
        i += static_cast<long long>(gridDim.x) * blockDim.x) {
     const ParamSlot& p = t.s[find_slot(t, i)];
-    if (!p.wb) continue;
     const long long e = i - p.offset;
     const int r = static_cast<int>(e / p.cols), c = static_cast<int>(e % p.cols);
     const __nv_bfloat16 b = __float2bfloat16_rn(p.w[e]);
@@ -1027,6 +1335,20 @@ bool make_map(CUtensorMap* m, const void* base, long long rows, long long cols, 
   cuuint32_t box[2] = {static_cast<cuuint32_t>(BK), static_cast<cuuint32_t>(box_rows)};
   cuuint32_t estr[2] = {1, 1};
   return fn(m, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, const_cast<void*>(base), dims, strides, box, estr,
+            CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
+            CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
+}
+
+// The same matrix as K blocks [cols / 64][rows][64], box `blocks` x box_rows x 64: a load lands as `blocks` tiles
+// one after the other.
+bool make_map_blocks(CUtensorMap* m, const void* base, long long rows, long long cols, int box_rows, int blocks) {
+  auto fn = encode_fn();
+  if (!fn) return false;
+  cuuint64_t dims[3] = {BK, static_cast<cuuint64_t>(rows), static_cast<cuuint64_t>(cols / BK)};
+  cuuint64_t strides[2] = {static_cast<cuuint64_t>(cols) * 2, BK * 2};
+  cuuint32_t box[3] = {BK, static_cast<cuuint32_t>(box_rows), static_cast<cuuint32_t>(blocks)};
+  cuuint32_t estr[3] = {1, 1, 1};
+  return fn(m, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 3, const_cast<void*>(base), dims, strides, box, estr,
             CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
             CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
 }
@@ -1068,27 +1390,70 @@ int sm_count() {
   return counts[dev];
 }
 
-// Outputs the epilogue does not write get the A map in their slot (never used).
-template <int BN, int EPI>
-cudaError_t launch_gemm(const CUtensorMap& a, const CUtensorMap& b, const CUtensorMap* c, const CUtensorMap* y,
-                        const CUtensorMap* yt, int M, int N, int K, int splits, const EpiArgs& ep,
-                        cudaStream_t stream, int inject = 0) {
-  static std::atomic<bool> attr_set[64] = {};
+// Launches with the dependent-launch attribute (grid_wait): the kernel may start once every block of the one
+// before it on the stream has called grid_launch_next.
+template <typename... P, typename... A>
+cudaError_t launch_dependent(void (*kernel)(P...), int grid, int threads, int smem, cudaStream_t stream, A&&... args) {
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(grid);
+  cfg.blockDim = dim3(threads);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = stream;
+  cudaLaunchAttribute at[1];
+  at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  at[0].val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = at;
+  cfg.numAttrs = 1;
+  return cudaLaunchKernelEx(&cfg, kernel, std::forward<A>(args)...);
+}
+
+// Sets a kernel's dynamic shared-memory limit, once per device.
+template <typename Kernel>
+cudaError_t allow_smem(Kernel kernel, int bytes, std::atomic<bool>* done) {
   int dev = 0;
   cudaGetDevice(&dev);
-  if (dev < 64 && !attr_set[dev]) {
-    cudaError_t err = cudaFuncSetAttribute(umma_gemm_kernel<BN, EPI>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                           Smem<BN, EPI>::BYTES);
-    if (err != cudaSuccess) return err;
-    attr_set[dev] = true;
-  }
+  if (dev >= 0 && dev < 64 && done[dev]) return cudaSuccess;
+  const cudaError_t err = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
+  if (err == cudaSuccess && dev >= 0 && dev < 64) done[dev] = true;
+  return err;
+}
+
+// Outputs the epilogue does not write get the A map in their slot (never used).  `step`: a kernel of a training
+// step, launched dependently.
+template <int BN, int EPI>
+cudaError_t launch_gemm(const CUtensorMap& a, const CUtensorMap& b, const CUtensorMap* c, const CUtensorMap* y,
+                        const CUtensorMap* yt, int M, int N, int K, const EpiArgs& ep, cudaStream_t stream,
+                        int inject = 0, bool step = false) {
+  static std::atomic<bool> attr_set[64] = {};
+  const cudaError_t err = allow_smem(umma_gemm_kernel<BN, EPI>, Smem<BN, EPI>::BYTES, attr_set);
+  if (err != cudaSuccess) return err;
   const int m_tiles = M / BM, n_tiles = N / BN;
-  const int tiles = m_tiles * n_tiles * splits;
-  const int grid = tiles < sm_count() ? tiles : sm_count();
-  umma_gemm_kernel<BN, EPI><<<grid, GEMM_THREADS, Smem<BN, EPI>::BYTES, stream>>>(
-      a, b, c ? *c : a, y ? *y : a, yt ? *yt : a, m_tiles, n_tiles, splits, K / BK / splits, ep,
-      inject ? INJECT_WAIT_LIMIT : WAIT_LIMIT, inject);
+  const int grid = std::min(m_tiles * n_tiles, sm_count());
+  const long long limit = inject ? INJECT_WAIT_LIMIT : WAIT_LIMIT;
+  if (step)
+    return launch_dependent(umma_gemm_kernel<BN, EPI>, grid, gemm_threads(BN), Smem<BN, EPI>::BYTES, stream, a, b,
+                            c ? *c : a, y ? *y : a, yt ? *yt : a, m_tiles, n_tiles, K / BK, ep, limit, inject);
+  umma_gemm_kernel<BN, EPI><<<grid, gemm_threads(BN), Smem<BN, EPI>::BYTES, stream>>>(
+      a, b, c ? *c : a, y ? *y : a, yt ? *yt : a, m_tiles, n_tiles, K / BK, ep, limit, inject);
   return cudaGetLastError();
+}
+
+// N tile of a training GEMM with 512 output columns: the widest that still gives every SM a tile, down to 32.
+// At a batch of 1,024 (8 x 512 / N tiles) a forward layer takes 10 us with N = 128 and 32 CTAs, whose epilogues
+// are most of it.
+int train_tile(int batch) {
+  const int m_tiles = batch / BM;
+  if (m_tiles * (HID / 128) >= sm_count()) return 128;
+  return m_tiles * (HID / 64) >= sm_count() ? 64 : 32;
+}
+
+template <int EPI>
+cudaError_t launch_train_gemm(int bn, const CUtensorMap& a, const CUtensorMap& a128, const CUtensorMap* b, const CUtensorMap* c,
+                              const CUtensorMap* y, const CUtensorMap* yt, int M, int K, const EpiArgs& ep,
+                              cudaStream_t stream) {
+  if (bn == 128) return launch_gemm<128, EPI>(a128, b[2], c, y, yt, M, HID, K, ep, stream, 0, true);
+  if (bn == 64) return launch_gemm<64, EPI>(a, b[1], c, y, yt, M, HID, K, ep, stream, 0, true);
+  return launch_gemm<32, EPI>(a, b[0], c, y, yt, M, HID, K, ep, stream, 0, true);
 }
 
 cudaError_t launch_fused_forward(const CUtensorMap& x, const CUtensorMap* w256, const CUtensorMap& w5,
@@ -1110,8 +1475,8 @@ cudaError_t launch_fused_forward(const CUtensorMap& x, const CUtensorMap* w256, 
   return cudaGetLastError();
 }
 
-// Split count for a weight-gradient GEMM: enough CTAs to cover the SMs, each split a whole number
-// of 64-wide K blocks.
+// Parts of the batch a layer's weight gradient is summed over (each a whole number of 64-row K blocks), from
+// the count of its 128-wide output tiles: the order of the sum, and so its rounding, depends on it.
 int choose_splits(int tiles, int K) {
   const int kblocks = K / BK;
   int s = 1;
@@ -1153,12 +1518,9 @@ struct gf_mlp {
   __nv_bfloat16 *x0 = nullptr, *x0t = nullptr;
   float* z[4] = {};
   __nv_bfloat16 *y[4] = {}, *yt[4] = {};
-  float* out = nullptr;
   __nv_bfloat16 *dout = nullptr, *doutt = nullptr;
   __nv_bfloat16 *dz[4] = {}, *dzt[4] = {};
-  float* wpart[GF_MLP_LAYERS] = {};
   float* bpart[GF_MLP_LAYERS] = {};
-  int wsplits[GF_MLP_LAYERS] = {};
   float* loss_part = nullptr;
   float* loss = nullptr;
   int* fault = nullptr;
@@ -1166,12 +1528,14 @@ struct gf_mlp {
   // tensor maps
   CUtensorMap fwd_a[GF_MLP_LAYERS], fwd_b[GF_MLP_LAYERS];     // A = input activations, B = W
   CUtensorMap fwd_b256[4];                                    // B = W in 256-row boxes (inference tiles)
-  CUtensorMap bwd_a[GF_MLP_LAYERS], bwd_b[GF_MLP_LAYERS];     // A = dZ_l (dOut), B = W_l^T  (l >= 2)
+  // training: A = input activations, B = W_l in 32-, 64- and 128-row boxes; A = dZ_l (dOut), B = W_l^T likewise
+  // (l >= 2); two K blocks a box for tiles of 32 and 64 columns
+  CUtensorMap train_a[4], train_b[4][3];
+  CUtensorMap bwd_a[GF_MLP_LAYERS], bwd_a128[GF_MLP_LAYERS], bwd_b[GF_MLP_LAYERS][3];
   CUtensorMap dw_a[GF_MLP_LAYERS], dw_b[GF_MLP_LAYERS];       // A = dZ_l^T, B = Y_{l-1}^T
   CUtensorMap out_z[4], out_y[4], out_yt[4];                  // forward outputs of the hidden layers
-  CUtensorMap out_final;                                      // layer-5 output (fp32)
+  CUtensorMap out_dout, out_doutt;                            // dOut, dOut^T
   CUtensorMap out_dz[4], out_dzt[4];                          // backward outputs dZ, dZ^T
-  CUtensorMap out_wpart[GF_MLP_LAYERS];                       // split-K weight-gradient slices
 
   std::vector<void*> allocations;
   int inject = 0;   // fault injection armed for the next forward pass (tests)
@@ -1211,46 +1575,12 @@ gf_status alloc(gf_mlp* m, T** p, long long count) {
   return GF_OK;
 }
 
-ParamTable param_table(gf_mlp* m, int batch) {
+ParamTable param_table(gf_mlp* m) {
   ParamTable t{};
-  long long off = 0;
   for (int l = 0; l < GF_MLP_LAYERS; ++l) {
-    ParamSlot& s = t.s[l];
-    s.w = m->w[l];
-    s.m = m->m_all + m->off_w[l];
-    s.v = m->v_all + m->off_w[l];
-    s.g = m->g_all + m->off_w[l];
-    s.wb = m->wb[l];
-    s.wt = m->wt[l];
-    s.part = m->wpart[l];
-    s.part_stride = static_cast<long long>(m->rows[l]) * m->cols[l];
-    s.nparts = m->wsplits[l];
-    s.rows = m->rows[l];
-    s.cols = m->cols[l];
-    s.rows_true = m->rows_true[l];
-    s.cols_true = m->cols_true[l];
-    s.offset = off;
-    off += s.part_stride;
+    t.s[l] = {m->w[l], m->wb[l], m->wt[l], m->rows[l], m->cols[l], t.total};
+    t.total += static_cast<long long>(m->rows[l]) * m->cols[l];
   }
-  for (int l = 0; l < GF_MLP_LAYERS; ++l) {
-    ParamSlot& s = t.s[GF_MLP_LAYERS + l];
-    s.w = m->b[l];
-    s.m = m->m_all + m->off_b[l];
-    s.v = m->v_all + m->off_b[l];
-    s.g = m->g_all + m->off_b[l];
-    s.wb = nullptr;
-    s.wt = nullptr;
-    s.part = m->bpart[l];
-    s.part_stride = m->rows[l];
-    s.nparts = batch / BM;
-    s.rows = 1;
-    s.cols = m->rows[l];
-    s.rows_true = 1;
-    s.cols_true = m->rows_true[l];
-    s.offset = off;
-    off += m->rows[l];
-  }
-  t.total = off;
   return t;
 }
 
@@ -1261,13 +1591,12 @@ gf_status check_batch(gf_mlp* m, int batch) {
   return GF_OK;
 }
 
-// Forward pass.  Training writes Z, Y, Y^T and the padded fp32 output; inference (d_out != nullptr)
-// writes Y only, on 128 x 256 tiles, and the last layer writes the caller's [batch][99] array.
-gf_status run_forward(gf_mlp* m, const float* d_inputs, int batch, bool train, float* d_out = nullptr) {
-  encode_inputs_kernel<<<(batch + 255) / 256, 256, 0, m->stream>>>(d_inputs, batch, m->x0, m->x0t, m->cap,
-                                                                  train ? 1 : 0);
+// Inference: writes Y only, on 128 x 256 tiles (or keeps it on chip, fused), and the last layer writes the
+// caller's [batch][99] array.
+gf_status run_forward(gf_mlp* m, const float* d_inputs, int batch, float* d_out) {
+  encode_inputs_kernel<<<(batch + 255) / 256, 256, 0, m->stream>>>(d_inputs, nullptr, batch, m->x0, m->x0t, m->cap, 0);
   MLP_CUDA(m, cudaGetLastError());
-  if (!train && m->fused) {
+  if (m->fused) {
     cudaError_t err = launch_fused_forward(m->fwd_a[0], m->fwd_b256, m->fwd_b[4], m->b, d_out, batch, m->stream,
                                            m->inject, m->fault);
     m->inject = 0;
@@ -1280,52 +1609,53 @@ gf_status run_forward(gf_mlp* m, const float* d_inputs, int batch, bool train, f
     ep.fault = m->fault;
     cudaError_t err;
     if (l < 4) {
-      err = train ? launch_gemm<128, EPI_FWD_GELU>(m->fwd_a[l], m->fwd_b[l], &m->out_z[l], &m->out_y[l],
-                                                   &m->out_yt[l], batch, HID, m->cols[l], 1, ep, m->stream)
-                  : launch_gemm<256, EPI_FWD_GELU_INFER>(m->fwd_a[l], m->fwd_b256[l], nullptr, &m->out_y[l],
-                                                         nullptr, batch, HID, m->cols[l], 1, ep, m->stream,
-                                                         l == 0 ? m->inject : 0);
+      err = launch_gemm<256, EPI_FWD_GELU_INFER>(m->fwd_a[l], m->fwd_b256[l], nullptr, &m->out_y[l], nullptr, batch, HID,
+                                                 m->cols[l], ep, m->stream, l == 0 ? m->inject : 0);
       if (l == 0) m->inject = 0;
-    } else if (train) {
-      err = launch_gemm<128, EPI_FWD_LINEAR>(m->fwd_a[l], m->fwd_b[l], &m->out_final, nullptr, nullptr, batch,
-                                             OUT_PAD, HID, 1, ep, m->stream);
     } else {
       ep.out = d_out;
       ep.out_cols = GF_MLP_OUTPUTS;
-      err = launch_gemm<128, EPI_FWD_OUT>(m->fwd_a[l], m->fwd_b[l], nullptr, nullptr, nullptr, batch, OUT_PAD, HID,
-                                          1, ep, m->stream);
+      err = launch_gemm<128, EPI_FWD_OUT>(m->fwd_a[l], m->fwd_b[l], nullptr, nullptr, nullptr, batch, OUT_PAD, HID, ep,
+                                          m->stream);
     }
     if (err != cudaSuccess) return mlp_fail(m, GF_ERR_CUDA, "forward GEMM %d: %s", l + 1, cudaGetErrorString(err));
   }
   return GF_OK;
 }
 
-gf_status run_backward(gf_mlp* m, const float* d_targets, int batch) {
-  const int tiles = batch / BM;
-  loss_kernel<<<tiles, BM, 0, m->stream>>>(m->out, d_targets, batch, m->dout, m->doutt, m->cap, m->bpart[4],
-                                          m->loss_part);
-  MLP_CUDA(m, cudaGetLastError());
-  loss_finish_kernel<<<1, 32, 0, m->stream>>>(m->loss_part, tiles, m->loss);
-  MLP_CUDA(m, cudaGetLastError());
-  for (int l = GF_MLP_LAYERS - 1; l >= 0; --l) {
-    // weight gradient partials of layer l+1
-    {
-      EpiArgs ep{};
-      ep.rows_per_split = m->rows[l];
-      ep.fault = m->fault;
-      const int M = m->rows[l], N = m->cols[l];
-      const int bn = (N % 128 == 0) ? 128 : 64;
-      const int splits = choose_splits((M / BM) * (N / bn), batch);
-      m->wsplits[l] = splits;
-      cudaError_t err = bn == 128
-          ? launch_gemm<128, EPI_PARTIAL>(m->dw_a[l], m->dw_b[l], &m->out_wpart[l], nullptr, nullptr, M, N, batch,
-                                          splits, ep, m->stream)
-          : launch_gemm<64, EPI_PARTIAL>(m->dw_a[l], m->dw_b[l], &m->out_wpart[l], nullptr, nullptr, M, N, batch,
-                                         splits, ep, m->stream);
-      if (err != cudaSuccess)
-        return mlp_fail(m, GF_ERR_CUDA, "weight-gradient GEMM %d: %s", l + 1, cudaGetErrorString(err));
+// Forward (Z, Y, Y^T of the hidden layers, dOut, dOut^T and the loss from the last), backward (dZ, dZ^T), then the
+// weight gradients with Adam (adam) or into g_all (null): eleven launches, each starting under the tail of
+// the one before (grid_wait).  idx: the batch's rows of d_inputs and d_targets (null: the first `batch`).
+//
+// Latency-bound at small batches: a chain of eleven kernels whose K loops are 1 to 8 blocks long.  At 1,024 a step
+// takes 88 us (97 with one K block a TMA box, 107 without the overlapped launches); in 23 separate launches it was
+// 230 us of kernels.  At 4,096: 149 us.
+gf_status run_step(gf_mlp* m, const float* d_inputs, const float* d_targets, const long long* idx, int batch,
+                   const AdamArgs* adam, float* d_loss) {
+  cudaError_t err = launch_dependent(encode_inputs_kernel, (batch + 255) / 256, 256, 0, m->stream, d_inputs, idx, batch,
+                                     m->x0, m->x0t, m->cap, 1);
+  if (err != cudaSuccess) return mlp_fail(m, GF_ERR_CUDA, "encoding the inputs: %s", cudaGetErrorString(err));
+  const int bn = train_tile(batch);
+  for (int l = 0; l < GF_MLP_LAYERS; ++l) {
+    EpiArgs ep{};
+    ep.bias = m->b[l];
+    ep.fault = m->fault;
+    if (l < 4) {
+      err = launch_train_gemm<EPI_FWD_GELU>(bn, m->train_a[l], m->fwd_a[l], m->train_b[l], &m->out_z[l], &m->out_y[l],
+                                            &m->out_yt[l], batch, m->cols[l], ep, m->stream);
+    } else {
+      ep.target = d_targets;
+      ep.idx = idx;
+      ep.batch = batch;
+      ep.loss_part = m->loss_part;
+      ep.bias_part = m->bpart[4];
+      ep.ld_bias_part = OUT_PAD;
+      err = launch_gemm<128, EPI_FWD_LOSS>(m->fwd_a[l], m->fwd_b[l], nullptr, &m->out_dout, &m->out_doutt, batch,
+                                           OUT_PAD, HID, ep, m->stream, 0, true);
     }
-    if (l == 0) break;
+    if (err != cudaSuccess) return mlp_fail(m, GF_ERR_CUDA, "forward GEMM %d: %s", l + 1, cudaGetErrorString(err));
+  }
+  for (int l = GF_MLP_LAYERS - 1; l > 0; --l) {
     // input gradient of layer l+1 = output gradient of layer l, times GELU'(Z_l)
     EpiArgs ep{};
     ep.z = m->z[l - 1];
@@ -1333,15 +1663,66 @@ gf_status run_backward(gf_mlp* m, const float* d_targets, int batch) {
     ep.bias_part = m->bpart[l - 1];
     ep.ld_bias_part = HID;
     ep.fault = m->fault;
-    cudaError_t err = launch_gemm<128, EPI_BWD_GELU>(m->bwd_a[l], m->bwd_b[l], nullptr, &m->out_dz[l - 1],
-                                                    &m->out_dzt[l - 1], batch, HID, m->rows[l], 1, ep, m->stream);
+    err = launch_train_gemm<EPI_BWD_GELU>(bn, m->bwd_a[l], m->bwd_a128[l], m->bwd_b[l], nullptr, &m->out_dz[l - 1],
+                                          &m->out_dzt[l - 1], batch, m->rows[l], ep, m->stream);
     if (err != cudaSuccess)
       return mlp_fail(m, GF_ERR_CUDA, "input-gradient GEMM %d: %s", l + 1, cudaGetErrorString(err));
   }
-  ParamTable t = param_table(m, batch);
-  reduce_grads_kernel<<<2 * 148, 256, 0, m->stream>>>(t);
-  MLP_CUDA(m, cudaGetLastError());
+  static std::atomic<bool> attr_set[64] = {};
+  err = allow_smem(weight_update_kernel, DW_SMEM, attr_set);
+  DwArgs A{};
+  int biases = 0;
+  for (int l = 0; l < GF_MLP_LAYERS; ++l) {
+    DwLayer& L = A.layer[l];
+    L.a = m->dw_a[l];
+    L.b = m->dw_b[l];
+    L.w = m->w[l];
+    L.m = m->m_all + m->off_w[l];
+    L.v = m->v_all + m->off_w[l];
+    L.g = m->g_all + m->off_w[l];
+    L.wb = m->wb[l];
+    L.wt = m->wt[l];
+    L.bias = m->b[l];
+    L.bm = m->m_all + m->off_b[l];
+    L.bv = m->v_all + m->off_b[l];
+    L.bg = m->g_all + m->off_b[l];
+    L.bias_part = m->bpart[l];
+    L.rows = m->rows[l];
+    L.cols = m->cols[l];
+    L.rows_true = m->rows_true[l];
+    L.cols_true = m->cols_true[l];
+    L.splits = choose_splits((L.rows / BM) * (L.cols % 128 == 0 ? L.cols / 128 : L.cols / 64), batch);
+    L.first = A.tiles;
+    A.tiles += (L.rows / BM) * (L.cols / DW_BN);
+    biases += L.rows;
+  }
+  if (adam) A.adam = *adam;
+  A.update = adam ? 1 : 0;
+  A.k_blocks = batch / BK;
+  A.batch_tiles = batch / BM;
+  A.loss_part = m->loss_part;
+  A.loss = m->loss;
+  A.loss_out = d_loss;
+  A.fault = m->fault;
+  A.wait_limit = WAIT_LIMIT;
+  if (err == cudaSuccess)
+    err = launch_dependent(weight_update_kernel, A.tiles + (biases + DW_THREADS - 1) / DW_THREADS, DW_THREADS, DW_SMEM,
+                           m->stream, A);
+  if (err != cudaSuccess) return mlp_fail(m, GF_ERR_CUDA, "weight gradients: %s", cudaGetErrorString(err));
   return GF_OK;
+}
+
+// Gradient step with the network's current learning rate.
+gf_status run_train_step(gf_mlp* m, const float* d_inputs, const float* d_targets, const long long* idx, int batch,
+                         float* d_loss) {
+  const long long step = m->step + 1;
+  const double bc1 = 1.0 - std::pow(static_cast<double>(m->cfg.beta1), static_cast<double>(step));
+  const double bc2 = 1.0 - std::pow(static_cast<double>(m->cfg.beta2), static_cast<double>(step));
+  const AdamArgs adam{m->cfg.lr, m->cfg.beta1, m->cfg.beta2, m->cfg.eps, static_cast<float>(bc1), static_cast<float>(bc2),
+                      m->cfg.weight_decay};
+  gf_status st = run_step(m, d_inputs, d_targets, idx, batch, &adam, d_loss);
+  if (st == GF_OK) m->step = step;
+  return st;
 }
 
 }  // namespace
@@ -1405,7 +1786,6 @@ gf_status gf_mlp_create(int32_t device, void* stream, const gf_mlp_config* confi
       const long long n = static_cast<long long>(m->rows[l]) * m->cols[l];
       MLP_TRY(alloc(m, &m->wb[l], n));
       MLP_TRY(alloc(m, &m->wt[l], n));
-      MLP_TRY(alloc(m, &m->wpart[l], n * MAX_SPLITS));
       MLP_TRY(alloc(m, &m->bpart[l], (m->cap / BM) * m->rows[l]));
     }
     const long long cap = m->cap;
@@ -1418,7 +1798,6 @@ gf_status gf_mlp_create(int32_t device, void* stream, const gf_mlp_config* confi
       MLP_TRY(alloc(m, &m->dz[l], cap * HID));
       MLP_TRY(alloc(m, &m->dzt[l], cap * HID));
     }
-    MLP_TRY(alloc(m, &m->out, cap * OUT_PAD));
     MLP_TRY(alloc(m, &m->dout, cap * OUT_PAD));
     MLP_TRY(alloc(m, &m->doutt, cap * OUT_PAD));
     MLP_TRY(alloc(m, &m->loss_part, cap / BM));
@@ -1434,14 +1813,22 @@ gf_status gf_mlp_create(int32_t device, void* stream, const gf_mlp_config* confi
       ok = ok && make_map(&m->fwd_a[l], in, cap, m->cols[l], BM);
       ok = ok && make_map(&m->fwd_b[l], m->wb[l], m->rows[l], m->cols[l], 128);
       if (l < 4) ok = ok && make_map(&m->fwd_b256[l], m->wb[l], m->rows[l], m->cols[l], 256);
-      if (l > 0) {   // layer 1's input gradient is never formed
-        ok = ok && make_map(&m->bwd_a[l], g, cap, m->rows[l], BM);
-        ok = ok && make_map(&m->bwd_b[l], m->wt[l], m->cols[l], m->rows[l], 128);
+      if (l < 4) {
+        const int two = std::min(2, m->cols[l] / BK);
+        ok = ok && make_map_blocks(&m->train_a[l], in, cap, m->cols[l], BM, two);
+        for (int w = 0; w < 2; ++w)
+          ok = ok && make_map_blocks(&m->train_b[l][w], m->wb[l], m->rows[l], m->cols[l], 32 << w, two);
+        ok = ok && make_map(&m->train_b[l][2], m->wb[l], m->rows[l], m->cols[l], 128);
       }
-      ok = ok && make_map(&m->dw_a[l], g_t, m->rows[l], cap, BM);
-      ok = ok && make_map(&m->dw_b[l], in_t, m->cols[l], cap, m->cols[l] % 128 == 0 ? 128 : 64);
-      ok = ok && make_out_map(&m->out_wpart[l], m->wpart[l], static_cast<long long>(MAX_SPLITS) * m->rows[l],
-                              m->cols[l], OUT_F32);
+      if (l > 0) {   // layer 1's input gradient is never formed
+        ok = ok && make_map_blocks(&m->bwd_a[l], g, cap, m->rows[l], BM, 2);
+        ok = ok && make_map(&m->bwd_a128[l], g, cap, m->rows[l], BM);
+        for (int w = 0; w < 2; ++w)
+          ok = ok && make_map_blocks(&m->bwd_b[l][w], m->wt[l], m->cols[l], m->rows[l], 32 << w, 2);
+        ok = ok && make_map(&m->bwd_b[l][2], m->wt[l], m->cols[l], m->rows[l], 128);
+      }
+      ok = ok && make_map_blocks(&m->dw_a[l], g_t, m->rows[l], cap, BM, DW_KS);
+      ok = ok && make_map_blocks(&m->dw_b[l], in_t, m->cols[l], cap, DW_BN, DW_KS);
     }
     for (int l = 0; l < 4; ++l) {
       ok = ok && make_out_map(&m->out_z[l], m->z[l], cap, HID, OUT_F32);
@@ -1450,7 +1837,8 @@ gf_status gf_mlp_create(int32_t device, void* stream, const gf_mlp_config* confi
       ok = ok && make_out_map(&m->out_dz[l], m->dz[l], cap, HID, OUT_BF16);
       ok = ok && make_out_map(&m->out_dzt[l], m->dzt[l], HID, cap, OUT_BF16_T);
     }
-    ok = ok && make_out_map(&m->out_final, m->out, cap, OUT_PAD, OUT_F32);
+    ok = ok && make_out_map(&m->out_dout, m->dout, cap, OUT_PAD, OUT_BF16);
+    ok = ok && make_out_map(&m->out_doutt, m->doutt, OUT_PAD, cap, OUT_BF16_T);
     if (!ok) {
       st = mlp_fail(m, GF_ERR_CUDA, "tensor map encoding failed");
       goto bad;
@@ -1499,7 +1887,7 @@ gf_status gf_mlp_set_params(gf_mlp* m, const float* params, int64_t count) {
   MLP_CUDA(m, cudaMemcpyAsync(m->w_all, h.data(), h.size() * sizeof(float), cudaMemcpyHostToDevice, m->stream));
   MLP_CUDA(m, cudaMemsetAsync(m->m_all, 0, h.size() * sizeof(float), m->stream));
   MLP_CUDA(m, cudaMemsetAsync(m->v_all, 0, h.size() * sizeof(float), m->stream));
-  ParamTable t = param_table(m, BM);
+  ParamTable t = param_table(m);
   refresh_bf16_kernel<<<2 * 148, 256, 0, m->stream>>>(t);
   MLP_CUDA(m, cudaGetLastError());
   MLP_CUDA(m, cudaStreamSynchronize(m->stream));
@@ -1545,7 +1933,7 @@ gf_status gf_mlp_forward(gf_mlp* m, const float* d_inputs, int32_t batch, float*
   MLP_CUDA(m, cudaSetDevice(m->device));
   if (reinterpret_cast<uintptr_t>(d_outputs) & 15)
     return mlp_fail(m, GF_ERR_INVALID_ARGUMENT, "d_outputs must be 16-byte aligned");
-  return run_forward(m, d_inputs, batch, false, d_outputs);
+  return run_forward(m, d_inputs, batch, d_outputs);
 }
 
 gf_status gf_mlp_gradients(gf_mlp* m, const float* d_inputs, const float* d_targets, int32_t batch, float* grads,
@@ -1554,8 +1942,7 @@ gf_status gf_mlp_gradients(gf_mlp* m, const float* d_inputs, const float* d_targ
   gf_status st = check_batch(m, batch);
   if (st != GF_OK) return st;
   MLP_CUDA(m, cudaSetDevice(m->device));
-  if ((st = run_forward(m, d_inputs, batch, true)) != GF_OK) return st;
-  if ((st = run_backward(m, d_targets, batch)) != GF_OK) return st;
+  if ((st = run_step(m, d_inputs, d_targets, nullptr, batch, nullptr, nullptr)) != GF_OK) return st;
   if (loss) {
     MLP_CUDA(m, cudaMemcpyAsync(loss, m->loss, sizeof(float), cudaMemcpyDeviceToHost, m->stream));
   }
@@ -1572,17 +1959,17 @@ gf_status gf_mlp_train_step(gf_mlp* m, const float* d_inputs, const float* d_tar
   gf_status st = check_batch(m, batch);
   if (st != GF_OK) return st;
   MLP_CUDA(m, cudaSetDevice(m->device));
-  if ((st = run_forward(m, d_inputs, batch, true)) != GF_OK) return st;
-  if ((st = run_backward(m, d_targets, batch)) != GF_OK) return st;
-  m->step += 1;
-  const double bc1 = 1.0 - std::pow(static_cast<double>(m->cfg.beta1), static_cast<double>(m->step));
-  const double bc2 = 1.0 - std::pow(static_cast<double>(m->cfg.beta2), static_cast<double>(m->step));
-  ParamTable t = param_table(m, batch);
-  adam_kernel<<<2 * 148, 256, 0, m->stream>>>(t, m->cfg.lr, m->cfg.beta1, m->cfg.beta2, m->cfg.eps,
-                                             static_cast<float>(bc1), static_cast<float>(bc2), m->cfg.weight_decay);
-  MLP_CUDA(m, cudaGetLastError());
-  if (d_loss) MLP_CUDA(m, cudaMemcpyAsync(d_loss, m->loss, sizeof(float), cudaMemcpyDeviceToDevice, m->stream));
-  return GF_OK;
+  return run_train_step(m, d_inputs, d_targets, nullptr, batch, d_loss);
+}
+
+gf_status gf_mlp_train_step_rows(gf_mlp* m, const float* d_inputs, const float* d_targets, const int64_t* d_rows,
+                                 int32_t batch, float* d_loss) {
+  if (!m || !d_inputs || !d_targets || !d_rows) return GF_ERR_INVALID_ARGUMENT;
+  gf_status st = check_batch(m, batch);
+  if (st != GF_OK) return st;
+  MLP_CUDA(m, cudaSetDevice(m->device));
+  static_assert(sizeof(long long) == sizeof(int64_t), "row indices");
+  return run_train_step(m, d_inputs, d_targets, reinterpret_cast<const long long*>(d_rows), batch, d_loss);
 }
 
 gf_status gf_mlp_check(gf_mlp* m) {
@@ -1623,8 +2010,8 @@ gf_status gf_bf16_gemm(const void* d_a, const void* d_b, int32_t M, int32_t N, i
     return GF_ERR_CUDA;
   EpiArgs ep{};
   cudaStream_t s = static_cast<cudaStream_t>(stream);
-  cudaError_t err = bn == 128 ? launch_gemm<128, EPI_STORE_F32>(a, b, &c, nullptr, nullptr, M, N, K, 1, ep, s)
-                              : launch_gemm<64, EPI_STORE_F32>(a, b, &c, nullptr, nullptr, M, N, K, 1, ep, s);
+  cudaError_t err = bn == 128 ? launch_gemm<128, EPI_STORE_F32>(a, b, &c, nullptr, nullptr, M, N, K, ep, s)
+                              : launch_gemm<64, EPI_STORE_F32>(a, b, &c, nullptr, nullptr, M, N, K, ep, s);
   return err == cudaSuccess ? GF_OK : GF_ERR_CUDA;
 }
 

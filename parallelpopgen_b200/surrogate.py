@@ -125,6 +125,11 @@ class Mlp:
     def train_step(self, x, t, d_loss: int | None = None):
         self._check(self.lib.gf_mlp_train_step(self.h, x.data_ptr(), t.data_ptr(), x.shape[0], d_loss))
 
+    def train_step_rows(self, x, t, rows, d_loss: int | None = None):
+        """train_step on rows `rows` (a CUDA int64 tensor) of x and t."""
+        self._check(self.lib.gf_mlp_train_step_rows(self.h, x.data_ptr(), t.data_ptr(), rows.data_ptr(), rows.shape[0],
+                                                    d_loss))
+
     def check(self):
         self._check(self.lib.gf_mlp_check(self.h))
 
@@ -289,17 +294,25 @@ def train(mlp: Mlp, x, t, steps: int, batch: int = 1024, lr: float = 1e-3, lr_mi
     gen = torch.Generator(device=x.device)
     gen.manual_seed(seed)
     d_loss = torch.zeros(1, dtype=torch.float32, device=x.device)
-    xb = torch.empty((batch, x.shape[1]), dtype=torch.float32, device=x.device)
-    tb = torch.empty((batch, t.shape[1]), dtype=torch.float32, device=x.device)
     losses = []
+    # rows of contiguous fp32 tables of the network's widths are read in place; others are gathered first
+    in_place = (x.dtype == t.dtype == torch.float32 and x.is_contiguous() and t.is_contiguous() and x.dim() == t.dim() == 2
+                and x.shape[1] == len(SUPPORT) and t.shape[1] == OUTPUTS and x.shape[0] <= t.shape[0]
+                and x.device == t.device)
+    if not in_place:
+        xb = torch.empty((batch, x.shape[1]), dtype=torch.float32, device=x.device)
+        tb = torch.empty((batch, t.shape[1]), dtype=torch.float32, device=x.device)
     torch.cuda.synchronize()
     t0 = time.perf_counter()
     for s in range(steps):
         mlp.set_learning_rate(lr_min + 0.5 * (lr - lr_min) * (1 + math.cos(math.pi * s / steps)))
         idx = torch.randint(0, x.shape[0], (batch,), device=x.device, generator=gen)
-        torch.index_select(x, 0, idx, out=xb)
-        torch.index_select(t, 0, idx, out=tb)
-        mlp.train_step(xb, tb, d_loss.data_ptr())
+        if in_place:
+            mlp.train_step_rows(x, t, idx, d_loss.data_ptr())
+        else:
+            torch.index_select(x, 0, idx, out=xb)
+            torch.index_select(t, 0, idx, out=tb)
+            mlp.train_step(xb, tb, d_loss.data_ptr())
         if log_every and (s % log_every == 0 or s == steps - 1):
             losses.append((s, float(d_loss.item())))
     torch.cuda.synchronize()
