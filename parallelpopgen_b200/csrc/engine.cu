@@ -270,10 +270,10 @@ constexpr int kScanThreads = 1024;
 constexpr int kScanItems = 8;
 
 // n_from_slots: if not null, n = ceil(*n_from_slots / 1024) -- the tile count of a generation whose
-// slot count only the device knows.
+// slot count only the device knows, and a count may come as two 16-bit halves (window_mp.cu).
 __global__ void __launch_bounds__(kScanThreads)
     scan_exclusive_kernel(const unsigned* __restrict__ in, unsigned* __restrict__ out, int n, int* total_out,
-                          const int* __restrict__ n_from_slots) {
+                          const int* __restrict__ n_from_slots, unsigned long long* mail = nullptr, unsigned tag = 0) {
   __shared__ unsigned s_warp[kScanThreads / 32];
   __shared__ unsigned s_carry;
   if (n_from_slots) n = (*n_from_slots + kTileSlots - 1) / kTileSlots;
@@ -288,6 +288,7 @@ __global__ void __launch_bounds__(kScanThreads)
     for (int k = 0; k < kScanItems; ++k) {
       const int idx = first + k;
       v[k] = (idx < n) ? in[idx] : 0u;
+      if (n_from_slots) v[k] = (v[k] & 0xFFFFu) + (v[k] >> 16);
       tsum += v[k];
     }
     unsigned incl = tsum;
@@ -320,7 +321,10 @@ __global__ void __launch_bounds__(kScanThreads)
     if (threadIdx.x == kScanThreads - 1) s_carry = run;
     __syncthreads();
   }
-  if (threadIdx.x == 0 && total_out) *total_out = static_cast<int>(s_carry);
+  if (threadIdx.x == 0 && total_out) {
+    *total_out = static_cast<int>(s_carry);
+    post_count(mail, tag, static_cast<int>(s_carry));
+  }
 }
 
 // The same over many counts, kScanTile to a block: the tiles' sums, their scan by the kernel above, then each
@@ -590,8 +594,6 @@ static void release_sim(Engine* e) {
   e->flags = nullptr;
   e->tile_count = nullptr;
   e->tile_offset = nullptr;
-  for (auto& pc : e->pending)
-    if (pc.event) e->free_events.push_back(pc.event);
   e->pending.clear();
   e->capacity = 0;
   e->active = false;
@@ -710,27 +712,16 @@ static gf_status begin_common(Engine* e, const gf_sim_config* c, long long initi
 static void poll_pending(Engine* e, bool wait_all) {
   while (!e->pending.empty()) {
     PendingCount& pc = e->pending.front();
-    long long count;
-    if (pc.event) {
-      if (wait_all) {
-        cudaEventSynchronize(pc.event);
-      } else if (cudaEventQuery(pc.event) != cudaSuccess) {
-        cudaGetLastError();
-        break;
-      }
-      count = e->h_pinned[pc.slot];
-      e->free_events.push_back(pc.event);
-    } else {
-      const volatile unsigned long long* mail = e->h_mail + pc.slot;
-      unsigned long long v = *mail;
-      if (static_cast<unsigned>(v >> 32) != pc.tag) {
-        if (!wait_all) break;
-        cudaStreamSynchronize(e->stream);
-        v = *mail;
-      }
-      // after a failed stream the mail may not have come: the bound stays as it is
-      count = static_cast<unsigned>(v >> 32) == pc.tag ? static_cast<long long>(v & 0xFFFFFFFFu) : e->M_upper;
+    const volatile unsigned long long* mail = e->h_mail + pc.slot;
+    unsigned long long v = *mail;
+    if (static_cast<unsigned>(v >> 32) != pc.tag) {
+      if (!wait_all) break;
+      cudaStreamSynchronize(e->stream);
+      v = *mail;
     }
+    // after a failed stream the mail may not have come: the bound stays as it is
+    const long long count =
+        static_cast<unsigned>(v >> 32) == pc.tag ? static_cast<long long>(v & 0xFFFFFFFFu) : e->M_upper;
     // a bound whatever came after (later compactions only lower the count), exact if nothing did
     const long long bound = count + pc.added;
     e->M_recent = count;
@@ -742,14 +733,16 @@ static void poll_pending(Engine* e, bool wait_all) {
   }
 }
 
-static gf_status get_event(Engine* e, cudaEvent_t* ev) {
-  if (!e->free_events.empty()) {
-    *ev = e->free_events.back();
-    e->free_events.pop_back();
-    return GF_OK;
-  }
-  GF_CUDA(e, cudaEventCreateWithFlags(ev, cudaEventDisableTiming));
-  return GF_OK;
+// A slot for the survivor count of the compaction that the caller is about to launch.
+static PendingCount new_mail(Engine* e) {
+  poll_pending(e, false);
+  if (static_cast<int>(e->pending.size()) >= e->pinned_slots - 1) poll_pending(e, true);
+  PendingCount pc;
+  pc.slot = e->next_slot;
+  e->next_slot = (e->next_slot + 1) % e->pinned_slots;
+  pc.tag = ++e->mail_tag;
+  if (pc.tag == 0) pc.tag = ++e->mail_tag;   // fresh slots hold tag 0
+  return pc;
 }
 
 int host_new_mutation_count(int seed1, int seed2, float mu, int Nchrom_e, float num_sites, int generation, int pop) {
@@ -888,6 +881,7 @@ static gf_status build_args(Engine* e, const gf_generation& gen, GenArgs& a, Gen
 // d_count[slot_out]), then the stable scatter of all P rows and the IDs back into freq[cur]
 // (compact, go_fish_impl.cuh:370-429).
 static gf_status launch_compaction(Engine* e, int tiles_bound, int slot_out, bool preserve) {
+  const PendingCount pc = new_mail(e);
   cudaEvent_t ev0 = nullptr, ev1 = nullptr;
   if (e->profiling) {
     ev0 = prof_event(e);
@@ -895,7 +889,7 @@ static gf_status launch_compaction(Engine* e, int tiles_bound, int slot_out, boo
     GF_CUDA(e, cudaEventRecord(ev0, e->stream));
   }
   scan_exclusive_kernel<<<1, kScanThreads, 0, e->stream>>>(e->tile_count, e->tile_offset, 0, e->d_count + slot_out,
-                                                            e->d_count + 3);
+                                                            e->d_count + 3, e->h_mail + pc.slot, pc.tag);
   const int sblocks = std::max(1, std::min(tiles_bound, e->num_sms * 8));
   GF_CUDA(e, cudaGetLastError());
   const int src = e->cur ^ 1;
@@ -917,6 +911,8 @@ static gf_status launch_compaction(Engine* e, int tiles_bound, int slot_out, boo
     e->prof_compact.emplace_back(ev0, ev1);
   }
   e->id_cur ^= 1;
+  e->pending.push_back(pc);
+  e->M_exact = false;
   return GF_OK;
 }
 
@@ -971,20 +967,6 @@ static gf_status launch_generation(Engine* e, GenArgs& h, GenArgs* d_table, int 
   if (h.flag) {
     gf_status cst = launch_compaction(e, tiles_bound, slot_out, gh.preserve);
     if (cst != GF_OK) return cst;
-    // asynchronous read-back of the survivor count
-    poll_pending(e, false);
-    PendingCount pc;
-    gf_status st = get_event(e, &pc.event);
-    if (st != GF_OK) return st;
-    pc.slot = e->next_slot;
-    e->next_slot = (e->next_slot + 1) % e->pinned_slots;
-    pc.added = 0;
-    GF_CUDA(e, cudaMemcpyAsync(e->h_pinned + pc.slot, e->d_count + slot_out, sizeof(int), cudaMemcpyDeviceToHost,
-                               e->stream));
-    GF_CUDA(e, cudaEventRecord(pc.event, e->stream));
-    if (static_cast<int>(e->pending.size()) >= e->pinned_slots - 1) poll_pending(e, true);
-    e->pending.push_back(pc);
-    e->M_exact = false;
   } else {
     e->cur ^= 1;
   }
@@ -1013,24 +995,6 @@ static gf_status ensure_capacity(Engine* e, long long new_slots, long long* need
     }
   }
   *need_out = need;
-  return GF_OK;
-}
-
-// Queue the asynchronous read-back of the survivor count in d_count[slot].
-static gf_status push_readback(Engine* e, int slot) {
-  poll_pending(e, false);
-  PendingCount pc;
-  gf_status st = get_event(e, &pc.event);
-  if (st != GF_OK) return st;
-  pc.slot = e->next_slot;
-  e->next_slot = (e->next_slot + 1) % e->pinned_slots;
-  pc.added = 0;
-  GF_CUDA(e, cudaMemcpyAsync(e->h_pinned + pc.slot, e->d_count + slot, sizeof(int), cudaMemcpyDeviceToHost,
-                             e->stream));
-  GF_CUDA(e, cudaEventRecord(pc.event, e->stream));
-  if (static_cast<int>(e->pending.size()) >= e->pinned_slots - 1) poll_pending(e, true);
-  e->pending.push_back(pc);
-  e->M_exact = false;
   return GF_OK;
 }
 
@@ -1099,12 +1063,7 @@ static gf_status launch_window(Engine* e, int b, int first, int count, const Gen
   w.sched = e->d_count + kSchedWord;
   PendingCount pc;
   if (w.any_compact) {
-    poll_pending(e, false);
-    if (static_cast<int>(e->pending.size()) >= e->pinned_slots - 1) poll_pending(e, true);
-    pc.slot = e->next_slot;
-    e->next_slot = (e->next_slot + 1) % e->pinned_slots;
-    pc.tag = ++e->mail_tag;
-    if (pc.tag == 0) pc.tag = ++e->mail_tag;   // fresh slots hold tag 0
+    pc = new_mail(e);
     w.mail = e->h_mail + pc.slot;
     w.mail_tag = pc.tag;
   }
@@ -1147,6 +1106,14 @@ static gf_status launch_window(Engine* e, int b, int first, int count, const Gen
 
 // Run generations [first, first + count) of a multi-population batch as one window launch; the
 // kernel reads their records from the device table d_table[b].
+//
+// kSmallMpSlots: expected slots (at the window's end) up to which it runs a slot per thread in small blocks, and
+// compacts in one launch.  Window kernels of 25 generations on a B200, that against packed half tiles: three
+// populations 49 / 91 us at 4,000 slots, 61 / 104 at 130,000, 126 / 163 at 456,000, 167 / 172 at 627,000 and
+// 227 / 195 at 854,000; two 131 / 141 at 523,000 and 168 / 145 at 697,000; four 156 / 171 at 479,000 and
+// 208 / 191 at 664,000.
+constexpr long long kSmallMpSlots = 600000;
+
 static gf_status launch_window_mp(Engine* e, int b, int first, int count, const GenHost* gh) {
   long long news = 0;
   int drifted = 0;
@@ -1184,6 +1151,7 @@ static gf_status launch_window_mp(Engine* e, int b, int first, int count, const 
   w.seed2 = e->seed2;
   w.stats = e->d_stats;
   w.tiles_bound = tiles_bound;
+  w.small = std::min(need, e->M_recent + news) <= kSmallMpSlots;
   cudaEvent_t ev0 = nullptr, ev1 = nullptr;
   if (e->profiling) {
     ev0 = prof_event(e);
@@ -1201,10 +1169,27 @@ static gf_status launch_window_mp(Engine* e, int b, int first, int count, const 
   for (auto& pc : e->pending) pc.added += news;
   e->step_index += count;
   if (compact) {
-    st = launch_compaction(e, tiles_bound, slot_out, preserve);
-    if (st != GF_OK) return st;
     e->count_slot ^= 1;
-    return push_readback(e, e->count_slot);
+    if (!w.small) return launch_compaction(e, tiles_bound, slot_out, preserve);
+    const PendingCount pc = new_mail(e);
+    if (e->profiling) {
+      ev0 = prof_event(e);
+      ev1 = prof_event(e);
+      GF_CUDA(e, cudaEventRecord(ev0, e->stream));
+    }
+    st = compact_mp_run(e, w, e->freq[e->cur], e->id_gp[e->id_cur ^ 1], e->id_tid[e->id_cur ^ 1], preserve,
+                        e->h_mail + pc.slot, pc.tag);
+    if (st != GF_OK) return st;
+    if (e->profiling) {
+      GF_CUDA(e, cudaEventRecord(ev1, e->stream));
+      e->prof_compact.emplace_back(ev0, ev1);
+    }
+    e->any_preserved = e->any_preserved || preserve;
+    e->compactions += 1;
+    e->id_cur ^= 1;
+    e->pending.push_back(pc);
+    e->M_exact = false;
+    return GF_OK;
   }
   e->cur ^= 1;
   e->count_slot ^= 1;
@@ -1366,14 +1351,12 @@ gf_status gf_engine_create(int device, void* cuda_stream, gf_engine** out) {
   }
   if (cudaMalloc(&e->d_count, sizeof(int) * kCountWords) != cudaSuccess ||
       cudaMalloc(&e->d_stats, sizeof(unsigned long long) * 2) != cudaSuccess ||
-      cudaMallocHost(&e->h_pinned, (sizeof(unsigned long long) + sizeof(int)) * e->pinned_slots) != cudaSuccess) {
+      cudaMallocHost(&e->h_mail, sizeof(unsigned long long) * e->pinned_slots) != cudaSuccess) {
     if (e->d_count) cudaFree(e->d_count);
     if (e->own_stream) cudaStreamDestroy(e->stream);
     delete g;
     return GF_ERR_OUT_OF_MEMORY;
   }
-  e->h_mail = reinterpret_cast<unsigned long long*>(e->h_pinned);   // the 64-bit slots first
-  e->h_pinned = reinterpret_cast<int*>(e->h_mail + e->pinned_slots);
   std::memset(e->h_mail, 0, sizeof(unsigned long long) * e->pinned_slots);
   cudaMemsetAsync(e->d_count, 0, sizeof(int) * kCountWords, e->stream);
   cudaMemsetAsync(e->d_stats, 0, sizeof(unsigned long long) * 2, e->stream);
@@ -1420,7 +1403,6 @@ void gf_engine_destroy(gf_engine* g) {
   for (cudaEvent_t ev : e->batch_ahead)
     if (ev) cudaEventDestroy(ev);
   if (e->pool) cudaMemPoolDestroy(e->pool);
-  for (auto ev : e->free_events) cudaEventDestroy(ev);
   if (e->spec_scratch) cudaFree(e->spec_scratch);
   if (e->spec_in) cudaFree(e->spec_in);
   if (e->spec_out) cudaFree(e->spec_out);

@@ -292,4 +292,12 @@ __device__ __forceinline__ void draw_quad(const float xs[4], const uint4 r, unsi
   __syncwarp();
 }
 
+// A compaction's survivor count to the host (PendingCount).
+__device__ __forceinline__ void post_count(unsigned long long* mail, unsigned tag, int count) {
+  if (!mail) return;
+  *reinterpret_cast<volatile unsigned long long*>(mail) =
+      static_cast<unsigned long long>(tag) << 32 | static_cast<unsigned>(count);
+  __threadfence_system();
+}
+
 }  // namespace gf

@@ -157,6 +157,7 @@ struct WindowMpLaunch {
   int seed1, seed2;
   unsigned long long* stats;
   int tiles_bound;           // launch tiles (an upper bound of the end-of-window tiles)
+  bool small;                // a slot per thread, no tile counts (the compaction counts the flags)
 };
 
 // What a batched super-step derives each replicate's window from on the device (precomputed records):
@@ -263,10 +264,9 @@ struct Batch {
   long long steps_enqueued = 0, slabs_enqueued = 0;
 };
 
-// A compaction's survivor count on its way to the host: copied behind an event into h_pinned[slot], or
-// (event null) stored by the compaction itself into h_mail[slot] with the tag above it.
+// A compaction's survivor count on its way to the host: the compaction stores it into h_mail[slot] with the tag
+// above it.
 struct PendingCount {
-  cudaEvent_t event = nullptr;
   int slot = 0;
   long long added = 0;   // new mutations appended after this compaction
   unsigned tag = 0;
@@ -310,8 +310,7 @@ struct Engine {
   int* d_count = nullptr;                   // [0],[1]: mutation count ping-pong; [2]: device status;
                                             // [3]: slots at the end of a launch; [4],[5]: window tile
                                             // scheduler (kSchedWord); kCountWords words in all
-  int* h_pinned = nullptr;                  // pinned readback slots
-  unsigned long long* h_mail = nullptr;     // the same, written by the device: tag << 32 | count
+  unsigned long long* h_mail = nullptr;     // page-locked survivor counts, stored by the device: tag << 32 | count
   unsigned mail_tag = 0;
   int pinned_slots = 64;
   int next_slot = 0;
@@ -337,7 +336,6 @@ struct Engine {
   float* h_sample_stage = nullptr;    // page-locked staging of a sample's rows
   size_t sample_stage_cap = 0;        // in floats
   std::deque<PendingCount> pending;
-  std::vector<cudaEvent_t> free_events;
 
   // per-generation parameter tables (double-buffered: the host fills one while the GPU reads the other)
   GenArgs* d_table[2] = {nullptr, nullptr};
@@ -421,6 +419,9 @@ gf_status window_run(Engine* e, const WindowLaunch& w, float* compact_dst, cudaE
                      cudaEvent_t before_compaction = nullptr);
 // Multi-population window launch (window_mp.cu); P in [2, 4].
 gf_status window_mp_run(Engine* e, const WindowMpLaunch& w);
+// The compaction of a `small` one into dst, posting the survivor count to mail.
+gf_status compact_mp_run(Engine* e, const WindowMpLaunch& w, float* dst, int* gp_dst, int* tid_dst, bool preserve,
+                         unsigned long long* mail, unsigned tag);
 constexpr int kMaxWindowPops = 4;
 
 // Host draw of one population's new-mutation count (engine.cu).

@@ -432,14 +432,6 @@ __global__ void __launch_bounds__(kWinThreads, KEYS ? GF_WINDOW_MIN_BLOCKS_KEYS 
   }
 }
 
-// A compaction's survivor count to the host (PendingCount).
-__device__ __forceinline__ void post_count(unsigned long long* mail, unsigned tag, int count) {
-  if (!mail) return;
-  *reinterpret_cast<volatile unsigned long long*>(mail) =
-      static_cast<unsigned long long>(tag) << 32 | static_cast<unsigned>(count);
-  __threadfence_system();
-}
-
 // ------------------------------------------------------------------------------------------------
 // Small windows: a slot per thread
 // ------------------------------------------------------------------------------------------------
