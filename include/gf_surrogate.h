@@ -61,6 +61,22 @@ gf_status gf_mlp_set_learning_rate(gf_mlp* mlp, float lr);
 gf_status gf_mlp_forward(gf_mlp* mlp, const float* d_inputs, int32_t batch, float* d_outputs);
 gf_status gf_mlp_set_fused_inference(gf_mlp* mlp, int32_t enable);
 
+/* Spectra of model parameters, host to host: rows x 6 doubles in, scaled to the network's inputs
+ * (2 (p - low) / (high - low) - 1; the second one through asinh(p / asinh_scale) between asinh_low and
+ * asinh_high), and rows x 99 doubles out, exp(std * output + mean) divided by each row's sum.  Any number of
+ * rows.  Synchronous. */
+typedef struct gf_mlp_scaling {
+  double low[GF_MLP_INPUTS], high[GF_MLP_INPUTS];
+  double asinh_scale, asinh_low, asinh_high;
+  double mean[GF_MLP_OUTPUTS], std[GF_MLP_OUTPUTS];
+} gf_mlp_scaling;
+gf_status gf_mlp_predict(gf_mlp* mlp, const double* params, int64_t rows, const gf_mlp_scaling* scaling,
+                         double* spectra);
+
+/* inside[i] = 1 where low <= row i of params [rows][columns] <= high in every column, else 0 (host). */
+gf_status gf_rows_inside(const double* params, int64_t rows, int32_t columns, const double* low, const double* high,
+                         uint8_t* inside);
+
 /* Mean-squared-error gradients of the loss (1 / (batch * 99)) sum (out - target)^2 with respect to
  * the master parameters, without an update: host fp32 gradients in the parameter layout, and the
  * loss.  Synchronous. */

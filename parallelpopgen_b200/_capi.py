@@ -83,6 +83,12 @@ class SimConfig(ctypes.Structure):
     ]
 
 
+class MlpScaling(ctypes.Structure):
+    _fields_ = [("low", ctypes.c_double * 6), ("high", ctypes.c_double * 6), ("asinh_scale", ctypes.c_double),
+                ("asinh_low", ctypes.c_double), ("asinh_high", ctypes.c_double), ("mean", ctypes.c_double * 99),
+                ("std", ctypes.c_double * 99)]
+
+
 class MlpConfig(ctypes.Structure):
     _fields_ = [("batch_capacity", ctypes.c_int32), ("lr", ctypes.c_float), ("beta1", ctypes.c_float),
                 ("beta2", ctypes.c_float), ("eps", ctypes.c_float), ("weight_decay", ctypes.c_float)]
@@ -148,6 +154,8 @@ SIGNATURES = {
     "gf_mlp_gradients": (_I, [_P, _P, _P, _I, _P, _P]),
     "gf_mlp_train_step": (_I, [_P, _P, _P, _I, _P]),
     "gf_mlp_train_step_rows": (_I, [_P, _P, _P, _P, _I, _P]),
+    "gf_mlp_predict": (_I, [_P, _P, ctypes.c_int64, ctypes.POINTER(MlpScaling), _P]),
+    "gf_rows_inside": (_I, [_P, ctypes.c_int64, _I, _P, _P, _P]),
     "gf_mlp_check": (_I, [_P]),
     "gf_mlp_inject_fault": (_I, [_P, _I]),
     "gf_bf16_gemm": (_I, [_P, _P, _I, _I, _I, _P, _P]),

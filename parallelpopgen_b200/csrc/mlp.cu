@@ -26,6 +26,8 @@
 #include <mutex>
 #include <new>
 #include <string>
+#include <system_error>
+#include <thread>
 #include <utility>
 #include <vector>
 
@@ -945,8 +947,60 @@ fused_forward_kernel(const __grid_constant__ CUtensorMap tma_x, const __grid_con
 // small kernels
 // ---------------------------------------------------------------------------------------------
 
-// Inputs [batch][6] fp32 (row idx[i] for batch row i where idx is given) -> X0 [cap][64] bf16 (one 16-byte store of columns 0..7 per row; columns
-// 8..63 stay zero) and, for training, X0^T [64][cap].
+// Host queries: parameters [rows][6] doubles -> X0, the batch's rows past them zero, in the host encoding's
+// arithmetic (double, rounded to fp32, then to bf16).
+__global__ void query_encode_kernel(const double* __restrict__ params, int rows, int batch, const gf_mlp_scaling s,
+                                    __nv_bfloat16* __restrict__ x0) {
+  const int b = blockIdx.x * blockDim.x + threadIdx.x;
+  if (b >= batch) return;
+  float v[8] = {};
+  if (b < rows) {
+#pragma unroll
+    for (int j = 0; j < GF_MLP_INPUTS; ++j) {
+      const double p = params[static_cast<long long>(b) * GF_MLP_INPUTS + j];
+      const double lo = j == 1 ? s.asinh_low : s.low[j], hi = j == 1 ? s.asinh_high : s.high[j];
+      const double at = j == 1 ? asinh(p / s.asinh_scale) : p;
+      v[j] = static_cast<float>(2.0 * (at - lo) / (hi - lo) - 1.0);
+    }
+  }
+  uint32_t w[4];
+#pragma unroll
+  for (int t = 0; t < 4; ++t) {
+    __nv_bfloat162 p = __floats2bfloat162_rn(v[2 * t], v[2 * t + 1]);
+    w[t] = *reinterpret_cast<uint32_t*>(&p);
+  }
+  *reinterpret_cast<uint4*>(x0 + static_cast<long long>(b) * IN_PAD) = make_uint4(w[0], w[1], w[2], w[3]);
+}
+
+// Outputs [rows][99] -> normalised spectra in double, a warp a row: the copy to the host, 792 bytes a row, is what
+// a query waits for, and the exponentials (270 us on the host at 4,096 rows, 475 more for the sums and quotients)
+// are a microsecond here.
+__global__ void query_spectra_kernel(const float* __restrict__ y, int rows, const gf_mlp_scaling s,
+                                     double* __restrict__ out) {
+  const int row = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
+  if (row >= rows) return;   // warp-uniform
+  double e[4];
+  double sum = 0.0;
+#pragma unroll
+  for (int i = 0; i < 4; ++i) {
+    const int j = 32 * i + lane;
+    e[i] = 0.0;
+    if (j < GF_MLP_OUTPUTS)
+      e[i] = exp(__dadd_rn(__dmul_rn(static_cast<double>(y[static_cast<long long>(row) * GF_MLP_OUTPUTS + j]), s.std[j]),
+                           s.mean[j]));
+    sum += e[i];
+  }
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) sum += __shfl_xor_sync(0xFFFFFFFFu, sum, o);
+#pragma unroll
+  for (int i = 0; i < 4; ++i) {
+    const int j = 32 * i + lane;
+    if (j < GF_MLP_OUTPUTS) out[static_cast<long long>(row) * GF_MLP_OUTPUTS + j] = e[i] / sum;
+  }
+}
+
+// Inputs [batch][6] fp32 (row idx[i] for batch row i where idx is given) -> X0 [cap][64] bf16 (one 16-byte
+// store of columns 0..7 per row; columns 8..63 stay zero) and, for training, X0^T [64][cap].
 __global__ void encode_inputs_kernel(const float* __restrict__ x, const long long* __restrict__ idx, int batch,
                                      __nv_bfloat16* __restrict__ x0, __nv_bfloat16* __restrict__ x0t, long long cap,
                                      int transposed) {
@@ -1525,6 +1579,14 @@ struct gf_mlp {
   float* loss = nullptr;
   int* fault = nullptr;
 
+  // host queries (gf_mlp_predict), once there has been one: rows at a time; device parameters, outputs and
+  // spectra; the page-locked ring (and one chunk's parameters), an event a chunk of it
+  long long q_rows = 0;
+  double *q_params = nullptr, *q_spec = nullptr;
+  float* q_out = nullptr;
+  double* q_ring = nullptr;
+  cudaEvent_t q_done[4] = {};
+
   // tensor maps
   CUtensorMap fwd_a[GF_MLP_LAYERS], fwd_b[GF_MLP_LAYERS];     // A = input activations, B = W
   CUtensorMap fwd_b256[4];                                    // B = W in 256-row boxes (inference tiles)
@@ -1593,9 +1655,7 @@ gf_status check_batch(gf_mlp* m, int batch) {
 
 // Inference: writes Y only, on 128 x 256 tiles (or keeps it on chip, fused), and the last layer writes the
 // caller's [batch][99] array.
-gf_status run_forward(gf_mlp* m, const float* d_inputs, int batch, float* d_out) {
-  encode_inputs_kernel<<<(batch + 255) / 256, 256, 0, m->stream>>>(d_inputs, nullptr, batch, m->x0, m->x0t, m->cap, 0);
-  MLP_CUDA(m, cudaGetLastError());
+gf_status run_forward_encoded(gf_mlp* m, int batch, float* d_out) {
   if (m->fused) {
     cudaError_t err = launch_fused_forward(m->fwd_a[0], m->fwd_b256, m->fwd_b[4], m->b, d_out, batch, m->stream,
                                            m->inject, m->fault);
@@ -1619,6 +1679,106 @@ gf_status run_forward(gf_mlp* m, const float* d_inputs, int batch, float* d_out)
                                           m->stream);
     }
     if (err != cudaSuccess) return mlp_fail(m, GF_ERR_CUDA, "forward GEMM %d: %s", l + 1, cudaGetErrorString(err));
+  }
+  return GF_OK;
+}
+
+gf_status run_forward(gf_mlp* m, const float* d_inputs, int batch, float* d_out) {
+  encode_inputs_kernel<<<(batch + 255) / 256, 256, 0, m->stream>>>(d_inputs, nullptr, batch, m->x0, m->x0t, m->cap, 0);
+  MLP_CUDA(m, cudaGetLastError());
+  return run_forward_encoded(m, batch, d_out);
+}
+
+// Buffers of gf_mlp_predict, made by its first call: at most kQueryRows rows are on the device at once, and their
+// spectra come back in chunks through a page-locked ring of four, each copied to the caller while others are on
+// their way.  The ring is short because page-locking 3 MB takes longer than several queries.
+constexpr long long kQueryRows = 64 * BM;
+constexpr int kQueryChunk = 256, kQueryRing = 4;
+constexpr size_t kQueryChunkDoubles = static_cast<size_t>(kQueryChunk) * GF_MLP_OUTPUTS;
+
+gf_status query_buffers(gf_mlp* m) {
+  if (m->q_rows) return GF_OK;
+  const long long rows = std::min(m->cap, kQueryRows);
+  const size_t par = rows * GF_MLP_INPUTS * sizeof(double), spec = rows * GF_MLP_OUTPUTS * sizeof(double);
+  if (!m->q_params) {
+    void* d = nullptr;
+    MLP_CUDA(m, cudaMalloc(&d, par + spec + rows * GF_MLP_OUTPUTS * sizeof(float)));
+    m->allocations.push_back(d);
+    m->q_params = static_cast<double*>(d);
+    m->q_spec = m->q_params + rows * GF_MLP_INPUTS;
+    m->q_out = reinterpret_cast<float*>(m->q_spec + rows * GF_MLP_OUTPUTS);
+  }
+  if (!m->q_ring)
+    MLP_CUDA(m, cudaMallocHost(&m->q_ring, (kQueryRing * kQueryChunkDoubles + kQueryChunk * GF_MLP_INPUTS) * sizeof(double)));
+  static_assert(kQueryRing == sizeof(m->q_done) / sizeof(m->q_done[0]), "an event a chunk of the ring");
+  for (cudaEvent_t& ev : m->q_done)
+    if (!ev) MLP_CUDA(m, cudaEventCreateWithFlags(&ev, cudaEventDisableTiming));
+  m->q_rows = rows;
+  return GF_OK;
+}
+
+// The copy of chunk c of n rows' spectra into the ring.
+cudaError_t issue_chunk(gf_mlp* m, int n, int c) {
+  const size_t rows = std::min(kQueryChunk, n - c * kQueryChunk);
+  const cudaError_t err =
+      cudaMemcpyAsync(m->q_ring + (c % kQueryRing) * kQueryChunkDoubles, m->q_spec + c * kQueryChunkDoubles,
+                      rows * GF_MLP_OUTPUTS * sizeof(double), cudaMemcpyDeviceToHost, m->stream);
+  return err != cudaSuccess ? err : cudaEventRecord(m->q_done[c % kQueryRing], m->stream);
+}
+
+// Chunks c = first, first + step, ... to the caller, each once it has arrived, its place in the ring then taken by
+// the chunk that follows it there (step divides the ring, so that one is this thread's too).
+cudaError_t take_chunks(gf_mlp* m, int n, int first, int step, double* spectra) {
+  for (int c = first; c * kQueryChunk < n; c += step) {
+    cudaError_t err = cudaEventSynchronize(m->q_done[c % kQueryRing]);
+    if (err != cudaSuccess) return err;
+    const size_t rows = std::min(kQueryChunk, n - c * kQueryChunk);
+    std::memcpy(spectra + c * kQueryChunkDoubles, m->q_ring + (c % kQueryRing) * kQueryChunkDoubles,
+                rows * GF_MLP_OUTPUTS * sizeof(double));
+    if ((c + kQueryRing) * kQueryChunk < n && (err = issue_chunk(m, n, c + kQueryRing)) != cudaSuccess) return err;
+  }
+  return cudaSuccess;
+}
+
+gf_status run_predict(gf_mlp* m, const double* params, long long rows, const gf_mlp_scaling& s, double* spectra) {
+  gf_status st = query_buffers(m);
+  if (st != GF_OK) return st;
+  double* const h_params = m->q_ring + kQueryRing * kQueryChunkDoubles;
+  for (long long r0 = 0; r0 < rows; r0 += m->q_rows) {
+    const int n = static_cast<int>(std::min(m->q_rows, rows - r0)), batch = (n + BM - 1) / BM * BM;
+    double* const to = spectra + r0 * GF_MLP_OUTPUTS;
+    const size_t bytes = static_cast<size_t>(n) * GF_MLP_INPUTS * sizeof(double);
+    // a single chunk's parameters and spectra cross the bus in the kernels themselves: two copies less to wait for
+    const bool direct = n <= kQueryChunk;
+    if (direct) std::memcpy(h_params, params + r0 * GF_MLP_INPUTS, bytes);
+    else
+      MLP_CUDA(m, cudaMemcpyAsync(m->q_params, params + r0 * GF_MLP_INPUTS, bytes, cudaMemcpyHostToDevice, m->stream));
+    query_encode_kernel<<<(batch + 127) / 128, 128, 0, m->stream>>>(direct ? h_params : m->q_params, n, batch, s, m->x0);
+    MLP_CUDA(m, cudaGetLastError());
+    if ((st = run_forward_encoded(m, batch, m->q_out)) != GF_OK) return st;
+    query_spectra_kernel<<<(n + 7) / 8, 256, 0, m->stream>>>(m->q_out, n, s, direct ? m->q_ring : m->q_spec);
+    MLP_CUDA(m, cudaGetLastError());
+    const int chunks = (n + kQueryChunk - 1) / kQueryChunk;
+    if (direct) MLP_CUDA(m, cudaEventRecord(m->q_done[0], m->stream));
+    else
+      for (int c = 0; c < std::min(chunks, kQueryRing); ++c) MLP_CUDA(m, issue_chunk(m, n, c));
+    // one thread copies 17 GB/s, a third of the bus: from eight chunks on two of them do, from sixteen four
+    const int threads = chunks >= 16 ? 4 : chunks >= 8 ? 2 : 1;
+    cudaError_t err[kQueryRing] = {};
+    std::thread helper[kQueryRing];
+    int started = 1;
+    try {
+      for (; started < threads; ++started)
+        helper[started] = std::thread([=, &err] {
+          err[started] = cudaSetDevice(m->device);
+          if (err[started] == cudaSuccess) err[started] = take_chunks(m, n, started, threads, to);
+        });
+    } catch (const std::system_error&) {   // this thread takes the shares of those that could not be started
+    }
+    err[0] = take_chunks(m, n, 0, threads, to);
+    for (int t = started; t < threads && err[0] == cudaSuccess; ++t) err[0] = take_chunks(m, n, t, threads, to);
+    for (int t = 1; t < started; ++t) helper[t].join();
+    for (const cudaError_t e : err) MLP_CUDA(m, e);
   }
   return GF_OK;
 }
@@ -1862,6 +2022,9 @@ gf_status gf_mlp_destroy(gf_mlp* mlp) {
   cudaSetDevice(mlp->device);
   cudaStreamSynchronize(mlp->stream);
   for (void* p : mlp->allocations) cudaFree(p);
+  if (mlp->q_ring) cudaFreeHost(mlp->q_ring);
+  for (cudaEvent_t ev : mlp->q_done)
+    if (ev) cudaEventDestroy(ev);
   delete mlp;
   return GF_OK;
 }
@@ -1934,6 +2097,24 @@ gf_status gf_mlp_forward(gf_mlp* m, const float* d_inputs, int32_t batch, float*
   if (reinterpret_cast<uintptr_t>(d_outputs) & 15)
     return mlp_fail(m, GF_ERR_INVALID_ARGUMENT, "d_outputs must be 16-byte aligned");
   return run_forward(m, d_inputs, batch, d_outputs);
+}
+
+gf_status gf_mlp_predict(gf_mlp* m, const double* params, int64_t rows, const gf_mlp_scaling* scaling,
+                         double* spectra) {
+  if (!m || rows < 0 || !scaling || (rows > 0 && (!params || !spectra))) return GF_ERR_INVALID_ARGUMENT;
+  MLP_CUDA(m, cudaSetDevice(m->device));
+  return run_predict(m, params, rows, *scaling, spectra);
+}
+
+gf_status gf_rows_inside(const double* params, int64_t rows, int32_t columns, const double* low, const double* high,
+                         uint8_t* inside) {
+  if (rows < 0 || columns < 0 || (rows > 0 && (!params || !low || !high || !inside))) return GF_ERR_INVALID_ARGUMENT;
+  for (int64_t i = 0; i < rows; ++i) {
+    bool in = true;
+    for (int32_t j = 0; j < columns; ++j) in &= params[i * columns + j] >= low[j] && params[i * columns + j] <= high[j];
+    inside[i] = in ? 1 : 0;
+  }
+  return GF_OK;
 }
 
 gf_status gf_mlp_gradients(gf_mlp* m, const float* d_inputs, const float* d_targets, int32_t batch, float* grads,

@@ -25,7 +25,7 @@ from dataclasses import dataclass
 import numpy as np
 
 from . import _capi
-from ._capi import GoFishError, MlpConfig
+from ._capi import GoFishError, MlpConfig, MlpScaling
 from .engine import ConstantModel, Engine, replicate
 
 N_SAMPLE = 100
@@ -130,6 +130,12 @@ class Mlp:
         self._check(self.lib.gf_mlp_train_step_rows(self.h, x.data_ptr(), t.data_ptr(), rows.data_ptr(), rows.shape[0],
                                                     d_loss))
 
+    def predict(self, params: np.ndarray, scaling: MlpScaling) -> np.ndarray:
+        """Normalised spectra [rows][99] (float64) of parameters [rows][6] (C-contiguous float64), scaled by `scaling`."""
+        out = np.empty((len(params), OUTPUTS))
+        self._check(self.lib.gf_mlp_predict(self.h, params.ctypes.data, len(params), ctypes.byref(scaling), out.ctypes.data))
+        return out
+
     def check(self):
         self._check(self.lib.gf_mlp_check(self.h))
 
@@ -157,6 +163,12 @@ def draw_parameters(count: int, seed: int) -> np.ndarray:
 
 
 def in_support(params: np.ndarray) -> np.ndarray:
+    if type(params) is np.ndarray and params.dtype == np.float64 and params.shape[1:] == (6,) and params.flags.c_contiguous:
+        inside = np.empty(len(params), bool)
+        lo, hi = (np.ascontiguousarray(v, np.float64) for v in (LOW, HIGH))
+        if lo.shape == hi.shape == (6,) and _capi.load().gf_rows_inside(
+                params.ctypes.data, len(params), 6, lo.ctypes.data, hi.ctypes.data, inside.ctypes.data) == 0:
+            return inside
     return np.all((params >= LOW) & (params <= HIGH), axis=1)
 
 
@@ -333,6 +345,29 @@ class Surrogate:
 
     def predict(self, params: np.ndarray) -> np.ndarray:
         """Normalised expected SFS (bins 1..99) of in-support rows, from the network."""
+        params = np.asarray(params, dtype=np.float64)
+        scaling = self._scaling() if params.ndim == 2 and params.shape[1] == len(SUPPORT) else None
+        if scaling is not None:   # on the device from the parameters to the spectra
+            return self.mlp.predict(np.ascontiguousarray(params), scaling)
+        return self._predict_arrays(params)
+
+    def _scaling(self) -> MlpScaling | None:
+        """How the network's inputs and outputs are scaled, where the library knows that scaling."""
+        if type(self.mlp) is not Mlp or not (self.scale is None or type(self.scale) is TargetScale):
+            return None
+        s = MlpScaling()
+        mean, std = (0.0, 1.0) if self.scale is None else (self.scale.mean, self.scale.std)
+        try:
+            s.low[:], s.high[:] = LOW.tolist(), HIGH.tolist()
+            s.mean[:] = np.broadcast_to(np.asarray(mean, np.float64), OUTPUTS).tolist()
+            s.std[:] = np.broadcast_to(np.asarray(std, np.float64), OUTPUTS).tolist()
+        except ValueError:
+            return None
+        s.asinh_scale = GAMMA_SCALE
+        s.asinh_low, s.asinh_high = np.arcsinh(LOW[1] / GAMMA_SCALE), np.arcsinh(HIGH[1] / GAMMA_SCALE)
+        return s
+
+    def _predict_arrays(self, params: np.ndarray) -> np.ndarray:
         import torch
         B = len(params)
         Bp = ((B + 127) // 128) * 128
@@ -353,6 +388,8 @@ class Surrogate:
         """(normalised SFS per row, routed_to_simulator mask)."""
         params = np.atleast_2d(np.asarray(params, dtype=np.float64))
         ok = in_support(params)
+        if len(ok) and ok.all():
+            return self.predict(params), ~ok
         res = np.zeros((len(params), OUTPUTS))
         if ok.any():
             res[ok] = self.predict(params[ok])
