@@ -56,18 +56,6 @@ __device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity, long l
   return true;
 }
 
-// The same, for a thread with nothing else to do meanwhile: it sleeps briefly between polls, so that
-// the warps sharing its scheduler get the issue slots.
-__device__ __forceinline__ bool mbar_wait_sleep(uint64_t* bar, uint32_t parity, long long limit) {
-  const uint32_t addr = smem_u32(bar);
-  const long long t0 = clock64();
-  while (!mbar_try_wait(addr, parity)) {
-    if (clock64() - t0 > limit) return false;
-    __nanosleep(64);
-  }
-  return true;
-}
-
 // ---------------------------------------------------------------------------------------------
 // TMA: 2-D tiled load global -> this CTA's shared memory, completion counted on an mbarrier
 // ---------------------------------------------------------------------------------------------
@@ -225,5 +213,69 @@ __device__ __forceinline__ void tmem_st_16cols(uint32_t taddr, const uint32_t* w
 
 // Every tensor-memory store this thread issued has completed.
 __device__ __forceinline__ void tmem_st_wait() { asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory"); }
+
+// ---------------------------------------------------------------------------------------------
+// Pairs of CTAs (clusters of two): one MMA of M = 256 over both SMs, each supplying its 128 rows of A and half the
+// rows of B from its own shared memory (same offsets) and holding its 128 rows of D
+// ---------------------------------------------------------------------------------------------
+// one lane of a converged warp; code around it stays warp-uniform, which keeps MMA and TMA operands in uniform registers
+__device__ __forceinline__ bool elect_one() {
+  uint32_t is;
+  asm volatile(
+      "{\n"
+      ".reg .pred p;\n"
+      "elect.sync _|p, 0xFFFFFFFF;\n"
+      "selp.u32 %0, 1, 0, p;\n"
+      "}\n"
+      : "=r"(is));
+  return is != 0;
+}
+__device__ __forceinline__ uint32_t cluster_rank() {
+  uint32_t r;
+  asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
+  return r;
+}
+__device__ __forceinline__ void cluster_sync() {   // all threads of both CTAs
+  asm volatile("barrier.cluster.arrive.release.aligned;\nbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+// arrive on the barrier at the same offset in CTA `rank` of the cluster
+__device__ __forceinline__ void mbar_arrive_remote(uint64_t* bar, uint32_t rank) {
+  asm volatile(
+      "{\n"
+      ".reg .b32 a;\n"
+      "mapa.shared::cluster.u32 a, %0, %1;\n"
+      "mbarrier.arrive.shared::cluster.b64 _, [a];\n"
+      "}\n" ::"r"(smem_u32(bar)),
+      "r"(rank)
+      : "memory");
+}
+__device__ __forceinline__ void tmem_alloc_pair(uint32_t* slot, uint32_t ncols) {  // a whole warp in each CTA
+  asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(slot)), "r"(ncols)
+               : "memory");
+  asm volatile("tcgen05.relinquish_alloc_permit.cta_group::2.sync.aligned;" ::: "memory");
+}
+__device__ __forceinline__ void tmem_dealloc_pair(uint32_t taddr, uint32_t ncols) {  // a whole warp in each CTA
+  asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;" ::"r"(taddr), "r"(ncols) : "memory");
+}
+// issued by one thread of the even CTA
+__device__ __forceinline__ void umma_bf16_pair(uint32_t tmem_d, uint64_t a_desc, uint64_t b_desc, uint32_t idesc,
+                                               uint32_t accumulate) {
+  asm volatile(
+      "{\n"
+      ".reg .pred p;\n"
+      "setp.ne.b32 p, %4, 0;\n"
+      "tcgen05.mma.cta_group::2.kind::f16 [%0], %1, %2, %3, p;\n"
+      "}\n" ::"r"(tmem_d),
+      "l"(a_desc), "l"(b_desc), "r"(idesc), "r"(accumulate)
+      : "memory");
+}
+// arrive on `bar` of both CTAs once every MMA this thread issued before has completed
+__device__ __forceinline__ void umma_commit_pair(uint64_t* bar) {
+  const uint16_t both = 3;
+  asm volatile("tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %1;" ::"r"(
+                   smem_u32(bar)),
+               "h"(both)
+               : "memory");
+}
 
 }  // namespace gfm

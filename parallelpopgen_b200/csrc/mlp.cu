@@ -535,53 +535,47 @@ umma_gemm_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constan
 }
 
 // ---------------------------------------------------------------------------------------------
-// Fused inference forward: all five layers of a 128-row tile in one CTA, the activations on chip.
+// Fused inference forward: all five layers of a 128-row tile in one CTA, the activations on chip, the
+// MMAs of two CTAs paired
 //
 // The layered path writes each hidden activation (batch x 512 bf16) to memory and reads it back in
 // the next layer's GEMM.  Here a CTA keeps its tile's activation H (128 x 512 bf16 = 128 KB) in
 // shared memory, in the 128-byte-swizzled K-major layout the MMA reads (eight 64-column K blocks of
 // 16 KB), and the layer's fp32 accumulator (128 x 512) in all 512 tensor-memory columns: N half 0
-// in region A (columns 0-255), N half 1 in region B (256-511).  Warp 1 issues the MMAs (A = H from
-// shared memory, B = weight K-blocks streamed by warp 0's TMA through a 3-stage ring from L2, where
-// every CTA finds the 1.3 MB of weights); 16 epilogue warps drain the accumulators (bias, GELU, bf16)
-// back into H for the next layer, overlapped with the MMAs: region A while N half 1 accumulates
-// (staged in tensor memory, since H is still being read), region B while the next layer's first
-// K blocks accumulate.  The last layer's epilogue writes acc + bias to the caller's [batch][99]
-// array.  Each layer's MMAs run in the order of the layered GEMMs (N halves of 256, K blocks 0..7,
-// four 16-wide slices each; layer 5 one 128-wide N tile), so the outputs are bit-identical to the
-// layered path.
+// in region A (columns 0-255), N half 1 in region B (256-511).  Two neighbouring tiles run on a cluster
+// of two CTAs: warp 1 of the even one issues MMAs of M = 256 over both (A = each CTA's H, B = weight K
+// blocks of which each CTA holds half the rows, streamed by its warp 0 through a ring of six from L2,
+// where every CTA finds the 1.3 MB of weights), warp 1 of the odd one reports what has landed there.  16
+// epilogue warps a CTA drain the accumulators (bias, GELU, bf16) back into H for the next layer,
+// overlapped with the MMAs: region A while N half 1 accumulates (staged in tensor memory, since H is
+// still being read), region B, two K blocks at a time, while the next layer's first K blocks accumulate.
+// The last layer's epilogue writes acc + bias to the caller's [batch][99] array.  Each layer's MMAs run
+// in the order of the layered GEMMs (N halves of 256, K blocks 0..7, four 16-wide slices each; layer 5
+// one 128-wide N tile), so the outputs are bit-identical to the layered path.
+//
+// A layer takes about 11,000 cycles, of which the MMAs 8,400 at their peak rate and the two epilogues 3,800 +
+// 3,200: they share tensor memory and shared memory, and each slows the other down.  32,768 rows (256 tiles,
+// two rounds of 74 pairs) take 62.5 us; with single-lane producer and issue code on single CTAs it was 86.4,
+// a K block taking 940 cycles to issue.  By step: pairs alone 89.5, converged producer and issue warps 71.9,
+// region B in two parts and the bias from L1 65.8, a ring of single K blocks 64.2, epilogue warps that wait
+// each for themselves 62.5; region B in four parts is slower again (64.4).
 // ---------------------------------------------------------------------------------------------
 constexpr int FF_EPI_WARPS = 16;                          // four per tensor-memory lane quarter
 constexpr int FF_THREADS = 64 + 32 * FF_EPI_WARPS;        // TMA warp, MMA warp, 16 epilogue warps
-constexpr int FF_WSTAGES = 3;
+constexpr int FF_WSTAGES = 6;
 constexpr int FF_KB_BYTES = BM * BK * 2;                  // one 128 x 64 bf16 K block of H: 16 KB
 constexpr int FF_H_BYTES = BM * HID * 2;                  // H: 128 KB
-constexpr int FF_WSTAGE_BYTES = 256 * BK * 2;             // a 256-row x 64 weight block: 32 KB
-constexpr int FF_BIAS_OFFSET = FF_H_BYTES + FF_WSTAGES * FF_WSTAGE_BYTES;   // the layer's bias (512 fp32)
-constexpr int FF_BAR_OFFSET = FF_BIAS_OFFSET + HID * 4;
+constexpr int FF_WSTAGE_BYTES = 128 * BK * 2;             // this CTA's 128 rows of a 256-row x 64 weight block: 16 KB
+constexpr int FF_BAR_OFFSET = FF_H_BYTES + FF_WSTAGES * FF_WSTAGE_BYTES;
 constexpr int FF_ALIGN_SLACK = 256;   // dynamic shared memory starts 1024-aligned when a kernel has no static
                                       // shared memory; up to this much misalignment is absorbed, more is a fault
 constexpr int FF_SMEM = FF_BAR_OFFSET + 256 + FF_ALIGN_SLACK;   // + barriers and flags
 static_assert(FF_SMEM <= SMEM_LIMIT, "fused forward shared memory");
-constexpr int FF_STAGES_PER_TILE = 2 + 3 * 16 + 8;        // weight blocks streamed per tile (58)
+constexpr int FF_LOADS_PER_TILE = 2 + 3 * 16 + 8;           // weight blocks streamed per tile
 constexpr int kFfStoreThread = 64;                         // the epilogue thread that issues the output stores
-constexpr int kFfPollThread = 64;                          // the epilogue thread that waits for the MMA hand-offs
 static_assert(BM * GF_MLP_OUTPUTS * 4 <= 4 * FF_KB_BYTES, "staged outputs fit in H's K blocks 1-4");
 
-// Weight block `i` of a tile's stream: layer, the N offset of its rows, the K block, its rows.
-struct FfBlock {
-  int layer, n0, kb, rows;
-};
-__device__ __forceinline__ FfBlock ff_block(int i) {
-  if (i < 2) return {0, 256 * i, 0, 256};                           // layer 1: K = 64, two N halves
-  if (i < 50) {                                                      // layers 2-4: N halves x 8 K blocks
-    const int j = i - 2;
-    return {1 + j / 16, 256 * ((j % 16) / 8), j % 8, 256};
-  }
-  return {4, 0, i - 50, OUT_PAD};                                    // layer 5: 128 rows x 8 K blocks
-}
-
-__global__ void __launch_bounds__(FF_THREADS, 1)
+__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(FF_THREADS, 1)
 fused_forward_kernel(const __grid_constant__ CUtensorMap tma_x, const __grid_constant__ CUtensorMap tma_w1,
                      const __grid_constant__ CUtensorMap tma_w2, const __grid_constant__ CUtensorMap tma_w3,
                      const __grid_constant__ CUtensorMap tma_w4, const __grid_constant__ CUtensorMap tma_w5,
@@ -590,33 +584,37 @@ fused_forward_kernel(const __grid_constant__ CUtensorMap tma_x, const __grid_con
                      int batch, int m_tiles, long long wait_limit, int inject, int* fault) {
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
-  if (smem - smem_raw > FF_ALIGN_SLACK) {   // the layout would not fit (uniform over the CTA)
+  if (smem - smem_raw > FF_ALIGN_SLACK) {   // the layout would not fit (the same in both CTAs)
     if (threadIdx.x == 0 && fault) atomicOr(fault, 1);
     return;
   }
   uint8_t* H = smem;
   uint8_t* W = smem + FF_H_BYTES;
-  float* s_bias = reinterpret_cast<float*>(smem + FF_BIAS_OFFSET);
   uint64_t* wfull = reinterpret_cast<uint64_t*>(smem + FF_BAR_OFFSET);
   uint64_t* wempty = wfull + FF_WSTAGES;
   uint64_t* xfull = wempty + FF_WSTAGES;   // the tile's inputs have landed in H's first K block
   uint64_t* accA = xfull + 1;              // N half 0 (region A) accumulated (MMA -> epilogue)
   uint64_t* accB = accA + 1;               // N half 1 (region B) accumulated: the layer's MMAs are done
   uint64_t* hlo = accB + 1;                // H's K blocks 0-3 written, region A drained (epilogue -> MMA)
-  uint64_t* hhi = hlo + 1;                 // H's K blocks 4-7 written, region B drained (epilogue -> MMA)
+  uint64_t* hmid = hlo + 1;                // H's K blocks 4-5 written (epilogue -> MMA)
+  uint64_t* hhi = hmid + 1;                // H's K blocks 6-7 written, region B drained (epilogue -> MMA)
   uint64_t* hfree = hhi + 1;               // the tile's last MMAs have read H (MMA -> producer)
-  uint64_t* drain = hfree + 1;             // MMA completion before tensor memory is released (abort)
+  uint64_t* staged = hfree + 1;            // the tile's output rows are staged (epilogue -> its storing thread)
+  uint64_t* sread = staged + 1;            // ... and have been read by the store (storing thread -> epilogue)
+  uint64_t* drain = sread + 1;             // MMA completion before tensor memory is released (abort)
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(drain + 1);
   int* flags = reinterpret_cast<int*>(tmem_slot + 1);
-  volatile int* abort_flag = flags;        // [0] a wait ran out; [1] epilogue verdict; [2] consumed
-  int* epi_fail = flags + 1;
+  volatile int* abort_flag = flags;        // [0] a wait ran out; [2], [3] consumed
   int* consumed_s = flags + 2;             // weight blocks the MMA thread received (for the drain)
   int* x_consumed_s = flags + 3;           // input tiles the MMA thread received
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const uint32_t rank = cluster_rank();
+  // a pair's tiles are neighbours; past the last one the odd CTA works on rows that nobody reads
+  const int tiles_up = m_tiles + (m_tiles & 1);
   auto wait = [&](uint64_t* bar, uint32_t parity) -> bool {
-    if (*abort_flag) return false;
     const uint32_t addr = smem_u32(bar);
+    if (mbar_try_wait(addr, parity)) return true;   // as a rule: the MMA thread has few issue slots to spare
     const long long t0 = clock64();
     while (!mbar_try_wait(addr, parity)) {
       if (*abort_flag) return false;
@@ -624,23 +622,6 @@ fused_forward_kernel(const __grid_constant__ CUtensorMap tma_x, const __grid_con
         *abort_flag = 1;
         return false;
       }
-    }
-    return true;
-  };
-
-  // the same, sleeping between polls: for the producer, whose polls otherwise take issue slots and
-  // barrier accesses from the MMA thread (~2%)
-  auto wait_sleep = [&](uint64_t* bar, uint32_t parity) -> bool {
-    if (*abort_flag) return false;
-    const uint32_t addr = smem_u32(bar);
-    const long long t0 = clock64();
-    while (!mbar_try_wait(addr, parity)) {
-      if (*abort_flag) return false;
-      if (clock64() - t0 > wait_limit) {
-        *abort_flag = 1;
-        return false;
-      }
-      __nanosleep(32);
     }
     return true;
   };
@@ -648,131 +629,179 @@ fused_forward_kernel(const __grid_constant__ CUtensorMap tma_x, const __grid_con
   if (threadIdx.x == 0) {
     tma_prefetch_desc(&tma_x);
     for (int s = 0; s < FF_WSTAGES; ++s) {
-      mbar_init(&wfull[s], 1);
+      mbar_init(&wfull[s], 2 - rank);   // in the even CTA also told of the other one's block
       mbar_init(&wempty[s], 1);
     }
-    mbar_init(xfull, 1);
+    mbar_init(xfull, 2 - rank);
     mbar_init(accA, 1);
     mbar_init(accB, 1);
-    mbar_init(hlo, FF_EPI_WARPS);
-    mbar_init(hhi, FF_EPI_WARPS);
+    mbar_init(hlo, 2 * FF_EPI_WARPS);   // in the even CTA, from both
+    mbar_init(hmid, 2 * FF_EPI_WARPS);
+    mbar_init(hhi, 2 * FF_EPI_WARPS);
     mbar_init(hfree, 1);
+    mbar_init(staged, FF_EPI_WARPS);
+    mbar_init(sread, 1);
     mbar_init(drain, 1);
     flags[0] = flags[1] = flags[2] = flags[3] = 0;
     mbar_fence_init();
   }
   __syncwarp();
-  if (warp == 1) tmem_alloc(tmem_slot, 512);
+  if (warp == 1) tmem_alloc_pair(tmem_slot, 512);
   tc_fence_before();
-  __syncthreads();
+  cluster_sync();   // both CTAs' barriers are there
   tc_fence_after();
   const uint32_t tmem = *tmem_slot;
   bool late = false;
   int issued = 0, x_issued = 0;
 
+  // Warps 0 and 1 stay converged, with one elected lane to issue: as single-lane code the producer took 500 to
+  // 1,000 cycles a box and the MMA issue 680 a K block, more than the tensor cores need.
   if (warp == 0) {
-    // ---- producer: the tile's inputs, then its 58 weight blocks in the order the MMAs use them ----
-    if (lane == 0) {
-      int it = 0, local = 0;
-      for (int tile = blockIdx.x; tile < m_tiles; tile += gridDim.x, ++local) {
-        if (local > 0 && !wait(hfree, (local - 1) & 1)) {   // the previous tile's MMAs are done with H
-          late = true;
-          break;
-        }
+    // ---- producer: the tile's inputs, then its weights in the order the MMAs use them ----
+    int s = 0, local = 0;
+    uint32_t phase = 1;
+    auto load = [&](const CUtensorMap& map, int n0, int kb, int bytes) -> bool {
+      if (!wait(&wempty[s], phase)) return false;
+      if (elect_one()) {
+        mbar_arrive_expect_tx(&wfull[s], bytes);
+        tma_load_2d(W + s * FF_WSTAGE_BYTES, &map, kb * BK, n0, &wfull[s]);
+      }
+      __syncwarp();
+      ++issued;
+      if (++s == FF_WSTAGES) {
+        s = 0;
+        phase ^= 1;
+      }
+      return true;
+    };
+    for (int tile = blockIdx.x; tile < tiles_up && !late; tile += gridDim.x, ++local) {
+      if (local > 0 && !wait(hfree, (local - 1) & 1)) {   // the previous tile's MMAs are done with H
+        late = true;
+        break;
+      }
+      if (elect_one()) {
         mbar_arrive_expect_tx(xfull, FF_KB_BYTES);
         tma_load_2d(H, &tma_x, 0, tile * BM, xfull);
-        ++x_issued;
-        bool stop = false;
-        for (int i = 0; i < FF_STAGES_PER_TILE; ++i, ++it) {
-          const int s = it % FF_WSTAGES;
-          if (!wait_sleep(&wempty[s], ((it / FF_WSTAGES) & 1) ^ 1)) {
-            stop = true;
-            break;
-          }
-          const FfBlock blk = ff_block(i);
-          const CUtensorMap* map = blk.layer == 0 ? &tma_w1 : blk.layer == 1 ? &tma_w2 : blk.layer == 2 ? &tma_w3
-                                   : blk.layer == 3 ? &tma_w4 : &tma_w5;
-          mbar_arrive_expect_tx(&wfull[s], blk.rows * BK * 2);
-          tma_load_2d(W + s * FF_WSTAGE_BYTES, map, blk.kb * BK, blk.n0, &wfull[s]);
-        }
-        if (stop) {
+      }
+      __syncwarp();
+      ++x_issued;
+      // this CTA's 128 (layer 5: 64) rows of each block
+      const int row = static_cast<int>(rank) * BM;
+      late = !load(tma_w1, row, 0, FF_KB_BYTES) || !load(tma_w1, 256 + row, 0, FF_KB_BYTES);
+      for (int n0 = row; n0 < HID && !late; n0 += 256)
+        for (int kb = 0; kb < 8 && !late; ++kb) late = !load(tma_w2, n0, kb, FF_WSTAGE_BYTES);
+      for (int n0 = row; n0 < HID && !late; n0 += 256)
+        for (int kb = 0; kb < 8 && !late; ++kb) late = !load(tma_w3, n0, kb, FF_WSTAGE_BYTES);
+      for (int n0 = row; n0 < HID && !late; n0 += 256)
+        for (int kb = 0; kb < 8 && !late; ++kb) late = !load(tma_w4, n0, kb, FF_WSTAGE_BYTES);
+      for (int kb = 0; kb < 8 && !late; ++kb) late = !load(tma_w5, row / 2, kb, FF_WSTAGE_BYTES / 2);
+    }
+  } else if (warp == 1 && rank == 1) {
+    // ---- the odd CTA tells the even one's MMA warp what has landed here ----
+    int s = 0, got = 0, local = 0;
+    uint32_t phase = 0;
+    for (int tile = blockIdx.x; tile < tiles_up && !late; tile += gridDim.x, ++local) {
+      if (!wait(xfull, local & 1)) {
+        late = true;
+        break;
+      }
+      if (lane == 0) {
+        *x_consumed_s = local + 1;
+        mbar_arrive_remote(xfull, 0);
+      }
+      __syncwarp();
+      for (int i = 0; i < FF_LOADS_PER_TILE; ++i) {
+        if (!wait(&wfull[s], phase)) {
           late = true;
           break;
+        }
+        ++got;
+        if (lane == 0) mbar_arrive_remote(&wfull[s], 0);
+        __syncwarp();
+        if (++s == FF_WSTAGES) {
+          s = 0;
+          phase ^= 1;
         }
       }
-      issued = it;
     }
+    if (lane == 0) *consumed_s = got;
     __syncwarp();
   } else if (warp == 1) {
-    // ---- MMA issue (one thread) ----
-    if (lane == 0) {
-      constexpr uint32_t idesc256 = bf16_idesc(BM, 256);
-      constexpr uint32_t idesc128 = bf16_idesc(BM, OUT_PAD);
-      int it = 0, local = 0, lo_waits = 0, hi_waits = 0, xs = 0;
-      const uint32_t h_addr = smem_u32(H);
-      // the four MMAs of weight block i of the tile's stream (ring slot it % 3): A = H's K block
-      auto stage = [&](int i, uint32_t d, uint32_t idesc) -> bool {
-        const int s = it % FF_WSTAGES;
-        if (!wait(&wfull[s], (it / FF_WSTAGES) & 1)) return false;
-        tc_fence_after();
-        const FfBlock blk = ff_block(i);
-        const uint32_t w_addr = smem_u32(W + s * FF_WSTAGE_BYTES);
-        const uint32_t a_addr = h_addr + blk.kb * FF_KB_BYTES;
+    // ---- MMA issue (the even CTA) ----
+    constexpr uint32_t idesc256 = bf16_idesc(2 * BM, 256);
+    constexpr uint32_t idesc128 = bf16_idesc(2 * BM, OUT_PAD);
+    int got = 0, local = 0, lo_waits = 0, hi_waits = 0, xs = 0;
+    const uint64_t h_desc = sw128_kmajor_desc(smem_u32(H)), w_desc = sw128_kmajor_desc(smem_u32(W));
+    int s = 0;
+    uint32_t phase = 0;
+    // the four MMAs of the next weight block (ring slot s): A = H's K block kb.  Descriptor addresses count 16 bytes.
+    auto stage = [&](int kb, uint32_t d, uint32_t idesc) -> bool {
+      if (!wait(&wfull[s], phase)) return false;
+      tc_fence_after();
+      const uint64_t a = h_desc + kb * (FF_KB_BYTES >> 4), w = w_desc + s * (FF_WSTAGE_BYTES >> 4);
+      if (elect_one()) {
 #pragma unroll
-        for (int kk = 0; kk < BK / 16; ++kk)
-          umma_bf16(d, sw128_kmajor_desc(a_addr + kk * 32), sw128_kmajor_desc(w_addr + kk * 32), idesc,
-                    (blk.kb | kk) != 0);
-        umma_commit(&wempty[s]);
-        ++it;
-        return true;
-      };
-      for (int tile = blockIdx.x; tile < m_tiles && !late; tile += gridDim.x, ++local) {
-        if (!wait(xfull, local & 1)) {
-          late = true;
-          break;
+        for (int kk = 0; kk < BK / 16; ++kk) umma_bf16_pair(d, a + 2 * kk, w + 2 * kk, idesc, (kb | kk) != 0);
+        umma_commit_pair(&wempty[s]);
+      }
+      __syncwarp();
+      ++got;
+      if (++s == FF_WSTAGES) {
+        s = 0;
+        phase ^= 1;
+      }
+      return true;
+    };
+    auto commit = [&](uint64_t* bar) {
+      if (elect_one()) umma_commit_pair(bar);
+      __syncwarp();
+    };
+    for (int tile = blockIdx.x; tile < tiles_up && !late; tile += gridDim.x, ++local) {
+      if (!wait(xfull, local & 1)) {
+        late = true;
+        break;
+      }
+      ++xs;
+      for (int layer = 0; layer < GF_MLP_LAYERS; ++layer) {
+        // region A drained (by the previous layer's staging copy, or the previous tile's output) and,
+        // from the second layer on, H's K blocks 0-3 written
+        if (local > 0 || layer > 0) {
+          if (!wait(hlo, lo_waits & 1)) {
+            late = true;
+            break;
+          }
+          ++lo_waits;
         }
-        ++xs;
-        int i = 0;
-        for (int layer = 0; layer < GF_MLP_LAYERS; ++layer) {
-          // region A drained (by the previous layer's staging copy, or the previous tile's output) and,
-          // from the second layer on, H's K blocks 0-3 written
-          if (local > 0 || layer > 0) {
-            if (!wait(hlo, lo_waits & 1)) {
+        tc_fence_after();
+        // N half 0 (the output layer's only N tile) into region A; K blocks 4-7 once H's K blocks 4-7
+        // are written (which also means region B is drained)
+        const int kblocks = layer == 0 ? 1 : 8;
+        for (int kb = 0; kb < kblocks && !late; ++kb) {
+          if (kb == 4 || kb == 6) {
+            if (!wait(kb == 4 ? hmid : hhi, hi_waits & 1)) {
               late = true;
               break;
             }
-            ++lo_waits;
+            if (kb == 6) ++hi_waits;
+            tc_fence_after();
           }
-          tc_fence_after();
-          const int kblocks = layer == 0 ? 1 : 8;
-          // N half 0 (the output layer's only N tile) into region A; K blocks 4-7 once H's K blocks 4-7
-          // are written (which also means region B is drained)
-          for (int kb = 0; kb < kblocks && !late; ++kb, ++i) {
-            if (kb == 4) {
-              if (!wait(hhi, hi_waits & 1)) {
-                late = true;
-                break;
-              }
-              ++hi_waits;
-              tc_fence_after();
-            }
-            if (!stage(i, tmem, layer == 4 ? idesc128 : idesc256)) late = true;
-          }
-          if (late) break;
-          // fault injection for tests: withhold the first accumulator hand-off
-          if (!((inject & 1) && local == 0 && layer == 0)) umma_commit(accA);
-          if (layer < 4) {
-            // N half 1 into region B, while the epilogue drains region A
-            for (int kb = 0; kb < kblocks && !late; ++kb, ++i)
-              if (!stage(i, tmem + 256, idesc256)) late = true;
-            if (late) break;
-            umma_commit(accB);   // also: every MMA of the layer has read H
-          }
+          late = !stage(kb, tmem, layer == 4 ? idesc128 : idesc256);
         }
         if (late) break;
-        umma_commit(hfree);
+        // fault injection for tests: withhold the first accumulator hand-off
+        if (!((inject & 1) && local == 0 && layer == 0)) commit(accA);
+        if (layer < 4) {
+          // N half 1 into region B, while the epilogue drains region A
+          for (int kb = 0; kb < kblocks && !late; ++kb) late = !stage(kb, tmem + 256, idesc256);
+          if (late) break;
+          commit(accB);   // also: every MMA of the layer has read H
+        }
       }
-      *consumed_s = it;
+      if (late) break;
+      commit(hfree);
+    }
+    if (lane == 0) {
+      *consumed_s = got;
       *x_consumed_s = xs;
     }
     __syncwarp();
@@ -789,28 +818,24 @@ fused_forward_kernel(const __grid_constant__ CUtensorMap tma_x, const __grid_con
     float* s_out = reinterpret_cast<float*>(H + FF_KB_BYTES);   // the last layer's staged outputs
     const uint32_t tlane = tmem + (static_cast<uint32_t>(qd * 32) << 16);
     int a_waits = 0, b_waits = 0;
-    // one thread waits for the MMA hand-off (sixteen pollers of the same barrier slow the MMAs down by
-    // ~5%); every epilogue warp then learns the verdict at the named barrier
-    auto handoff = [&](uint64_t* bar, int& n, bool store_read) -> bool {
-      if (threadIdx.x == kFfPollThread && !mbar_wait_sleep(bar, n & 1, wait_limit)) atomicOr(epi_fail, 1);
+    const float* bias = b1;
+    // every warp waits for the MMA hand-off itself: nothing in the epilogue waits for all of its warps
+    auto handoff = [&](uint64_t* bar, int& n) -> bool {
+      const bool ok = wait(bar, n & 1);
       ++n;
-      // the previous tile's output store has read its staging rows before this tile writes H
-      if (store_read && threadIdx.x == kFfStoreThread) bulk_wait_read<0>();
-      named_barrier_sync(4, 32 * FF_EPI_WARPS);
-      if (*reinterpret_cast<volatile int*>(epi_fail)) return false;
       __syncwarp();
       tc_fence_after();
-      return true;
+      return ok;
     };
     // bias + GELU of the 32 accumulator columns at tensor-memory column tcol (output columns c0 ..
     // c0 + 31), rounded to 16 bf16 pairs
     auto gelu_pack = [&](uint32_t tcol, int c0, uint32_t (&w)[16]) {
       float v[32];
       tmem_ld_32cols(tlane + tcol, v);
-      const float4* b4v = reinterpret_cast<const float4*>(s_bias + c0);
+      const float4* b4v = reinterpret_cast<const float4*>(bias + c0);
 #pragma unroll
       for (int q4 = 0; q4 < 8; ++q4) {
-        const float4 bb = b4v[q4];
+        const float4 bb = __ldg(b4v + q4);
         v[4 * q4] = gelu(v[4 * q4] + bb.x);
         v[4 * q4 + 1] = gelu(v[4 * q4 + 1] + bb.y);
         v[4 * q4 + 2] = gelu(v[4 * q4 + 2] + bb.z);
@@ -832,18 +857,12 @@ fused_forward_kernel(const __grid_constant__ CUtensorMap tma_x, const __grid_con
         *reinterpret_cast<uint4*>(rowp + (((u0 + q) ^ (r & 7)) << 4)) =
             make_uint4(w[4 * q], w[4 * q + 1], w[4 * q + 2], w[4 * q + 3]);
     };
-    for (int tile = blockIdx.x; tile < m_tiles; tile += gridDim.x) {
+    int local = 0;
+    for (int tile = blockIdx.x; tile < tiles_up; tile += gridDim.x, ++local) {
       bool stop = false;
       for (int layer = 0; layer < GF_MLP_LAYERS; ++layer) {
-        // the layer's bias into shared memory while its MMAs run (every epilogue warp passed the
-        // barrier at the end of the previous layer, so the buffer is free)
-        {
-          const float* bias = layer == 0 ? b1 : layer == 1 ? b2 : layer == 2 ? b3 : layer == 3 ? b4 : b5;
-          const int nb = layer < 4 ? HID : OUT_PAD;
-          const int et = threadIdx.x - 64;
-          if (et < nb) s_bias[et] = __ldg(bias + et);
-        }
-        if (!handoff(accA, a_waits, false)) {
+        bias = layer == 0 ? b1 : layer == 1 ? b2 : layer == 2 ? b3 : layer == 3 ? b4 : b5;   // 16-byte aligned, in L1
+        if (!handoff(accA, a_waits)) {
           stop = true;
           break;
         }
@@ -857,7 +876,19 @@ fused_forward_kernel(const __grid_constant__ CUtensorMap tma_x, const __grid_con
             tmem_st_16cols(tlane + cg * 64 + 16 * h, w);
           }
           tmem_st_wait();
-          if (!handoff(accB, b_waits, layer == 0)) {   // every MMA of the layer is done with H
+          // the previous tile's output store has read its staging rows before this tile writes H
+          if (layer == 0 && local > 0) {
+            if (threadIdx.x == kFfStoreThread) {
+              bulk_wait_read<0>();
+              mbar_arrive(sread);
+            }
+            __syncwarp();
+            if (!wait(sread, (local - 1) & 1)) {
+              stop = true;
+              break;
+            }
+          }
+          if (!handoff(accB, b_waits)) {   // every MMA of the layer is done with H
             stop = true;
             break;
           }
@@ -876,19 +907,19 @@ fused_forward_kernel(const __grid_constant__ CUtensorMap tma_x, const __grid_con
           fence_proxy_async_smem();   // H is read by the tensor cores (async proxy)
           tc_fence_before();
           __syncwarp();
-          if (lane == 0) mbar_arrive(hlo);   // H's K blocks 0-3 written, region A drained
-          // N half 1: output columns 256 + cg*64 .. +63 straight into H's K block 4 + cg
+          if (lane == 0) mbar_arrive_remote(hlo, 0);   // H's K blocks 0-3 written, region A drained
+          // N half 1 straight into H, K blocks 4-5 before 6-7, so that the MMAs can follow
 #pragma unroll 1
           for (int h = 0; h < 2; ++h) {
             uint32_t w[16];
-            const int c0 = 256 + cg * 64 + 32 * h;
+            const int c0 = 256 + 128 * h + 32 * cg;
             gelu_pack(c0, c0, w);
             store_h(c0, w);
+            fence_proxy_async_smem();
+            tc_fence_before();
+            __syncwarp();
+            if (lane == 0) mbar_arrive_remote(h == 0 ? hmid : hhi, 0);   // K blocks 4-5; 6-7, region B drained
           }
-          fence_proxy_async_smem();
-          tc_fence_before();
-          __syncwarp();
-          if (lane == 0) mbar_arrive(hhi);   // H's K blocks 4-7 written, region B drained
         } else {
           // layer 5: 128 padded outputs, one 32-column chunk per warp.  The first 99 of each row are
           // staged in H's K blocks 1-4 (row stride 99 words: the lanes' rows fall in distinct banks), and
@@ -901,19 +932,22 @@ fused_forward_kernel(const __grid_constant__ CUtensorMap tma_x, const __grid_con
           float* o = s_out + r * GF_MLP_OUTPUTS;
 #pragma unroll
           for (int j = 0; j < 32; ++j)
-            if (c0 + j < GF_MLP_OUTPUTS) o[c0 + j] = v[j] + s_bias[c0 + j];
+            if (c0 + j < GF_MLP_OUTPUTS) o[c0 + j] = v[j] + __ldg(bias + c0 + j);
           fence_proxy_async_smem();   // the staged rows are read by the bulk copy (async proxy)
           tc_fence_before();
-          named_barrier_sync(4, 32 * FF_EPI_WARPS);   // every row is staged
-          if (threadIdx.x == kFfStoreThread) {
+          __syncwarp();
+          if (lane == 0) {
+            mbar_arrive_remote(hlo, 0);   // region A drained: the next tile's first MMAs may write it
+            mbar_arrive(staged);
+          }
+          if (threadIdx.x == kFfStoreThread && wait(staged, local & 1) && tile < m_tiles) {
             // batch is a multiple of 128 (checked by the caller): the tile's rows are all in range
             bulk_store_1d(out + static_cast<long long>(tile) * BM * GF_MLP_OUTPUTS, s_out,
                           BM * GF_MLP_OUTPUTS * 4);
             bulk_commit();
           }
-          if (lane == 0) mbar_arrive(hlo);   // region A drained: the next tile's first MMAs may write it
+          __syncwarp();
         }
-        named_barrier_sync(4, 32 * FF_EPI_WARPS);   // every warp is done with s_bias before it is refilled
       }
       if (stop) {
         late = true;
@@ -934,13 +968,14 @@ fused_forward_kernel(const __grid_constant__ CUtensorMap tma_x, const __grid_con
         mbar_wait(&wfull[it % FF_WSTAGES], (it / FF_WSTAGES) & 1, wait_limit);
       for (int x = *x_consumed_s; x < x_issued; ++x) mbar_wait(xfull, x & 1, wait_limit);
       if (fault) atomicOr(fault, 1);
-    } else if (threadIdx.x == 32) {
-      umma_commit(drain);
+    } else if (threadIdx.x == 32 && rank == 0) {
+      umma_commit_pair(drain);
       mbar_wait(drain, 0, wait_limit);
     }
     __syncthreads();
   }
-  if (warp == 1) tmem_dealloc(tmem, 512);
+  cluster_sync();   // the other CTA's MMAs, commits and arrivals are done with this one
+  if (warp == 1) tmem_dealloc_pair(tmem, 512);
 }
 
 // ---------------------------------------------------------------------------------------------
@@ -1510,7 +1545,7 @@ cudaError_t launch_train_gemm(int bn, const CUtensorMap& a, const CUtensorMap& a
   return launch_gemm<32, EPI>(a, b[0], c, y, yt, M, HID, K, ep, stream, 0, true);
 }
 
-cudaError_t launch_fused_forward(const CUtensorMap& x, const CUtensorMap* w256, const CUtensorMap& w5,
+cudaError_t launch_fused_forward(const CUtensorMap& x, const CUtensorMap* w,
                                  float* const* bias, float* out, int batch, cudaStream_t stream, int inject,
                                  int* fault) {
   static std::atomic<bool> attr_set[64] = {};
@@ -1522,9 +1557,10 @@ cudaError_t launch_fused_forward(const CUtensorMap& x, const CUtensorMap* w256, 
     attr_set[dev] = true;
   }
   const int m_tiles = batch / BM;
-  const int grid = m_tiles < sm_count() ? m_tiles : sm_count();
+  const int pairs = std::min((m_tiles + 1) / 2, sm_count() / 2);
+  const int grid = 2 * pairs;
   fused_forward_kernel<<<grid, FF_THREADS, FF_SMEM, stream>>>(
-      x, w256[0], w256[1], w256[2], w256[3], w5, bias[0], bias[1], bias[2], bias[3], bias[4], out, batch, m_tiles,
+      x, w[0], w[1], w[2], w[3], w[4], bias[0], bias[1], bias[2], bias[3], bias[4], out, batch, m_tiles,
       inject ? INJECT_WAIT_LIMIT : WAIT_LIMIT, inject, fault);
   return cudaGetLastError();
 }
@@ -1590,6 +1626,7 @@ struct gf_mlp {
   // tensor maps
   CUtensorMap fwd_a[GF_MLP_LAYERS], fwd_b[GF_MLP_LAYERS];     // A = input activations, B = W
   CUtensorMap fwd_b256[4];                                    // B = W in 256-row boxes (inference tiles)
+  CUtensorMap fwd_pair[GF_MLP_LAYERS];                        // B = W in boxes of a paired CTA's half of the rows
   // training: A = input activations, B = W_l in 32-, 64- and 128-row boxes; A = dZ_l (dOut), B = W_l^T likewise
   // (l >= 2); two K blocks a box for tiles of 32 and 64 columns
   CUtensorMap train_a[4], train_b[4][3];
@@ -1657,7 +1694,7 @@ gf_status check_batch(gf_mlp* m, int batch) {
 // caller's [batch][99] array.
 gf_status run_forward_encoded(gf_mlp* m, int batch, float* d_out) {
   if (m->fused) {
-    cudaError_t err = launch_fused_forward(m->fwd_a[0], m->fwd_b256, m->fwd_b[4], m->b, d_out, batch, m->stream,
+    cudaError_t err = launch_fused_forward(m->fwd_a[0], m->fwd_pair, m->b, d_out, batch, m->stream,
                                            m->inject, m->fault);
     m->inject = 0;
     if (err != cudaSuccess) return mlp_fail(m, GF_ERR_CUDA, "fused forward: %s", cudaGetErrorString(err));
@@ -1972,6 +2009,7 @@ gf_status gf_mlp_create(int32_t device, void* stream, const gf_mlp_config* confi
       const void* g_t = l == 4 ? static_cast<const void*>(m->doutt) : m->dzt[l];
       ok = ok && make_map(&m->fwd_a[l], in, cap, m->cols[l], BM);
       ok = ok && make_map(&m->fwd_b[l], m->wb[l], m->rows[l], m->cols[l], 128);
+      ok = ok && make_map(&m->fwd_pair[l], m->wb[l], m->rows[l], m->cols[l], l < 4 ? 128 : OUT_PAD / 2);
       if (l < 4) ok = ok && make_map(&m->fwd_b256[l], m->wb[l], m->rows[l], m->cols[l], 256);
       if (l < 4) {
         const int two = std::min(2, m->cols[l] / BK);
