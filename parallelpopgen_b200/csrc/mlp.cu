@@ -219,8 +219,8 @@ umma_gemm_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constan
   // all of them leave the tile loop together.  An aborted CTA never touches unsynchronised data: it
   // drains what it issued and releases tensor memory.
   auto wait = [&](uint64_t* bar, uint32_t parity) -> bool {
-    if (*abort_flag) return false;
     const uint32_t addr = smem_u32(bar);
+    if (mbar_try_wait(addr, parity)) return true;
     const long long t0 = clock64();
     while (!mbar_try_wait(addr, parity)) {
       if (*abort_flag) return false;
@@ -263,19 +263,19 @@ umma_gemm_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constan
   bool late = false;
   int issued = 0;   // K-blocks the producer issued (for the drain after a timeout)
 
+  // warps 0 and 1 stay converged and elect the lane that issues, which keeps the operands in uniform registers
   if (warp == 0) {
-    if (lane == 0) {
-      int it = 0;
-      for (int tile = blockIdx.x; tile < tiles; tile += gridDim.x) {
-        const int nt = tile % n_tiles, mt = tile / n_tiles;
-        for (int kb = 0; kb < k_blocks; kb += L::KS, ++it) {
-          const int s = it % STAGES;
-          const uint32_t ph = (it / STAGES) & 1;
-          if (!wait(&empty[s], ph ^ 1)) {
-            late = true;
-            goto producer_done;
-          }
-          uint8_t* a = smem + s * L::STAGE_BYTES;
+    int s = 0;
+    uint32_t phase = 1;
+    for (int tile = blockIdx.x; tile < tiles && !late; tile += gridDim.x) {
+      const int nt = tile % n_tiles, mt = tile / n_tiles;
+      for (int kb = 0; kb < k_blocks; kb += L::KS) {
+        if (!wait(&empty[s], phase)) {
+          late = true;
+          break;
+        }
+        uint8_t* a = smem + s * L::STAGE_BYTES;
+        if (elect_one()) {
           if constexpr (L::KS == 1) {
             mbar_arrive_expect_tx(&full[s], L::STAGE_BYTES);
             tma_load_2d(a, &tma_a, kb * BK, mt * BM, &full[s]);
@@ -286,52 +286,61 @@ umma_gemm_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constan
             tma_load_3d(a + L::KS * L::A_BYTES, &tma_b, 0, nt * BN, kb, &full[s]);
           }
         }
+        __syncwarp();
+        ++issued;
+        if (++s == STAGES) {
+          s = 0;
+          phase ^= 1;
+        }
       }
-    producer_done:
-      issued = it;
     }
-    __syncwarp();
   } else if (warp == 1) {
-    if (lane == 0) {
-      constexpr uint32_t idesc = bf16_idesc(BM, BN);
-      int it = 0, local = 0;
-      for (int tile = blockIdx.x; tile < tiles; tile += gridDim.x, ++local) {
-        const int acc = local & 1;
-        const uint32_t use = static_cast<uint32_t>(local >> 1);
-        if (!wait(&tempty[acc], (use & 1) ^ 1)) {
+    constexpr uint32_t idesc = bf16_idesc(BM, BN);
+    const uint64_t desc = sw128_kmajor_desc(smem_u32(smem));
+    int s = 0, received = 0, local = 0;
+    uint32_t phase = 0;
+    for (int tile = blockIdx.x; tile < tiles && !late; tile += gridDim.x, ++local) {
+      const int acc = local & 1;
+      const uint32_t use = static_cast<uint32_t>(local >> 1);
+      if (!wait(&tempty[acc], (use & 1) ^ 1)) {
+        late = true;
+        break;
+      }
+      tc_fence_after();
+      const uint32_t d = tmem + static_cast<uint32_t>(acc * BN);
+      for (int kb = 0; kb < k_blocks; kb += L::KS) {
+        if (!wait(&full[s], phase)) {
           late = true;
           break;
         }
+        ++received;
         tc_fence_after();
-        const uint32_t d = tmem + static_cast<uint32_t>(acc * BN);
-        bool stop = false;
-        for (int kb = 0; kb < k_blocks; kb += L::KS, ++it) {
-          const int s = it % STAGES;
-          const uint32_t ph = (it / STAGES) & 1;
-          if (!wait(&full[s], ph)) {
-            late = true;
-            stop = true;
-            break;
-          }
-          tc_fence_after();
-          const uint32_t stage = smem_u32(smem + s * L::STAGE_BYTES);
+        // descriptor addresses count 16 bytes
+        const uint64_t a = desc + s * (L::STAGE_BYTES >> 4), b = a + (L::KS * L::A_BYTES >> 4);
+        if (elect_one()) {
 #pragma unroll
           for (int h = 0; h < L::KS; ++h) {
-            if (kb + h >= k_blocks) break;
-            const uint32_t a_addr = stage + h * L::A_BYTES, b_addr = stage + L::KS * L::A_BYTES + h * L::B_BYTES;
+            if (kb + h < k_blocks) {
 #pragma unroll
-            for (int kk = 0; kk < BK / 16; ++kk)
-              umma_bf16(d, sw128_kmajor_desc(a_addr + kk * 32), sw128_kmajor_desc(b_addr + kk * 32), idesc,
-                        (kb | h | kk) != 0);
+              for (int kk = 0; kk < BK / 16; ++kk)
+                umma_bf16(d, a + h * (L::A_BYTES >> 4) + 2 * kk, b + h * (L::B_BYTES >> 4) + 2 * kk, idesc,
+                          (kb | h | kk) != 0);
+            }
           }
           umma_commit(&empty[s]);
         }
-        if (stop) break;
-        // fault injection for tests: withhold the first accumulator hand-off
-        if (!((inject & 1) && local == 0)) umma_commit(&tfull[acc]);
+        __syncwarp();
+        if (++s == STAGES) {
+          s = 0;
+          phase ^= 1;
+        }
       }
-      *consumed_s = it;
+      if (late) break;
+      // fault injection for tests: withhold the first accumulator hand-off
+      if (!((inject & 1) && local == 0) && elect_one()) umma_commit(&tfull[acc]);
+      __syncwarp();
     }
+    if (lane == 0) *consumed_s = received;
     __syncwarp();
   } else {
     // epilogue warps: TMEM lane quarter = warp % 4; the two warps of a quarter take alternate
@@ -525,8 +534,8 @@ umma_gemm_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constan
       // loads issued but never received by the MMA thread are still landing
       for (int it = *consumed_s; it < issued; ++it) mbar_wait(&full[it % STAGES], (it / STAGES) & 1, wait_limit);
       if (ep.fault) atomicOr(ep.fault, 1);
-    } else if (threadIdx.x == 32) {
-      umma_commit(drain);   // arrives once every MMA this thread issued has completed
+    } else if (warp == 1) {
+      if (elect_one()) umma_commit(drain);   // arrives once every MMA that lane issued has completed
       mbar_wait(drain, 0, wait_limit);
     }
     __syncthreads();
@@ -968,8 +977,8 @@ fused_forward_kernel(const __grid_constant__ CUtensorMap tma_x, const __grid_con
         mbar_wait(&wfull[it % FF_WSTAGES], (it / FF_WSTAGES) & 1, wait_limit);
       for (int x = *x_consumed_s; x < x_issued; ++x) mbar_wait(xfull, x & 1, wait_limit);
       if (fault) atomicOr(fault, 1);
-    } else if (threadIdx.x == 32 && rank == 0) {
-      umma_commit_pair(drain);
+    } else if (warp == 1 && rank == 0) {
+      if (elect_one()) umma_commit_pair(drain);
       mbar_wait(drain, 0, wait_limit);
     }
     __syncthreads();
@@ -1073,7 +1082,7 @@ __global__ void encode_inputs_kernel(const float* __restrict__ x, const long lon
 // caller asked for it.  Further blocks do the biases (partials summed in tile order) and the loss.
 //
 // At a batch of 1,024 the five GEMMs, their reduction over 27 MB of slices and Adam took 29 + 10 + 17 us in seven
-// launches; here they take 13 us.
+// launches; here they take one of 13 us.
 constexpr int DW_BN = 64;
 constexpr int DW_EPI_WARPS = 8;
 constexpr int DW_THREADS = 64 + 32 * DW_EPI_WARPS;
@@ -1175,8 +1184,8 @@ __global__ void __launch_bounds__(DW_THREADS, 1) weight_update_kernel(const __gr
   volatile int* abort_flag = timed_out;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   auto wait = [&](uint64_t* bar, uint32_t parity) -> bool {   // as in umma_gemm_kernel
-    if (*abort_flag) return false;
     const uint32_t addr = smem_u32(bar);
+    if (mbar_try_wait(addr, parity)) return true;
     const long long t0 = clock64();
     while (!mbar_try_wait(addr, parity)) {
       if (*abort_flag) return false;
@@ -1214,55 +1223,68 @@ __global__ void __launch_bounds__(DW_THREADS, 1) weight_update_kernel(const __gr
   int issued = 0;
 
   if (warp == 0) {
-    if (lane == 0) {
-      int it = 0;
-      for (; it < A.k_blocks / DW_KS; ++it) {
-        const int s = it % DW_STAGES;
-        if (!wait(&empty[s], ((it / DW_STAGES) & 1) ^ 1)) {
-          late = true;
-          break;
-        }
-        uint8_t* a = smem + s * DW_STAGE_BYTES;
-        mbar_arrive_expect_tx(&full[s], DW_STAGE_BYTES);
-        tma_load_3d(a, &L.a, 0, mt * BM, it * DW_KS, &full[s]);
-        tma_load_3d(a + DW_KS * DW_A_BYTES, &L.b, 0, nt * DW_BN, it * DW_KS, &full[s]);
+    int s = 0;
+    uint32_t phase = 1;
+    for (; issued < A.k_blocks / DW_KS; ++issued) {
+      if (!wait(&empty[s], phase)) {
+        late = true;
+        break;
       }
-      issued = it;
+      uint8_t* a = smem + s * DW_STAGE_BYTES;
+      if (elect_one()) {
+        mbar_arrive_expect_tx(&full[s], DW_STAGE_BYTES);
+        tma_load_3d(a, &L.a, 0, mt * BM, issued * DW_KS, &full[s]);
+        tma_load_3d(a + DW_KS * DW_A_BYTES, &L.b, 0, nt * DW_BN, issued * DW_KS, &full[s]);
+      }
+      __syncwarp();
+      if (++s == DW_STAGES) {
+        s = 0;
+        phase ^= 1;
+      }
     }
-    __syncwarp();
   } else if (warp == 1) {
-    if (lane == 0) {
-      constexpr uint32_t idesc = bf16_idesc(BM, DW_BN);
-      int blk = 0, received = 0;
-      for (int sp = 0; sp < L.splits && !late; ++sp) {
-        const int acc = sp & 1;
-        if (!wait(&tempty[acc], ((sp >> 1) & 1) ^ 1)) {
-          late = true;
-          break;
-        }
-        tc_fence_after();
-        for (int kb = 0; kb < per_split; ++kb, ++blk) {   // a split may end within a stage
-          const int it = blk / DW_KS, h = blk % DW_KS, s = it % DW_STAGES;
-          if (h == 0) {
-            if (!wait(&full[s], (it / DW_STAGES) & 1)) {
-              late = true;
-              break;
-            }
-            ++received;
-            tc_fence_after();
+    constexpr uint32_t idesc = bf16_idesc(BM, DW_BN);
+    const uint64_t desc = sw128_kmajor_desc(smem_u32(smem));
+    int s = 0, h = 0, received = 0;   // a split may end within a stage
+    uint32_t phase = 0;
+    for (int sp = 0; sp < L.splits && !late; ++sp) {
+      const int acc = sp & 1;
+      if (!wait(&tempty[acc], ((sp >> 1) & 1) ^ 1)) {
+        late = true;
+        break;
+      }
+      tc_fence_after();
+      for (int kb = 0; kb < per_split; ++kb) {
+        if (h == 0) {
+          if (!wait(&full[s], phase)) {
+            late = true;
+            break;
           }
-          const uint32_t stage = smem_u32(smem + s * DW_STAGE_BYTES);
-          const uint32_t a_addr = stage + h * DW_A_BYTES, b_addr = stage + DW_KS * DW_A_BYTES + h * DW_B_BYTES;
+          ++received;
+          tc_fence_after();
+        }
+        const uint64_t a = desc + s * (DW_STAGE_BYTES >> 4) + h * (DW_A_BYTES >> 4);
+        const uint64_t b = desc + s * (DW_STAGE_BYTES >> 4) + (DW_KS * DW_A_BYTES >> 4) + h * (DW_B_BYTES >> 4);
+        if (elect_one()) {
 #pragma unroll
           for (int kk = 0; kk < BK / 16; ++kk)
-            umma_bf16(tmem + acc * DW_BN, sw128_kmajor_desc(a_addr + kk * 32), sw128_kmajor_desc(b_addr + kk * 32), idesc,
-                      (kb | kk) != 0);
+            umma_bf16(tmem + acc * DW_BN, a + 2 * kk, b + 2 * kk, idesc, (kb | kk) != 0);
           if (h == DW_KS - 1) umma_commit(&empty[s]);
         }
-        if (!late) umma_commit(&tfull[acc]);
+        __syncwarp();
+        if (++h == DW_KS) {
+          h = 0;
+          if (++s == DW_STAGES) {
+            s = 0;
+            phase ^= 1;
+          }
+        }
       }
-      *consumed_s = received;
+      if (late) break;
+      if (elect_one()) umma_commit(&tfull[acc]);
+      __syncwarp();
     }
+    if (lane == 0) *consumed_s = received;
     __syncwarp();
   } else {
     // epilogue warps: one 32 x 32 piece each (tensor-memory lane quarter, column half)
@@ -1354,8 +1376,8 @@ __global__ void __launch_bounds__(DW_THREADS, 1) weight_update_kernel(const __gr
     if (threadIdx.x == 0) {
       for (int it = *consumed_s; it < issued; ++it) mbar_wait(&full[it % DW_STAGES], (it / DW_STAGES) & 1, A.wait_limit);
       if (A.fault) atomicOr(A.fault, 1);
-    } else if (threadIdx.x == 32) {
-      umma_commit(drain);
+    } else if (warp == 1) {
+      if (elect_one()) umma_commit(drain);
       mbar_wait(drain, 0, A.wait_limit);
     }
     __syncthreads();
@@ -1825,8 +1847,8 @@ gf_status run_predict(gf_mlp* m, const double* params, long long rows, const gf_
 // the one before (grid_wait).  idx: the batch's rows of d_inputs and d_targets (null: the first `batch`).
 //
 // Latency-bound at small batches: a chain of eleven kernels whose K loops are 1 to 8 blocks long.  At 1,024 a step
-// takes 88 us (97 with one K block a TMA box, 107 without the overlapped launches); in 23 separate launches it was
-// 230 us of kernels.  At 4,096: 149 us.
+// takes 76 us; with single-lane producer and issue code 88, with one K block a TMA box as well 97, without the
+// overlapped launches 107; in 23 separate launches it was 230 us of kernels.  At 128: 68 us, at 4,096: 120.
 gf_status run_step(gf_mlp* m, const float* d_inputs, const float* d_targets, const long long* idx, int batch,
                    const AdamArgs* adam, float* d_loss) {
   cudaError_t err = launch_dependent(encode_inputs_kernel, (batch + 255) / 256, 256, 0, m->stream, d_inputs, idx, batch,
