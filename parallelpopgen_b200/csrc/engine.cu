@@ -1005,7 +1005,7 @@ static bool window_eligible(const Engine* e, const gf_generation& g) {
 
 constexpr int kMaxWindow = kMaxWindowGenerations;
 
-// Generations a multi-population window may hold (2 <= P <= 4): every population is either drifted
+// Generations a multi-population window may hold (2 <= P <= 8): every population is either drifted
 // with Nc > 0, or not drifted and its rows are zero in both state buffers (`live`: the populations
 // whose rows may hold a nonzero value, given the generations before this one).  Extinction
 // generations and every generation after an extinction run one launch each.
@@ -1253,7 +1253,7 @@ static gf_status run_batch(Engine* e, const gf_generation* gens, int n) {
     if (windows_mp && window_mp_eligible(e, gens[i], e->live_rows)) {
       int j = i;
       int live = e->live_rows;
-      while (j < n && j - i < kMaxWindow && window_mp_eligible(e, gens[j], live)) {
+      while (j < n && j - i < mp_max_window(e->P) && window_mp_eligible(e, gens[j], live)) {
         live |= drift_bits(gens[j], e->P);
         const bool ends = e->h_table[b][j].flag != 0;
         ++j;

@@ -422,7 +422,11 @@ gf_status window_mp_run(Engine* e, const WindowMpLaunch& w);
 // The compaction of a `small` one into dst, posting the survivor count to mail.
 gf_status compact_mp_run(Engine* e, const WindowMpLaunch& w, float* dst, int* gp_dst, int* tid_dst, bool preserve,
                          unsigned long long* mail, unsigned tag);
-constexpr int kMaxWindowPops = 4;
+// Populations a window may hold: up to eight the records, rows and lists of a block fit in 48 KB of shared memory.
+// Generations of 5 to 8 populations as windows of 25 against one launch each: see window_mp.cu.
+constexpr int kMaxWindowPops = 8;
+// Longest window of P populations: its records stay within 30 KB of shared memory.
+constexpr int mp_max_window(int P) { return P <= 4 ? kMaxWindowGenerations : 64; }
 
 // Host draw of one population's new-mutation count (engine.cu).
 int host_new_mutation_count(int seed1, int seed2, float mu, int Nchrom_e, float num_sites, int generation, int pop);

@@ -1637,7 +1637,7 @@ struct gf_mlp {
   float* loss = nullptr;
   int* fault = nullptr;
 
-  // host queries (gf_mlp_predict), once there has been one: rows at a time; device parameters, outputs and
+  // host queries (gf_mlp_predict): rows at a time; device parameters, outputs and
   // spectra; the page-locked ring (and one chunk's parameters), an event a chunk of it
   long long q_rows = 0;
   double *q_params = nullptr, *q_spec = nullptr;
@@ -1748,7 +1748,7 @@ gf_status run_forward(gf_mlp* m, const float* d_inputs, int batch, float* d_out)
   return run_forward_encoded(m, batch, d_out);
 }
 
-// Buffers of gf_mlp_predict, made by its first call: at most kQueryRows rows are on the device at once, and their
+// Buffers of gf_mlp_predict: at most kQueryRows rows are on the device at once, and their
 // spectra come back in chunks through a page-locked ring of four, each copied to the caller while others are on
 // their way.  The ring is short because page-locking 3 MB takes longer than several queries.
 constexpr long long kQueryRows = 64 * BM;
@@ -2069,6 +2069,10 @@ gf_status gf_mlp_create(int32_t device, void* stream, const gf_mlp_config* confi
     }
   }
 #undef MLP_TRY
+  if (query_buffers(m) != GF_OK) {   // the first query tries again, and reports it
+    cudaGetLastError();
+    m->error.clear();
+  }
   *out = m;
   return GF_OK;
 bad:

@@ -1,4 +1,4 @@
-// Windowed drift for 2 to 4 populations: every generation of a compaction window in one launch.
+// Windowed drift for 2 to 8 populations: every generation of a compaction window in one launch.
 //
 // Migration mixes the frequencies of one mutation across populations and nothing else, so a thread
 // can carry the P rows of one slot through all generations of a window, as the single-population
@@ -32,10 +32,12 @@ namespace gf {
 // Issue-bound (76 % of issue slots, 24 of 32 lanes).  Windows of 25 generations on a B200, against a quad per
 // thread with the rows of its four slots in registers (four blocks an SM, lost slots carried along): three
 // populations, N = 50,000, L = 1e8 (35 generations, 1.6 M slots at the end) 462 -> 370 us; two, N = 100,000 285 -> 265;
-// four, N = 30,000 391 -> 282; three of N = 2,000 to 20,000 (4,000 to 130,000 slots) 137 -> 50 to 61.  Packing at half
+// four, N = 30,000 391 -> 282; three of N = 2,000 to 20,000 (4,000 to 130,000 slots) 137 -> 50 to 61.  Five to
+// eight populations, which had a launch per generation: 25 generations of six, N = 2,000 532 -> 87 us, N = 30,000,
+// L = 5e7 776 -> 398; of eight 637 -> 111, N = 30,000, L = 4e7 982 -> 604.  Packing at half
 // the tile instead of three quarters: the same within 1 %.
-// Resident blocks: 5 (48 registers), 4 for four populations, whose rows would spill.  6 is 10 % slower for three.
-constexpr int mp_min_blocks(int P, bool small) { return small ? 8 : P == 4 ? 4 : 5; }
+// Resident blocks: 5 (48 registers), 4 from four populations on, whose rows would spill.  6 is 10 % slower for three.
+constexpr int mp_min_blocks(int P, bool small) { return small ? (P <= 4 ? 8 : 6) : P <= 3 ? 5 : P <= 4 ? 4 : 3; }
 
 // Slots of a thread, threads of a block: large states hand out half compaction tiles (512 slots; a whole one is
 // too coarse for the few hundred that carry the old mutations) and pack them; small ones spread over many SMs.
@@ -47,6 +49,11 @@ struct MpShape {
 };
 static_assert(2 * MpShape<false>::kTile == kTileSlots, "a window tile is half a compaction tile");
 static_assert(MpShape<true>::kThreads >= kMaxWindowGenerations, "a thread per record");
+
+template <int P>
+struct MpLimit {
+  static constexpr int kGens = mp_max_window(P);
+};
 
 // The fields of one generation record the drift reads.
 template <int P>
@@ -111,14 +118,17 @@ template <int P, bool QUAD>
 __device__ __forceinline__ void mp_generation(float (&x)[P], bool live, int e, const MpGen<P>& G, const PhiloxKeys& keys,
                                               int lane) {
   const uint32_t q2 = static_cast<uint32_t>((e >> 2) + 2), g = static_cast<uint32_t>(G.generation);
-  uint32_t bits[4];
+  uint32_t bits[(P + 3) / 4][4];
   if (QUAD) {
-    const uint4 r = philox4x32_10_keys(make_uint4(q2, g, static_cast<uint32_t>(lane & 3), 0u), keys);
-    bits[0] = r.x;
-    bits[1] = r.y;
-    bits[2] = r.z;
-    bits[3] = r.w;
-    transpose_quad(bits, lane);
+#pragma unroll
+    for (int b = 0; b < (P + 3) / 4; ++b) {   // four populations at a time
+      const uint4 r = philox4x32_10_keys(make_uint4(q2, g, static_cast<uint32_t>(4 * b + (lane & 3)), 0u), keys);
+      bits[b][0] = r.x;
+      bits[b][1] = r.y;
+      bits[b][2] = r.z;
+      bits[b][3] = r.w;
+      transpose_quad(bits[b], lane);
+    }
   }
   if (!live) return;
   float xm[P];
@@ -136,7 +146,7 @@ __device__ __forceinline__ void mp_generation(float (&x)[P], bool live, int e, c
       if (xs != 0.f) {
         uint32_t b;
         if (QUAD) {
-          b = bits[p];
+          b = bits[p / 4][p % 4];
         } else {
           const uint4 r = philox4x32_10_keys(make_uint4(q2, g, static_cast<uint32_t>(p), 0u), keys);
           b = (e & 2) ? ((e & 1) ? r.w : r.z) : ((e & 1) ? r.y : r.x);
@@ -250,7 +260,7 @@ __global__ void __launch_bounds__(MpShape<SMALL>::kThreads, mp_min_blocks(P, SMA
                      const GenArgs* __restrict__ table, int ngen, long long births, int compact, int check_preserved,
                      int seed1, int seed2, unsigned long long* __restrict__ stats, const PhiloxKeys keys) {
   constexpr int kThreads = MpShape<SMALL>::kThreads, kSlots = MpShape<SMALL>::kSlots, kTile = MpShape<SMALL>::kTile;
-  __shared__ MpGen<P> s_gen[kMaxWindowGenerations];
+  __shared__ MpGen<P> s_gen[MpLimit<P>::kGens];
   __shared__ float s_x[SMALL ? 1 : P][SMALL ? 1 : kTile];
   __shared__ unsigned short s_list[2][SMALL ? 1 : kTile];
   __shared__ int s_part[2][kThreads / 32];
@@ -539,11 +549,15 @@ static void launch_compact_mp(Engine* e, const WindowMpLaunch& w, float* dst, in
 }
 
 gf_status window_mp_run(Engine* e, const WindowMpLaunch& w) {
-  if (w.ngen < 1 || w.ngen > kMaxWindowGenerations) return fail(e, GF_ERR_INVALID_ARGUMENT, "window of %d generations", w.ngen);
+  if (w.ngen < 1 || w.ngen > mp_max_window(w.P)) return fail(e, GF_ERR_INVALID_ARGUMENT, "window of %d generations", w.ngen);
   switch (w.P) {
     case 2: launch_mp_sized<2>(e, w); break;
     case 3: launch_mp_sized<3>(e, w); break;
     case 4: launch_mp_sized<4>(e, w); break;
+    case 5: launch_mp_sized<5>(e, w); break;
+    case 6: launch_mp_sized<6>(e, w); break;
+    case 7: launch_mp_sized<7>(e, w); break;
+    case 8: launch_mp_sized<8>(e, w); break;
     default: return fail(e, GF_ERR_INVALID_ARGUMENT, "multi-population window for %d populations", w.P);
   }
   GF_CUDA(e, cudaGetLastError());
@@ -557,7 +571,11 @@ gf_status compact_mp_run(Engine* e, const WindowMpLaunch& w, float* dst, int* gp
   switch (w.P) {
     case 2: launch_compact_mp<2>(e, w, dst, gp_dst, tid_dst, preserve, mail, tag); break;
     case 3: launch_compact_mp<3>(e, w, dst, gp_dst, tid_dst, preserve, mail, tag); break;
-    default: launch_compact_mp<4>(e, w, dst, gp_dst, tid_dst, preserve, mail, tag); break;
+    case 4: launch_compact_mp<4>(e, w, dst, gp_dst, tid_dst, preserve, mail, tag); break;
+    case 5: launch_compact_mp<5>(e, w, dst, gp_dst, tid_dst, preserve, mail, tag); break;
+    case 6: launch_compact_mp<6>(e, w, dst, gp_dst, tid_dst, preserve, mail, tag); break;
+    case 7: launch_compact_mp<7>(e, w, dst, gp_dst, tid_dst, preserve, mail, tag); break;
+    default: launch_compact_mp<8>(e, w, dst, gp_dst, tid_dst, preserve, mail, tag); break;
   }
   GF_CUDA(e, cudaGetLastError());
   e->kernel_launches += 1;

@@ -8,16 +8,24 @@ import pytest
 
 from parallelpopgen_b200 import Engine
 
-from test_gpu_window_mp import assert_same, mse_start, run_both, schedule
+from test_gpu_window_mp import assert_same, mse_start, run_both
+from test_gpu_window_mp import schedule as schedule_four
+
+
+def schedule(P, *args, **kw):
+    """The schedule with inbreeding and dominance for eight populations."""
+    return schedule_four(P, *args, F=(0.0, 0.0, 0.2, 0.1, 0.0, 0.3, 0.0, 0.1),
+                         h=(0.5, 0.3, 0.5, 0.8, 0.1, 0.6, 0.5, 0.0), **kw)
+
 
 pytestmark = pytest.mark.gpu
 
 
 # a window ends with under 600,000 slots at the two smaller sizes, with a million and more at the largest
-@pytest.mark.parametrize("P", [2, 3, 4])
+@pytest.mark.parametrize("P", [2, 3, 4, 5, 6, 7, 8])
 @pytest.mark.parametrize("num_sites", [2e5, 2e7, 1.5e8])
 def test_windows_of_every_size(P, num_sites):
-    gens = schedule(P, 1, 110, found=(0, 1, 30), compact_interval=25, sample_every=60)
+    gens = schedule(P, 1, 110, found=(0, 1, 10), compact_interval=25, sample_every=60)
     out = run_both(lambda e: e.begin_mse(mse_start(P), seed1=7, seed2=8, num_sites=num_sites, compact_interval=25),
                    [gens])
     l1, l0 = assert_same(out, min_slots=100)
@@ -51,3 +59,13 @@ def test_resumed_states_of_edge_sizes(M):
     gens = schedule(2, 1, 40, found=(0, 1), sizes=(2000, 2000), mu=0.0, compact_interval=17)
     out = run_both(lambda e: e.begin_from_state(freq, ids, seed1=1, seed2=2, num_sites=2e6, compact_interval=17), [gens])
     assert_same(out, min_slots=0 if M < 200 else M // 8)
+
+
+@pytest.mark.parametrize("P", [4, 5, 8])
+def test_windows_at_their_length_limit(P):
+    """128 generations up to four populations, 64 above; without compactions a window ends there."""
+    gens = schedule(P, 1, 200, compact_interval=0, sample_every=10**6)
+    gens["compact"] = 0
+    gens["preserve"] = 0
+    out = run_both(lambda e: e.begin_mse(mse_start(P), seed1=3, seed2=4, num_sites=3e5, compact_interval=0), [gens])
+    assert_same(out, min_slots=100)
