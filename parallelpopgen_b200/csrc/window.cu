@@ -637,7 +637,7 @@ __global__ void __launch_bounds__(kWinThreads)
 // its quad's Philox block alone), repacking every few generations.  A slot's counters depend on its position
 // only, so who computes it does not matter.  Lost slots cost nothing from then on.
 //
-// Issue-bound (78 % of issue slots, 25 of 32 lanes).  Windows of 25 generations on a B200, against a quad per
+// Issue-bound (79 % of issue slots, 23 of 32 lanes).  Windows of 25 generations on a B200, against a quad per
 // thread throughout (window_kernel): N = 2e5, L = 2.5e8, neutral 354 -> 293 us, gamma = -10 357 -> 293; N = 1e4 with 4
 // million slots 201 -> 157; the batched windows of 256 replicates (N0 in [1e3, 1e4]) 400 -> 310 ms in all.
 // A third of that is the shorter draw (binom_draw_count) and generation loop: 20 % fewer warp instructions.
