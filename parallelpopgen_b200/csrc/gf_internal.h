@@ -122,6 +122,7 @@ struct WindowLaunch {
   // keys from its seeds, as kernel parameters
   WinRep one{};
   long long expected_slots = 0;   // about how many slots it ends with (which kernels run it, not what they do)
+  bool pack = true;               // packing pays (likewise)
   // where the compaction also stores the survivor count (tagged), in page-locked host memory; null: nowhere
   unsigned long long* mail = nullptr;
   unsigned mail_tag = 0;
@@ -239,6 +240,7 @@ struct Batch {
   std::vector<int> active;                    // unfinished replicates, in index order
   bool active_dirty = true;
   long long active_cadence_sum = 0;           // sum of their cadences (generations per super-step)
+  bool pack = true;                           // windows pack living slots (refresh_active)
   std::vector<std::vector<int>> finish_at;    // [k]: replicates whose last window is super-step k
   // precomputed records: a replicate table of all R replicates in index order, whose per-window fields
   // (records, generations, tiles, births; none once finished) a kernel derives from the super-step

@@ -1146,10 +1146,11 @@ static int resident_blocks(Kernel kernel) {
   return o;
 }
 
-// One large or several replicates: lane order on the packing kernel, the other draw schedules on window_kernel.
+// One large or several replicates: lane order on the packing kernel where that pays, else, and for the other draw
+// schedules, window_kernel.
 template <int DRAW, bool KEYS>
 static void launch_window_kernel(Engine* e, const WindowLaunch& w) {
-  if constexpr (DRAW == kDrawLanes) {
+  if (DRAW == kDrawLanes && w.pack) {
     static const int occupancy = resident_blocks(window_pack_kernel<KEYS>);   // thread-safe, once
     launch_window_tiles<KEYS>(e, w, window_pack_kernel<KEYS>, occupancy);
   } else {
