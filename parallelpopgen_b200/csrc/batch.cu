@@ -521,6 +521,7 @@ static gf_status batch_begin(Engine* e, const gf_replicate* in, int R) {
   Batch* b = new Batch();
   e->batch = b;
   b->R = R;
+  b->longest = longest_window(in, R);
   b->reps.resize(R);
   // ---- MSE classes ----
   std::vector<MseRep> mr(R);
@@ -790,6 +791,7 @@ static gf_status enqueue_step(Engine* e, Batch* b) {
   w.total_tiles_dev = b->d_total_tiles;
   w.any_compact = true;
   w.pack = b->pack;
+  w.longest = b->longest;
   w.stats = e->d_stats;
   w.fault = e->d_count + 2;
   w.sched = e->d_count + kSchedWord;
@@ -1016,6 +1018,7 @@ static gf_status batch_super_step_fallback(Engine* e, int* active_out) {
   w.total_tiles = tiles;
   w.any_compact = true;
   w.pack = b->pack;
+  w.longest = b->longest;
   w.stats = e->d_stats;
   w.fault = e->d_count + 2;
   w.sched = e->d_count + kSchedWord;

@@ -1056,6 +1056,7 @@ static gf_status launch_window(Engine* e, int b, int first, int count, const Gen
   w.nreps = 1;
   w.recs = e->d_wgen[b];
   w.total_tiles = R.ntiles;
+  w.longest = count;
   w.expected_slots = std::min(need, e->M_recent + news);
   w.any_compact = R.compact != 0;
   w.stats = e->d_stats;

@@ -123,6 +123,7 @@ struct WindowLaunch {
   WinRep one{};
   long long expected_slots = 0;   // about how many slots it ends with (which kernels run it, not what they do)
   bool pack = true;               // packing pays (likewise)
+  int longest = 0;                // generations of the longest window in the launch
   // where the compaction also stores the survivor count (tagged), in page-locked host memory; null: nowhere
   unsigned long long* mail = nullptr;
   unsigned mail_tag = 0;
@@ -132,9 +133,6 @@ struct WindowLaunch {
 // Words of the engine's device counter block (d_count) and the first of the window scheduler's two.
 constexpr int kCountWords = 8;
 constexpr int kSchedWord = 4;
-
-// Longest window (generations per window launch).
-constexpr int kMaxWindowGenerations = 128;
 
 // One multi-population window launch of the plain engine (window_mp.cu): generations
 // table[0 .. ngen) from state A into state B, counts in d_count[slot_in] -> d_count[slot_out] (and
@@ -241,6 +239,7 @@ struct Batch {
   bool active_dirty = true;
   long long active_cadence_sum = 0;           // sum of their cadences (generations per super-step)
   bool pack = true;                           // windows pack living slots (refresh_active)
+  int longest = 0;                            // generations of the longest window
   std::vector<std::vector<int>> finish_at;    // [k]: replicates whose last window is super-step k
   // precomputed records: a replicate table of all R replicates in index order, whose per-window fields
   // (records, generations, tiles, births; none once finished) a kernel derives from the super-step

@@ -1,7 +1,7 @@
 // Host-only planning logic of the engine, free of CUDA so that it compiles and is tested with a plain
 // C++ compiler: the layout of the batched engine's generation records (regions of slabs, resident or
-// cycling through a ring of slots), the lock-step finishing schedule of its replicates, and which
-// generations a multi-population window may hold.
+// cycling through a ring of slots), the lock-step finishing schedule of its replicates, which
+// generations a multi-population window may hold, and which kernel runs a window.
 #pragma once
 
 #include <algorithm>
@@ -117,6 +117,36 @@ inline bool mp_window_generation_ok(const gf_generation& g, int P, int live_rows
     }
   }
   return true;
+}
+
+// Generations whose records a block of the single- or multi-population window kernels stages in shared memory.
+// The plain engine ends its windows there; a batched replicate's window is its compaction cadence, of any length.
+constexpr int kMaxWindowGenerations = 128;
+
+// Generations of the longest window of a batch.
+inline int longest_window(const gf_replicate* reps, int R) {
+  int n = 0;
+  for (int r = 0; r < R; ++r) n = std::max(n, std::min(reps[r].compact_interval, reps[r].num_generations));
+  return n;
+}
+
+// Expected slots (at the window's end) up to which one replicate's window runs a slot per thread.  Window
+// kernels of 25 generations on a B200, a slot per thread against the packing kernel: 23 / 53 us at 12,000
+// slots, 27 / 55 at 92,000, 50 / 70 at 368,000, 74 / 80 at 552,000 (N = 1e4, neutral), 92 / 104 at 648,000 (gamma = -10),
+// 86 / 86 at 625,000, 98 / 90 at 736,000 and 111 / 94 at 833,000 (neutral, N = 1e4 and 2e5).
+#ifndef GF_SLOT_WINDOW_SLOTS
+#define GF_SLOT_WINDOW_SLOTS 600000
+#endif
+constexpr long long kSlotWindowSlots = GF_SLOT_WINDOW_SLOTS;
+
+// The kernel of a single-population window launch: a slot per thread (one small replicate), a quad per thread
+// with the living slots packed later (where packing pays), or a quad per thread throughout.  The first two stage
+// the window's records, so a launch that holds a longer window takes the third, which reads them from memory.
+enum class WindowForm { slots, pack, quads };
+inline WindowForm window_form(bool single, bool lane_order, bool pack, long long expected_slots, int longest) {
+  if (!lane_order || longest > kMaxWindowGenerations) return WindowForm::quads;
+  if (single && expected_slots <= kSlotWindowSlots) return WindowForm::slots;
+  return pack ? WindowForm::pack : WindowForm::quads;
 }
 
 inline int drifted_populations(const gf_generation& g, int P) {

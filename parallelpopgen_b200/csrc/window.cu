@@ -1146,11 +1146,10 @@ static int resident_blocks(Kernel kernel) {
   return o;
 }
 
-// One large or several replicates: lane order on the packing kernel where that pays, else, and for the other draw
-// schedules, window_kernel.
+// One large or several replicates: window_pack_kernel (lane order only) or window_kernel.
 template <int DRAW, bool KEYS>
-static void launch_window_kernel(Engine* e, const WindowLaunch& w) {
-  if (DRAW == kDrawLanes && w.pack) {
+static void launch_window_kernel(Engine* e, const WindowLaunch& w, WindowForm form) {
+  if (DRAW == kDrawLanes && form == WindowForm::pack) {
     static const int occupancy = resident_blocks(window_pack_kernel<KEYS>);   // thread-safe, once
     launch_window_tiles<KEYS>(e, w, window_pack_kernel<KEYS>, occupancy);
   } else {
@@ -1159,21 +1158,13 @@ static void launch_window_kernel(Engine* e, const WindowLaunch& w) {
   }
 }
 
-// Expected slots (at the window's end) up to which one replicate's window runs a slot per thread.  Window
-// kernels of 25 generations on a B200, a slot per thread against the packing kernel: 23 / 53 us at 12,000
-// slots, 27 / 55 at 92,000, 50 / 70 at 368,000, 74 / 80 at 552,000 (N = 1e4, neutral), 92 / 104 at 648,000 (gamma = -10),
-// 86 / 86 at 625,000, 98 / 90 at 736,000 and 111 / 94 at 833,000 (neutral, N = 1e4 and 2e5).
-#ifndef GF_SLOT_WINDOW_SLOTS
-#define GF_SLOT_WINDOW_SLOTS 600000
-#endif
-constexpr long long kSlotWindowSlots = GF_SLOT_WINDOW_SLOTS;
-
 // Launch a window over w.nreps replicates (one passed by value) and, for the replicates that compact, the
 // segmented scan and scatter into `compact_dst` (the other state buffer).
 gf_status window_run(Engine* e, const WindowLaunch& w, float* compact_dst, cudaEvent_t after_window,
                      cudaEvent_t before_compaction) {
   const bool single = w.reps == nullptr;
-  const bool slots = single && w.expected_slots <= kSlotWindowSlots && e->draw_strategy == kDrawLanes;
+  const WindowForm form = window_form(single, e->draw_strategy == kDrawLanes, w.pack, w.expected_slots, w.longest);
+  const bool slots = form == WindowForm::slots;
   if (slots) {
     const long long blocks = (w.one.ntiles * static_cast<long long>(kWinTile) + kSlotThreads - 1) / kSlotThreads;
     window_slots_kernel<<<static_cast<int>(std::max(1ll, std::min(blocks, 16ll * e->num_sms))), kSlotThreads, 0,
@@ -1182,24 +1173,24 @@ gf_status window_run(Engine* e, const WindowLaunch& w, float* compact_dst, cudaE
   } else {
     switch (e->draw_strategy) {
       case kDrawWarp:
-        if (single) launch_window_kernel<kDrawWarp, true>(e, w);
-        else launch_window_kernel<kDrawWarp, false>(e, w);
+        if (single) launch_window_kernel<kDrawWarp, true>(e, w, form);
+        else launch_window_kernel<kDrawWarp, false>(e, w, form);
         break;
       case kDrawGrouped:
-        if (single) launch_window_kernel<kDrawGrouped, true>(e, w);
-        else launch_window_kernel<kDrawGrouped, false>(e, w);
+        if (single) launch_window_kernel<kDrawGrouped, true>(e, w, form);
+        else launch_window_kernel<kDrawGrouped, false>(e, w, form);
         break;
       case kDrawNormalAll:
-        if (single) launch_window_kernel<kDrawNormalAll, true>(e, w);
-        else launch_window_kernel<kDrawNormalAll, false>(e, w);
+        if (single) launch_window_kernel<kDrawNormalAll, true>(e, w, form);
+        else launch_window_kernel<kDrawNormalAll, false>(e, w, form);
         break;
       case kDrawPooledSearch:
-        if (single) launch_window_kernel<kDrawPooledSearch, true>(e, w);
-        else launch_window_kernel<kDrawPooledSearch, false>(e, w);
+        if (single) launch_window_kernel<kDrawPooledSearch, true>(e, w, form);
+        else launch_window_kernel<kDrawPooledSearch, false>(e, w, form);
         break;
       default:
-        if (single) launch_window_kernel<kDrawLanes, true>(e, w);
-        else launch_window_kernel<kDrawLanes, false>(e, w);
+        if (single) launch_window_kernel<kDrawLanes, true>(e, w, form);
+        else launch_window_kernel<kDrawLanes, false>(e, w, form);
         break;
     }
   }
