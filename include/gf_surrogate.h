@@ -64,7 +64,7 @@ gf_status gf_mlp_set_fused_inference(gf_mlp* mlp, int32_t enable);
 /* Spectra of model parameters, host to host: rows x 6 doubles in, scaled to the network's inputs
  * (2 (p - low) / (high - low) - 1; the second one through asinh(p / asinh_scale) between asinh_low and
  * asinh_high), and rows x 99 doubles out, exp(std * output + mean) divided by each row's sum.  Any number of
- * rows.  Synchronous. */
+ * rows.  Synchronous; a kernel fault (gf_mlp_check) is reported by the call itself and cleared. */
 typedef struct gf_mlp_scaling {
   double low[GF_MLP_INPUTS], high[GF_MLP_INPUTS];
   double asinh_scale, asinh_low, asinh_high;

@@ -1018,9 +1018,11 @@ __global__ void query_encode_kernel(const double* __restrict__ params, int rows,
 
 // Outputs [rows][99] -> normalised spectra in double, a warp a row: the copy to the host, 792 bytes a row, is what
 // a query waits for, and the exponentials (270 us on the host at 4,096 rows, 475 more for the sums and quotients)
-// are a microsecond here.
+// are a microsecond here.  The network's fault word goes to the host with them (host_fault, page-locked): outputs
+// of a pass that gave up are not spectra.
 __global__ void query_spectra_kernel(const float* __restrict__ y, int rows, const gf_mlp_scaling s,
-                                     double* __restrict__ out) {
+                                     double* __restrict__ out, const int* __restrict__ fault, int* host_fault) {
+  if (blockIdx.x == 0 && threadIdx.x == 0) *host_fault = *fault;
   const int row = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
   if (row >= rows) return;   // warp-uniform
   double e[4];
@@ -1638,7 +1640,7 @@ struct gf_mlp {
   int* fault = nullptr;
 
   // host queries (gf_mlp_predict): rows at a time; device parameters, outputs and
-  // spectra; the page-locked ring (and one chunk's parameters), an event a chunk of it
+  // spectra; the page-locked ring (one chunk's parameters and the fault word behind it), an event a chunk of it
   long long q_rows = 0;
   double *q_params = nullptr, *q_spec = nullptr;
   float* q_out = nullptr;
@@ -1768,7 +1770,7 @@ gf_status query_buffers(gf_mlp* m) {
     m->q_out = reinterpret_cast<float*>(m->q_spec + rows * GF_MLP_OUTPUTS);
   }
   if (!m->q_ring)
-    MLP_CUDA(m, cudaMallocHost(&m->q_ring, (kQueryRing * kQueryChunkDoubles + kQueryChunk * GF_MLP_INPUTS) * sizeof(double)));
+    MLP_CUDA(m, cudaMallocHost(&m->q_ring, (kQueryRing * kQueryChunkDoubles + kQueryChunk * GF_MLP_INPUTS + 1) * sizeof(double)));
   static_assert(kQueryRing == sizeof(m->q_done) / sizeof(m->q_done[0]), "an event a chunk of the ring");
   for (cudaEvent_t& ev : m->q_done)
     if (!ev) MLP_CUDA(m, cudaEventCreateWithFlags(&ev, cudaEventDisableTiming));
@@ -1803,6 +1805,7 @@ gf_status run_predict(gf_mlp* m, const double* params, long long rows, const gf_
   gf_status st = query_buffers(m);
   if (st != GF_OK) return st;
   double* const h_params = m->q_ring + kQueryRing * kQueryChunkDoubles;
+  int* const h_fault = reinterpret_cast<int*>(h_params + kQueryChunk * GF_MLP_INPUTS);
   for (long long r0 = 0; r0 < rows; r0 += m->q_rows) {
     const int n = static_cast<int>(std::min(m->q_rows, rows - r0)), batch = (n + BM - 1) / BM * BM;
     double* const to = spectra + r0 * GF_MLP_OUTPUTS;
@@ -1815,7 +1818,8 @@ gf_status run_predict(gf_mlp* m, const double* params, long long rows, const gf_
     query_encode_kernel<<<(batch + 127) / 128, 128, 0, m->stream>>>(direct ? h_params : m->q_params, n, batch, s, m->x0);
     MLP_CUDA(m, cudaGetLastError());
     if ((st = run_forward_encoded(m, batch, m->q_out)) != GF_OK) return st;
-    query_spectra_kernel<<<(n + 7) / 8, 256, 0, m->stream>>>(m->q_out, n, s, direct ? m->q_ring : m->q_spec);
+    query_spectra_kernel<<<(n + 7) / 8, 256, 0, m->stream>>>(m->q_out, n, s, direct ? m->q_ring : m->q_spec, m->fault,
+                                                             h_fault);
     MLP_CUDA(m, cudaGetLastError());
     const int chunks = (n + kQueryChunk - 1) / kQueryChunk;
     if (direct) MLP_CUDA(m, cudaEventRecord(m->q_done[0], m->stream));
@@ -1838,6 +1842,7 @@ gf_status run_predict(gf_mlp* m, const double* params, long long rows, const gf_
     for (int t = started; t < threads && err[0] == cudaSuccess; ++t) err[0] = take_chunks(m, n, t, threads, to);
     for (int t = 1; t < started; ++t) helper[t].join();
     for (const cudaError_t e : err) MLP_CUDA(m, e);
+    if (*h_fault) return gf_mlp_check(m);   // written by the kernel whose spectra have arrived
   }
   return GF_OK;
 }
