@@ -56,6 +56,24 @@ __device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity, long l
   return true;
 }
 
+// The same by a whole converged warp, with one verdict for all its lanes: code behind it elects lanes and meets at
+// warp barriers, which lanes that disagreed (one saw the phase complete, another the limit pass) would not reach
+// together.  Gives up as soon as any wait of the CTA has (`abort_flag`).  A lane that has seen the phase sees it again:
+// the barrier cannot go on before this warp does.
+__device__ __forceinline__ bool mbar_wait_warp(uint64_t* bar, uint32_t parity, long long limit,
+                                               volatile int* abort_flag) {
+  const uint32_t addr = smem_u32(bar);
+  if (__all_sync(0xFFFFFFFFu, mbar_try_wait(addr, parity))) return true;
+  const long long t0 = clock64();
+  while (!__all_sync(0xFFFFFFFFu, mbar_try_wait(addr, parity))) {
+    if (__any_sync(0xFFFFFFFFu, *abort_flag || clock64() - t0 > limit)) {
+      *abort_flag = 1;
+      return false;
+    }
+  }
+  return true;
+}
+
 // ---------------------------------------------------------------------------------------------
 // TMA: 2-D tiled load global -> this CTA's shared memory, completion counted on an mbarrier
 // ---------------------------------------------------------------------------------------------

@@ -218,19 +218,7 @@ umma_gemm_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constan
   // run out (`wait`); the epilogue warps wait on the barrier alone and then agree on the outcome, so
   // all of them leave the tile loop together.  An aborted CTA never touches unsynchronised data: it
   // drains what it issued and releases tensor memory.
-  auto wait = [&](uint64_t* bar, uint32_t parity) -> bool {
-    const uint32_t addr = smem_u32(bar);
-    if (mbar_try_wait(addr, parity)) return true;
-    const long long t0 = clock64();
-    while (!mbar_try_wait(addr, parity)) {
-      if (*abort_flag) return false;
-      if (clock64() - t0 > wait_limit) {
-        *abort_flag = 1;
-        return false;
-      }
-    }
-    return true;
-  };
+  auto wait = [&](uint64_t* bar, uint32_t parity) { return mbar_wait_warp(bar, parity, wait_limit, abort_flag); };
 
   if (threadIdx.x == 0) {
     tma_prefetch_desc(&tma_a);
@@ -621,19 +609,7 @@ fused_forward_kernel(const __grid_constant__ CUtensorMap tma_x, const __grid_con
   const uint32_t rank = cluster_rank();
   // a pair's tiles are neighbours; past the last one the odd CTA works on rows that nobody reads
   const int tiles_up = m_tiles + (m_tiles & 1);
-  auto wait = [&](uint64_t* bar, uint32_t parity) -> bool {
-    const uint32_t addr = smem_u32(bar);
-    if (mbar_try_wait(addr, parity)) return true;   // as a rule: the MMA thread has few issue slots to spare
-    const long long t0 = clock64();
-    while (!mbar_try_wait(addr, parity)) {
-      if (*abort_flag) return false;
-      if (clock64() - t0 > wait_limit) {
-        *abort_flag = 1;
-        return false;
-      }
-    }
-    return true;
-  };
+  auto wait = [&](uint64_t* bar, uint32_t parity) { return mbar_wait_warp(bar, parity, wait_limit, abort_flag); };
 
   if (threadIdx.x == 0) {
     tma_prefetch_desc(&tma_x);
@@ -949,11 +925,15 @@ fused_forward_kernel(const __grid_constant__ CUtensorMap tma_x, const __grid_con
             mbar_arrive_remote(hlo, 0);   // region A drained: the next tile's first MMAs may write it
             mbar_arrive(staged);
           }
-          if (threadIdx.x == kFfStoreThread && wait(staged, local & 1) && tile < m_tiles) {
-            // batch is a multiple of 128 (checked by the caller): the tile's rows are all in range
-            bulk_store_1d(out + static_cast<long long>(tile) * BM * GF_MLP_OUTPUTS, s_out,
-                          BM * GF_MLP_OUTPUTS * 4);
-            bulk_commit();
+          if (threadIdx.x == kFfStoreThread) {
+            if (!mbar_wait(staged, local & 1, wait_limit)) {
+              *abort_flag = 1;
+            } else if (tile < m_tiles) {
+              // batch is a multiple of 128 (checked by the caller): the tile's rows are all in range
+              bulk_store_1d(out + static_cast<long long>(tile) * BM * GF_MLP_OUTPUTS, s_out,
+                            BM * GF_MLP_OUTPUTS * 4);
+              bulk_commit();
+            }
           }
           __syncwarp();
         }
@@ -1185,19 +1165,7 @@ __global__ void __launch_bounds__(DW_THREADS, 1) weight_update_kernel(const __gr
   int* consumed_s = timed_out + 2;
   volatile int* abort_flag = timed_out;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  auto wait = [&](uint64_t* bar, uint32_t parity) -> bool {   // as in umma_gemm_kernel
-    const uint32_t addr = smem_u32(bar);
-    if (mbar_try_wait(addr, parity)) return true;
-    const long long t0 = clock64();
-    while (!mbar_try_wait(addr, parity)) {
-      if (*abort_flag) return false;
-      if (clock64() - t0 > A.wait_limit) {
-        *abort_flag = 1;
-        return false;
-      }
-    }
-    return true;
-  };
+  auto wait = [&](uint64_t* bar, uint32_t parity) { return mbar_wait_warp(bar, parity, A.wait_limit, abort_flag); };
   if (threadIdx.x == 0) {
     tma_prefetch_desc(&L.a);
     tma_prefetch_desc(&L.b);
