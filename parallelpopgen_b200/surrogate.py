@@ -72,6 +72,8 @@ class Mlp:
                  eps: float = 1e-8, weight_decay: float = 0.0, device: int = 0, stream=None):
         self.lib = _capi.load()
         self.capacity = capacity
+        self.device = int(device)
+        self.stream = getattr(stream, "value", stream) or 0   # the handle its work is queued on
         cfg = MlpConfig(int(capacity), float(lr), float(beta1), float(beta2), float(eps), float(weight_decay))
         h = ctypes.c_void_p()
         st = self.lib.gf_mlp_create(int(device), stream, ctypes.byref(cfg), ctypes.byref(h))
@@ -126,7 +128,9 @@ class Mlp:
         self._check(self.lib.gf_mlp_train_step(self.h, x.data_ptr(), t.data_ptr(), x.shape[0], d_loss))
 
     def train_step_rows(self, x, t, rows, d_loss: int | None = None):
-        """train_step on rows `rows` (a CUDA int64 tensor) of x and t."""
+        """train_step on rows `rows` (a contiguous CUDA int64 tensor) of x and t."""
+        if str(rows.dtype) != "torch.int64" or not rows.is_contiguous():
+            raise ValueError("row indices must be a contiguous int64 tensor")
         self._check(self.lib.gf_mlp_train_step_rows(self.h, x.data_ptr(), t.data_ptr(), rows.data_ptr(), rows.shape[0],
                                                     d_loss))
 
@@ -299,6 +303,21 @@ class TrainResult:
     losses: list
 
 
+def _reads_rows_in_place(mlp, x, t) -> bool:
+    """Whether a training step may read a minibatch from the tables by its row indices: contiguous fp32 tables of the
+    network's widths on its device, and a network whose work is queued on the stream that draws the indices --
+    on another stream it could read indices not drawn yet, or memory already drawn into again, and from them any
+    address.  Other networks (a class of the caller's own) and tables that need gradients take train_step."""
+    import torch
+    if type(mlp) is not Mlp or not x.is_cuda or x.device != t.device or x.device.index != mlp.device:
+        return False
+    if torch.is_grad_enabled() and (x.requires_grad or t.requires_grad):
+        return False
+    return (x.dtype == t.dtype == torch.float32 and x.is_contiguous() and t.is_contiguous() and x.dim() == t.dim() == 2
+            and x.shape[1] == len(SUPPORT) and t.shape[1] == OUTPUTS and x.shape[0] <= t.shape[0]
+            and mlp.stream == torch.cuda.current_stream(x.device).cuda_stream)
+
+
 def train(mlp: Mlp, x, t, steps: int, batch: int = 1024, lr: float = 1e-3, lr_min: float = 1e-5,
           seed: int = 0, log_every: int = 500) -> TrainResult:
     """Adam on minibatches drawn with replacement, cosine learning-rate decay; x, t are CUDA tensors."""
@@ -307,10 +326,7 @@ def train(mlp: Mlp, x, t, steps: int, batch: int = 1024, lr: float = 1e-3, lr_mi
     gen.manual_seed(seed)
     d_loss = torch.zeros(1, dtype=torch.float32, device=x.device)
     losses = []
-    # rows of contiguous fp32 tables of the network's widths are read in place; others are gathered first
-    in_place = (x.dtype == t.dtype == torch.float32 and x.is_contiguous() and t.is_contiguous() and x.dim() == t.dim() == 2
-                and x.shape[1] == len(SUPPORT) and t.shape[1] == OUTPUTS and x.shape[0] <= t.shape[0]
-                and x.device == t.device)
+    in_place = _reads_rows_in_place(mlp, x, t)   # else each minibatch is gathered first
     if not in_place:
         xb = torch.empty((batch, x.shape[1]), dtype=torch.float32, device=x.device)
         tb = torch.empty((batch, t.shape[1]), dtype=torch.float32, device=x.device)
