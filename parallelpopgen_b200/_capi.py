@@ -164,6 +164,11 @@ SIGNATURES = {
 _lib = None
 
 
+def available() -> bool:
+    """Whether load() has the library or finds it built."""
+    return _lib is not None or LIB_PATH.exists()
+
+
 def load(path: os.PathLike | str | None = None) -> ctypes.CDLL:
     """Load libgofish_b200.so and declare every entry point; raises if it is missing."""
     global _lib

@@ -167,7 +167,8 @@ def draw_parameters(count: int, seed: int) -> np.ndarray:
 
 
 def in_support(params: np.ndarray) -> np.ndarray:
-    if type(params) is np.ndarray and params.dtype == np.float64 and params.shape[1:] == (6,) and params.flags.c_contiguous:
+    if (type(params) is np.ndarray and params.dtype == np.float64 and params.shape[1:] == (6,)
+            and params.flags.c_contiguous and params.flags.aligned and _capi.available()):   # NumPy needs no library
         inside = np.empty(len(params), bool)
         lo, hi = (np.ascontiguousarray(v, np.float64) for v in (LOW, HIGH))
         if lo.shape == hi.shape == (6,) and _capi.load().gf_rows_inside(
