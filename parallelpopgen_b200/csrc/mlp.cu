@@ -23,10 +23,10 @@
 #include <cstdarg>
 #include <cstdio>
 #include <cstring>
+#include <exception>
 #include <mutex>
 #include <new>
 #include <string>
-#include <system_error>
 #include <thread>
 #include <utility>
 #include <vector>
@@ -1804,7 +1804,7 @@ gf_status run_predict(gf_mlp* m, const double* params, long long rows, const gf_
           err[started] = cudaSetDevice(m->device);
           if (err[started] == cudaSuccess) err[started] = take_chunks(m, n, started, threads, to);
         });
-    } catch (const std::system_error&) {   // this thread takes the shares of those that could not be started
+    } catch (const std::exception&) {   // no thread or no memory for it: this one takes the shares left over
     }
     err[0] = take_chunks(m, n, 0, threads, to);
     for (int t = started; t < threads && err[0] == cudaSuccess; ++t) err[0] = take_chunks(m, n, t, threads, to);
