@@ -594,7 +594,7 @@ static void release_sim(Engine* e) {
   e->flags = nullptr;
   e->tile_count = nullptr;
   e->tile_offset = nullptr;
-  e->pending.clear();
+  e->count.pending.clear();
   e->capacity = 0;
   e->active = false;
 }
@@ -701,17 +701,15 @@ static gf_status begin_common(Engine* e, const gf_sim_config* c, long long initi
   GF_CUDA(e, cudaMemsetAsync(e->d_count, 0, sizeof(int) * kCountWords, e->stream));
   GF_CUDA(e, cudaMemsetAsync(e->d_stats, 0, sizeof(unsigned long long) * 2, e->stream));
   e->compactions = 0;
-  e->M_upper = initial_mutations;
-  e->M_recent = initial_mutations;
-  e->M_exact = true;
+  e->count.known(initial_mutations);
   e->active = true;
   return GF_OK;
 }
 
 // Retire completed survivor-count read-backs, tightening the host's upper bound.
 static void poll_pending(Engine* e, bool wait_all) {
-  while (!e->pending.empty()) {
-    PendingCount& pc = e->pending.front();
+  while (!e->count.pending.empty()) {
+    const PendingCount& pc = e->count.pending.front();
     const volatile unsigned long long* mail = e->h_mail + pc.slot;
     unsigned long long v = *mail;
     if (static_cast<unsigned>(v >> 32) != pc.tag) {
@@ -720,23 +718,15 @@ static void poll_pending(Engine* e, bool wait_all) {
       v = *mail;
     }
     // after a failed stream the mail may not have come: the bound stays as it is
-    const long long count =
-        static_cast<unsigned>(v >> 32) == pc.tag ? static_cast<long long>(v & 0xFFFFFFFFu) : e->M_upper;
-    // a bound whatever came after (later compactions only lower the count), exact if nothing did
-    const long long bound = count + pc.added;
-    e->M_recent = count;
-    if (bound <= e->M_upper) {
-      e->M_upper = bound;
-      if (e->pending.size() == 1) e->M_exact = true;
-    }
-    e->pending.pop_front();
+    e->count.survivors(static_cast<unsigned>(v >> 32) == pc.tag ? static_cast<long long>(v & 0xFFFFFFFFu)
+                                                                : e->count.upper);
   }
 }
 
 // A slot for the survivor count of the compaction that the caller is about to launch.
 static PendingCount new_mail(Engine* e) {
   poll_pending(e, false);
-  if (static_cast<int>(e->pending.size()) >= e->pinned_slots - 1) poll_pending(e, true);
+  if (static_cast<int>(e->count.pending.size()) >= e->pinned_slots - 1) poll_pending(e, true);
   PendingCount pc;
   pc.slot = e->next_slot;
   e->next_slot = (e->next_slot + 1) % e->pinned_slots;
@@ -911,8 +901,7 @@ static gf_status launch_compaction(Engine* e, int tiles_bound, int slot_out, boo
     e->prof_compact.emplace_back(ev0, ev1);
   }
   e->id_cur ^= 1;
-  e->pending.push_back(pc);
-  e->M_exact = false;
+  e->count.compaction(pc);
   return GF_OK;
 }
 
@@ -920,23 +909,23 @@ static gf_status launch_compaction(Engine* e, int tiles_bound, int slot_out, boo
 static gf_status launch_generation(Engine* e, GenArgs& h, GenArgs* d_table, int index, const GenHost& gh) {
   const int P = e->P;
   const long long new_total = h.new_total;
-  if (!e->pending.empty()) poll_pending(e, false);
+  if (!e->count.pending.empty()) poll_pending(e, false);
   // the preserved check is decided when the generation launches (earlier compactions may set it)
   if (h.flag && e->any_preserved && !h.check_preserved) {
     h.check_preserved = 1;
     GF_CUDA(e, cudaMemcpyAsync(&d_table[index].check_preserved, &h.check_preserved, sizeof(int),
                                cudaMemcpyHostToDevice, e->stream));
   }
-  long long need = e->M_upper + new_total;
+  long long need = e->count.upper + new_total;
   if (need > e->capacity) {
     poll_pending(e, true);
-    need = e->M_upper + new_total;
+    need = e->count.upper + new_total;
     if (need > e->capacity) {
       // exact count, then grow
       int M = 0;
       GF_CUDA(e, cudaMemcpyAsync(&M, e->d_count + e->count_slot, sizeof(int), cudaMemcpyDeviceToHost, e->stream));
       GF_CUDA(e, cudaStreamSynchronize(e->stream));
-      e->M_upper = M;
+      e->count.known(M);
       need = M + new_total;
       if (need > e->capacity) {
         gf_status st = set_capacity(e, std::max<long long>(need + need / 2, e->capacity * 3 / 2), M);
@@ -961,8 +950,7 @@ static gf_status launch_generation(Engine* e, GenArgs& h, GenArgs* d_table, int 
     GF_CUDA(e, cudaEventRecord(ev1, e->stream));
     e->prof_drift.emplace_back(ev0, ev1);
   }
-  e->M_upper = need;
-  for (auto& pc : e->pending) pc.added += new_total;
+  e->count.births(new_total);
 
   if (h.flag) {
     gf_status cst = launch_compaction(e, tiles_bound, slot_out, gh.preserve);
@@ -978,15 +966,15 @@ static gf_status launch_generation(Engine* e, GenArgs& h, GenArgs* d_table, int 
 // Make room for `need` slots: tighten the host bound from finished read-backs, then from an exact
 // (synchronizing) read of the count, and grow the arrays if still short.
 static gf_status ensure_capacity(Engine* e, long long new_slots, long long* need_out) {
-  long long need = e->M_upper + new_slots;
+  long long need = e->count.upper + new_slots;
   if (need > e->capacity) {
     poll_pending(e, true);
-    need = e->M_upper + new_slots;
+    need = e->count.upper + new_slots;
     if (need > e->capacity) {
       int M = 0;
       GF_CUDA(e, cudaMemcpyAsync(&M, e->d_count + e->count_slot, sizeof(int), cudaMemcpyDeviceToHost, e->stream));
       GF_CUDA(e, cudaStreamSynchronize(e->stream));
-      e->M_upper = M;
+      e->count.known(M);
       need = M + new_slots;
       if (need > e->capacity) {
         gf_status st = set_capacity(e, std::max<long long>(need + need / 2, e->capacity * 3 / 2), M);
@@ -1057,7 +1045,7 @@ static gf_status launch_window(Engine* e, int b, int first, int count, const Gen
   w.recs = e->d_wgen[b];
   w.total_tiles = R.ntiles;
   w.longest = count;
-  w.expected_slots = std::min(need, e->M_recent + news);
+  w.expected_slots = std::min(need, e->count.recent + news);
   w.any_compact = R.compact != 0;
   w.stats = e->d_stats;
   w.fault = e->d_count + 2;
@@ -1089,16 +1077,14 @@ static gf_status launch_window(Engine* e, int b, int first, int count, const Gen
       e->prof_pool.push_back(ev1);
     }
   }
-  e->M_upper = need;
-  for (auto& earlier : e->pending) earlier.added += news;
+  e->count.births(news);
   e->count_slot ^= 1;
   e->step_index += count;
   if (R.compact) {
     if (R.preserve) e->any_preserved = true;
     e->id_cur ^= 1;
     e->compactions += 1;
-    e->pending.push_back(pc);
-    e->M_exact = false;
+    e->count.compaction(pc);
   } else {
     e->cur ^= 1;
   }
@@ -1152,7 +1138,7 @@ static gf_status launch_window_mp(Engine* e, int b, int first, int count, const 
   w.seed2 = e->seed2;
   w.stats = e->d_stats;
   w.tiles_bound = tiles_bound;
-  w.small = std::min(need, e->M_recent + news) <= kSmallMpSlots;
+  w.small = std::min(need, e->count.recent + news) <= kSmallMpSlots;
   cudaEvent_t ev0 = nullptr, ev1 = nullptr;
   if (e->profiling) {
     ev0 = prof_event(e);
@@ -1166,8 +1152,7 @@ static gf_status launch_window_mp(Engine* e, int b, int first, int count, const 
     e->prof_drift.emplace_back(ev0, ev1);
   }
   e->live_rows |= drifted;
-  e->M_upper = need;
-  for (auto& pc : e->pending) pc.added += news;
+  e->count.births(news);
   e->step_index += count;
   if (compact) {
     e->count_slot ^= 1;
@@ -1188,8 +1173,7 @@ static gf_status launch_window_mp(Engine* e, int b, int first, int count, const 
     e->any_preserved = e->any_preserved || preserve;
     e->compactions += 1;
     e->id_cur ^= 1;
-    e->pending.push_back(pc);
-    e->M_exact = false;
+    e->count.compaction(pc);
     return GF_OK;
   }
   e->cur ^= 1;
@@ -1288,9 +1272,7 @@ static gf_status current_count(Engine* e, int* M) {
   gf_status st = check_device_fault(e);
   if (st != GF_OK) return st;
   poll_pending(e, true);
-  e->M_upper = *M;
-  e->M_recent = *M;
-  e->M_exact = true;
+  e->count.known(*M);
   return GF_OK;
 }
 
@@ -1704,7 +1686,7 @@ gf_status gf_sim_sample_begin(gf_engine* g, float* freq_out, int32_t* ids_out, i
     if (e->sample_in_flight) return fail(e, GF_ERR_STATE, "a time sample is already in flight");
     GF_CUDA(e, cudaSetDevice(e->device));
     poll_pending(e, false);
-    long long bound = e->M_upper;
+    long long bound = e->count.upper;
     if (bound > max_mutations) {   // the bound is loose: read the count itself
       int M = 0;
       gf_status st = current_count(e, &M);

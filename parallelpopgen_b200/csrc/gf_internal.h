@@ -265,14 +265,6 @@ struct Batch {
   long long steps_enqueued = 0, slabs_enqueued = 0;
 };
 
-// A compaction's survivor count on its way to the host: the compaction stores it into h_mail[slot] with the tag
-// above it.
-struct PendingCount {
-  int slot = 0;
-  long long added = 0;   // new mutations appended after this compaction
-  unsigned tag = 0;
-};
-
 struct Engine {
   int device = 0;
   int num_sms = 148;
@@ -317,10 +309,7 @@ struct Engine {
   int next_slot = 0;
 
   // host tracking of the mutation count
-  long long M_upper = 0;   // upper bound on the current count (exact when nothing is pending)
-  long long M_recent = 0;  // the last count read back: what a window's size is expected from (the bound
-                           // grows by the births of every window enqueued ahead of the read-backs)
-  bool M_exact = true;
+  SlotCount count;
   // an asynchronous time sample (gf_sim_sample_begin / _wait): the state packed into device scratch on
   // the engine's stream, copied to the caller's arrays on a second stream
   cudaStream_t copy_stream = nullptr;
@@ -336,7 +325,6 @@ struct Engine {
   bool sample_to_stage = false;       // the wait copies into the engine's staging
   float* h_sample_stage = nullptr;    // page-locked staging of a sample's rows
   size_t sample_stage_cap = 0;        // in floats
-  std::deque<PendingCount> pending;
 
   // per-generation parameter tables (double-buffered: the host fills one while the GPU reads the other)
   GenArgs* d_table[2] = {nullptr, nullptr};

@@ -6,6 +6,7 @@
 
 #include <algorithm>
 #include <cstdint>
+#include <deque>
 #include <vector>
 
 #include "../../include/gofish_b200.h"
@@ -118,6 +119,38 @@ inline bool mp_window_generation_ok(const gf_generation& g, int P, int live_rows
   }
   return true;
 }
+
+// A compaction's survivor count on its way to the host: the compaction stores it into h_mail[slot] with the tag
+// above it.
+struct PendingCount {
+  int slot = 0;
+  long long added = 0;   // new mutations appended after this compaction
+  unsigned tag = 0;
+};
+
+// What the host knows of the mutation count while launches are queued ahead of the read-backs.
+struct SlotCount {
+  long long upper = 0;    // upper bound on the count after everything enqueued
+  long long recent = 0;   // the last count read back: what a window's size is expected from (the bound
+                          // grows by the births of every window enqueued ahead of the read-backs)
+  std::deque<PendingCount> pending;   // compactions whose survivor counts are not here yet, oldest first
+
+  // The count itself, everything enqueued having run.
+  void known(long long M) { upper = recent = M; }
+  // `n` births enqueued.  They are added to whatever the bound is by then: a count may have arrived since the
+  // launch was sized.
+  void births(long long n) {
+    upper += n;
+    for (PendingCount& pc : pending) pc.added += n;
+  }
+  void compaction(const PendingCount& pc) { pending.push_back(pc); }
+  // The oldest compaction's count is here: a bound whatever came after (later compactions only lower the count).
+  void survivors(long long M) {
+    recent = M;
+    upper = std::min(upper, M + pending.front().added);
+    pending.pop_front();
+  }
+};
 
 // Generations whose records a block of the single- or multi-population window kernels stages in shared memory.
 // The plain engine ends its windows there; a batched replicate's window is its compaction cadence, of any length.
