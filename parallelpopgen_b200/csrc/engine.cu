@@ -1045,7 +1045,7 @@ static gf_status launch_window(Engine* e, int b, int first, int count, const Gen
   w.recs = e->d_wgen[b];
   w.total_tiles = R.ntiles;
   w.longest = count;
-  w.expected_slots = std::min(need, e->count.recent + news);
+  w.expected_slots = e->count.expected(news);
   w.any_compact = R.compact != 0;
   w.stats = e->d_stats;
   w.fault = e->d_count + 2;
@@ -1138,7 +1138,7 @@ static gf_status launch_window_mp(Engine* e, int b, int first, int count, const 
   w.seed2 = e->seed2;
   w.stats = e->d_stats;
   w.tiles_bound = tiles_bound;
-  w.small = std::min(need, e->count.recent + news) <= kSmallMpSlots;
+  w.small = e->count.expected(news) <= kSmallMpSlots;
   cudaEvent_t ev0 = nullptr, ev1 = nullptr;
   if (e->profiling) {
     ev0 = prof_event(e);

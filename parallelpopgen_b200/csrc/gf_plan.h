@@ -131,19 +131,29 @@ struct PendingCount {
 // What the host knows of the mutation count while launches are queued ahead of the read-backs.
 struct SlotCount {
   long long upper = 0;    // upper bound on the count after everything enqueued
-  long long recent = 0;   // the last count read back: what a window's size is expected from (the bound
-                          // grows by the births of every window enqueued ahead of the read-backs)
+  long long recent = 0;   // the last count read back
+  long long open = 0;     // births since the compaction enqueued last: no compaction has thinned them
   std::deque<PendingCount> pending;   // compactions whose survivor counts are not here yet, oldest first
 
   // The count itself, everything enqueued having run.
-  void known(long long M) { upper = recent = M; }
+  void known(long long M) {
+    upper = recent = M;
+    open = 0;
+  }
+  // About how many slots a window with `n` births ends with: the survivors of a compaction differ little from one
+  // to the next, while the bound grows by the births of every window enqueued ahead of the read-backs.
+  long long expected(long long n) const { return std::min(upper, recent + open) + n; }
   // `n` births enqueued.  They are added to whatever the bound is by then: a count may have arrived since the
   // launch was sized.
   void births(long long n) {
     upper += n;
+    open += n;
     for (PendingCount& pc : pending) pc.added += n;
   }
-  void compaction(const PendingCount& pc) { pending.push_back(pc); }
+  void compaction(const PendingCount& pc) {
+    pending.push_back(pc);
+    open = 0;
+  }
   // The oldest compaction's count is here: a bound whatever came after (later compactions only lower the count).
   void survivors(long long M) {
     recent = M;

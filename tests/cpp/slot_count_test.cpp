@@ -1,5 +1,5 @@
 // Host-only checks of what the engine knows of its mutation count while launches run ahead of the read-backs
-// (SlotCount, gf_plan.h): always a bound, and one that follows the counts as they arrive.
+// (SlotCount, gf_plan.h): always a bound, one that follows the counts as they arrive, and the size a window is expected to end with.
 #include <cstdio>
 #include <deque>
 
@@ -34,11 +34,43 @@ static void check_bound(long long living, long long births, int lag) {
   CHECK(c.upper == living, "bound %lld of %lld at the end", c.upper, living);
 }
 
+// What a window is expected to end with: the births of windows that end without a compaction (long cadences are
+// cut at 128 generations) are still there, those of windows that compact are not.
+static void check_expected() {
+  gf::SlotCount c;
+  c.known(1000);
+  CHECK(c.expected(100) == 1100, "%lld", c.expected(100));
+  for (int w = 0; w < 50; ++w) {
+    CHECK(c.expected(100) == 1000 + 100 * (w + 1), "window %d without a compaction: %lld", w, c.expected(100));
+    c.births(100);
+  }
+  c.compaction(gf::PendingCount{});
+  CHECK(c.expected(100) == 1100, "after the compaction, its count not here: %lld", c.expected(100));
+  for (int w = 0; w < 50; ++w) {   // compacting windows ahead of the read-backs
+    c.births(100);
+    c.compaction(gf::PendingCount{});
+  }
+  CHECK(c.expected(100) == 1100 && c.upper == 11000, "%lld of %lld", c.expected(100), c.upper);
+  c.survivors(1500);
+  CHECK(c.expected(100) == 1600, "%lld", c.expected(100));
+  c.births(100);
+  CHECK(c.expected(100) == 1700, "%lld", c.expected(100));
+  c.known(30);
+  CHECK(c.expected(5) == 35, "%lld", c.expected(5));
+  gf::SlotCount d;
+  d.known(10);
+  d.births(5);
+  d.compaction(gf::PendingCount{});
+  d.survivors(3);
+  CHECK(d.expected(0) == 3 && d.upper == 3, "%lld of %lld", d.expected(0), d.upper);
+}
+
 int main() {
   for (int lag : {1, 2, 7, 62}) {
     check_bound(1000, 300, lag);
     check_bound(0, 5, lag);
   }
+  check_expected();
   std::printf(failures ? "FAILED %d\n" : "OK\n", failures);
   return failures ? 1 : 0;
 }
