@@ -587,6 +587,7 @@ static gf_status batch_begin(Engine* e, const gf_replicate* in, int R) {
     arena += br.capacity;
   }
   b->arena = arena;
+  b->pack = batch_packs(in, R, arena / kBatchTile);
   {
     // slices of one engine-owned allocation, 256-byte aligned, laid out in a fixed order
     size_t need = 0;
@@ -750,13 +751,6 @@ static void refresh_active(Batch* b) {
     b->active.push_back(r);
     b->active_cadence_sum += br.p.compact_interval;
   }
-  // Short windows of small replicates, whose tiles are mostly last ones and share no records, do not repay the
-  // packing kernel's start.  1,024 replicates, a quad per thread against packing: N0 up to 1e4 (some 60 tiles of
-  // capacity each) 442 / 508 ms at a cadence of 10, 439 / 456 at 25, 470 / 447 at 35; up to 3e4 (some 140) 1.24 / 1.29 s at 20,
-  // 1.31 / 1.26 at 30; 128 up to 1e5 (some 350) 2.36 / 1.99 s at 10; spectra of 256 (some 800) 305 / 307 ms at 10, 377 / 315 at 25.
-  constexpr long long kLargeTiles = 240, kPackCadence = 26;
-  b->pack = b->all_tiles >= kLargeTiles * b->R ||
-            b->active_cadence_sum >= kPackCadence * static_cast<long long>(b->active.size());
   b->active_dirty = false;
 }
 

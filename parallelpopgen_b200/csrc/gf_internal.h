@@ -238,7 +238,7 @@ struct Batch {
   std::vector<int> active;                    // unfinished replicates, in index order
   bool active_dirty = true;
   long long active_cadence_sum = 0;           // sum of their cadences (generations per super-step)
-  bool pack = true;                           // windows pack living slots (refresh_active)
+  bool pack = true;                           // windows pack living slots (batch_packs)
   int longest = 0;                            // generations of the longest window
   std::vector<std::vector<int>> finish_at;    // [k]: replicates whose last window is super-step k
   // precomputed records: a replicate table of all R replicates in index order, whose per-window fields

@@ -173,6 +173,23 @@ inline int longest_window(const gf_replicate* reps, int R) {
   return n;
 }
 
+// Whether a batch's windows pack their living slots, decided once: its launches are also captured in graphs.  `tiles`:
+// of 1,024 slots, over all segments.  Short windows of small replicates, whose tiles are mostly last ones and share no
+// records, do not repay the packing kernel's start.  1,024 replicates, a quad per thread against packing: N0 up to
+// 1e4 (some 60 tiles of capacity each) 442 / 508 ms at a cadence of 10, 439 / 456 at 25, 470 / 447 at 35; up to 3e4 (some 140)
+// 1.24 / 1.29 s at 20, 1.31 / 1.26 at 30; 128 up to 1e5 (some 350) 2.36 / 1.99 s at 10; spectra of 256 (some 800) 305 / 307 ms at
+// 10, 377 / 315 at 25.
+inline bool batch_packs(const gf_replicate* reps, int R, long long tiles) {
+  constexpr long long kLargeTiles = 240, kPackCadence = 26;
+  long long cadences = 0, run = 0;   // of the replicates that run at all
+  for (int r = 0; r < R; ++r)
+    if (reps[r].num_generations > 0) {
+      cadences += reps[r].compact_interval;
+      ++run;
+    }
+  return tiles >= kLargeTiles * R || cadences >= kPackCadence * run;
+}
+
 // Expected slots (at the window's end) up to which one replicate's window runs a slot per thread.  Window
 // kernels of 25 generations on a B200, a slot per thread against the packing kernel: 23 / 53 us at 12,000
 // slots, 27 / 55 at 92,000, 50 / 70 at 368,000, 74 / 80 at 552,000 (N = 1e4, neutral), 92 / 104 at 648,000 (gamma = -10),

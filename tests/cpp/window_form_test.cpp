@@ -37,6 +37,19 @@ static void check_batches() {
   CHECK(form({rep(25, 1000)}, false) == WindowForm::quads);
 }
 
+// The packing rule is the batch's own: it does not move as replicates finish, and needs no resident records.
+static void check_packing() {
+  auto packs = [](const std::vector<gf_replicate>& reps, long long tiles) {
+    return gf::batch_packs(reps.data(), static_cast<int>(reps.size()), tiles);
+  };
+  CHECK(!packs({rep(25, 100), rep(25, 100)}, 100));
+  CHECK(packs({rep(26, 100), rep(26, 100)}, 100));
+  CHECK(!packs({rep(10, 100), rep(41, 100)}, 100) && packs({rep(10, 100), rep(42, 100)}, 100));
+  CHECK(!packs({rep(10, 100), rep(10, 100)}, 479) && packs({rep(10, 100), rep(10, 100)}, 480));
+  CHECK(!packs({rep(10, 100), rep(1000, 0)}, 2));   // a replicate that never runs
+  CHECK(packs({rep(30, 100), rep(1, 0)}, 2));
+}
+
 static void check_single() {
   using gf::WindowForm;
   const long long line = gf::kSlotWindowSlots;
@@ -49,6 +62,7 @@ static void check_single() {
 
 int main() {
   check_batches();
+  check_packing();
   check_single();
   std::printf(failures ? "FAILED %d\n" : "OK\n", failures);
   return failures ? 1 : 0;
