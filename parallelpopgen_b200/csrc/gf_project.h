@@ -34,7 +34,8 @@ inline size_t project_scratch(int n, int parts, int rows) {
 cudaError_t project_rows(const ProjSource& src, int n, int rows, int parts, double extra0, const float* rep_L,
                          double* scratch, float* out, cudaStream_t stream);
 
-// Loads the projection's kernels and sets their shared-memory limits on the current device (idempotent).
+// Loads the kernels of every sample size and sets their shared-memory limits on the current device (idempotent); without
+// it a size is set up by its first projection.
 cudaError_t project_ready();
 
 }  // namespace gf
