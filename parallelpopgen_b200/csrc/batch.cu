@@ -1190,12 +1190,16 @@ gf_status gf_batch_sfs(gf_engine* g, int32_t n, float* out) {
       rows.L[r] = b->reps[r].p.num_sites;
       most = std::max<long long>(most, rows.M[r]);
     }
+    // rows of one launch: gridDim.y is limited to 65,535, and the sums in double (twice the output) of many replicates
+    // to 64 MB, which the next launch takes over
     const int parts = project_parts(n, most, R, e->num_sms);
+    const int per_launch = static_cast<int>(
+        std::min<size_t>({static_cast<size_t>(R), 65535, (size_t{64} << 20) / (sizeof(double) * project_scratch(n, parts, 1))}));
     char* d_rows = nullptr;
     double* d_scratch = nullptr;
     float* d_out = nullptr;
     gf_status ast = pool_alloc(e, reinterpret_cast<void**>(&d_rows), 16 * static_cast<size_t>(R));
-    if (ast == GF_OK) ast = pool_alloc(e, reinterpret_cast<void**>(&d_scratch), sizeof(double) * project_scratch(n, parts, R));
+    if (ast == GF_OK) ast = pool_alloc(e, reinterpret_cast<void**>(&d_scratch), sizeof(double) * project_scratch(n, parts, per_launch));
     if (ast == GF_OK) ast = pool_alloc(e, reinterpret_cast<void**>(&d_out), sizeof(float) * static_cast<size_t>(R) * n);
     cudaError_t err = cudaSuccess;
     if (ast == GF_OK) {
@@ -1209,11 +1213,9 @@ gf_status gf_batch_sfs(gf_engine* g, int32_t n, float* out) {
       src.freq = b->freq[0];
       src.rep_base = d_base;
       src.rep_M = d_M;
-      // gridDim.y is limited to 65,535: more replicates in several launches
-      for (int r0 = 0; r0 < R && err == cudaSuccess; r0 += 65535) {
-        const int rn = std::min(R - r0, 65535);
-        err = project_rows(src, n, rn, parts, 0.0, d_L + r0, d_scratch + project_scratch(n, parts, r0),
-                           d_out + static_cast<size_t>(r0) * n, e->stream);
+      for (int r0 = 0; r0 < R && err == cudaSuccess; r0 += per_launch) {
+        const int rn = std::min(R - r0, per_launch);
+        err = project_rows(src, n, rn, parts, 0.0, d_L + r0, d_scratch, d_out + static_cast<size_t>(r0) * n, e->stream);
         src.rep_base += rn;
         src.rep_M += rn;
         e->kernel_launches += 2;
