@@ -1614,6 +1614,8 @@ struct gf_mlp {
   float* q_out = nullptr;
   double* q_ring = nullptr;
   cudaEvent_t q_done[4] = {};
+  std::mutex querying;    // one host query at a time: held from its parameters to its spectra
+  std::mutex enqueueing;  // a pass reads the inputs that were encoded just before it
 
   // tensor maps
   CUtensorMap fwd_a[GF_MLP_LAYERS], fwd_b[GF_MLP_LAYERS];     // A = input activations, B = W
@@ -1713,6 +1715,7 @@ gf_status run_forward_encoded(gf_mlp* m, int batch, float* d_out) {
 }
 
 gf_status run_forward(gf_mlp* m, const float* d_inputs, int batch, float* d_out) {
+  std::lock_guard<std::mutex> lock(m->enqueueing);
   encode_inputs_kernel<<<(batch + 255) / 256, 256, 0, m->stream>>>(d_inputs, nullptr, batch, m->x0, m->x0t, m->cap, 0);
   MLP_CUDA(m, cudaGetLastError());
   return run_forward_encoded(m, batch, d_out);
@@ -1783,9 +1786,12 @@ gf_status run_predict(gf_mlp* m, const double* params, long long rows, const gf_
     if (direct) std::memcpy(h_params, params + r0 * GF_MLP_INPUTS, bytes);
     else
       MLP_CUDA(m, cudaMemcpyAsync(m->q_params, params + r0 * GF_MLP_INPUTS, bytes, cudaMemcpyHostToDevice, m->stream));
-    query_encode_kernel<<<(batch + 127) / 128, 128, 0, m->stream>>>(direct ? h_params : m->q_params, n, batch, s, m->x0);
-    MLP_CUDA(m, cudaGetLastError());
-    if ((st = run_forward_encoded(m, batch, m->q_out)) != GF_OK) return st;
+    {
+      std::lock_guard<std::mutex> lock(m->enqueueing);
+      query_encode_kernel<<<(batch + 127) / 128, 128, 0, m->stream>>>(direct ? h_params : m->q_params, n, batch, s, m->x0);
+      MLP_CUDA(m, cudaGetLastError());
+      if ((st = run_forward_encoded(m, batch, m->q_out)) != GF_OK) return st;
+    }
     query_spectra_kernel<<<(n + 7) / 8, 256, 0, m->stream>>>(m->q_out, n, s, direct ? m->q_ring : m->q_spec, m->fault,
                                                              h_fault);
     MLP_CUDA(m, cudaGetLastError());
@@ -2139,6 +2145,7 @@ gf_status gf_mlp_forward(gf_mlp* m, const float* d_inputs, int32_t batch, float*
 gf_status gf_mlp_predict(gf_mlp* m, const double* params, int64_t rows, const gf_mlp_scaling* scaling,
                          double* spectra) {
   if (!m || rows < 0 || !scaling || (rows > 0 && (!params || !spectra))) return GF_ERR_INVALID_ARGUMENT;
+  std::lock_guard<std::mutex> lock(m->querying);
   MLP_CUDA(m, cudaSetDevice(m->device));
   return run_predict(m, params, rows, *scaling, spectra);
 }
