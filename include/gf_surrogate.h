@@ -89,7 +89,8 @@ gf_status gf_mlp_train_step(gf_mlp* mlp, const float* d_inputs, const float* d_t
                             float* d_loss);
 
 /* The same on rows d_rows[0 .. batch) (device, int64) of d_inputs and d_targets: a minibatch without a copy
- * of it. */
+ * of it.  The rows are not checked: each must lie within both arrays, and be there in the order of the network's
+ * stream. */
 gf_status gf_mlp_train_step_rows(gf_mlp* mlp, const float* d_inputs, const float* d_targets, const int64_t* d_rows,
                                  int32_t batch, float* d_loss);
 

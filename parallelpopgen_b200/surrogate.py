@@ -135,7 +135,10 @@ class Mlp:
                                                     d_loss))
 
     def predict(self, params: np.ndarray, scaling: MlpScaling) -> np.ndarray:
-        """Normalised spectra [rows][99] (float64) of parameters [rows][6] (C-contiguous float64), scaled by `scaling`."""
+        """Normalised spectra [rows][99] (float64) of parameters [rows][6], scaled by `scaling`."""
+        params = np.ascontiguousarray(params, np.float64)
+        if params.ndim != 2 or params.shape[1] != len(SUPPORT):
+            raise ValueError(f"parameters of shape {params.shape}, not [rows][{len(SUPPORT)}]")
         out = np.empty((len(params), OUTPUTS))
         self._check(self.lib.gf_mlp_predict(self.h, params.ctypes.data, len(params), ctypes.byref(scaling), out.ctypes.data))
         return out
@@ -365,7 +368,7 @@ class Surrogate:
         params = np.asarray(params, dtype=np.float64)
         scaling = self._scaling() if params.ndim == 2 and params.shape[1] == len(SUPPORT) else None
         if scaling is not None:   # on the device from the parameters to the spectra
-            return self.mlp.predict(np.ascontiguousarray(params), scaling)
+            return self.mlp.predict(params, scaling)
         return self._predict_arrays(params)
 
     def _scaling(self) -> MlpScaling | None:
