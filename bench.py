@@ -312,7 +312,7 @@ def run_b200(args, rank, local_rank, world):
         "gpu_launches": int(launches),
         "roofline": {
             "bound": "hbm",
-            "kernel": "window_kernel (every generation of a compaction window per launch: selection, drift, "
+            "kernel": "window_pack_kernel (every generation of a compaction window per launch: selection, drift, "
                       "births, compaction flags); its segmented scan and scatter are compact_ms_per_step",
             "achieved": achieved,
             "peak": peak,

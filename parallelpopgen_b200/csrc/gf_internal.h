@@ -406,7 +406,7 @@ void batch_step_tiles(Engine* e, WinRep* d_table, int R, const int* M_in, const 
 // kernel and its compaction (two events, so that each timing pair owns its own)
 gf_status window_run(Engine* e, const WindowLaunch& w, float* compact_dst, cudaEvent_t after_window = nullptr,
                      cudaEvent_t before_compaction = nullptr);
-// Multi-population window launch (window_mp.cu); P in [2, 4].
+// Multi-population window launch (window_mp.cu); P in [2, 8].
 gf_status window_mp_run(Engine* e, const WindowMpLaunch& w);
 // The compaction of a `small` one into dst, posting the survivor count to mail.
 gf_status compact_mp_run(Engine* e, const WindowMpLaunch& w, float* dst, int* gp_dst, int* tid_dst, bool preserve,

@@ -181,10 +181,10 @@ __device__ __forceinline__ void stage_bf16_col(uint8_t* buf, int r, const float*
   for (int j = 0; j < 32; ++j) *reinterpret_cast<__nv_bfloat16*>(buf + j * 64 + 2 * r) = __float2bfloat16_rn(v[j]);
 }
 
-// Persistent tensor-core GEMM: CTAs stride over 128 x BN output tiles (N fastest, then M).  Warp 0 streams A/B K-blocks with TMA into a 4-stage ring, warp 1 issues tcgen05 MMAs
-// into one of two tensor-memory accumulators, warps 2-5 drain the other accumulator through the
-// epilogue (tcgen05.ld -> registers -> swizzled shared staging -> TMA store), so a tile's epilogue
-// overlaps the next tile's MMAs.
+// Persistent tensor-core GEMM: CTAs stride over 128 x BN output tiles (N fastest, then M).  Warp 0 streams A/B
+// K-blocks with TMA into a ring of two to four stages, warp 1 issues tcgen05 MMAs into one of two tensor-memory
+// accumulators, four (32-wide tiles) or eight epilogue warps drain the other one (tcgen05.ld -> registers ->
+// swizzled shared staging -> TMA store), so a tile's epilogue overlaps the next tile's MMAs.
 template <int BN, int EPI>
 __global__ void __launch_bounds__(gemm_threads(BN), BN == 32 ? 2 : 1)   // 2: the next kernel's CTA beside it
 umma_gemm_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constant__ CUtensorMap tma_b,
@@ -1056,7 +1056,7 @@ __global__ void encode_inputs_kernel(const float* __restrict__ x, const long lon
 // ---------------------------------------------------------------------------------------------
 // The end of a training step: the weight gradients of all layers, then Adam, in one launch
 // ---------------------------------------------------------------------------------------------
-// dW_l = dZ_l^T Y_{l-1} has few output tiles (104 of 128 x 64 over the five layers) and the batch as its
+// dW_l = dZ_l^T Y_{l-1} has few output tiles (108 of 128 x 64 over the five layers) and the batch as its
 // reduction dimension.  A CTA owns one tile of one layer: the batch is cut into `splits` parts, each
 // accumulated on its own in one of two tensor-memory accumulators and added up in registers in order (the
 // sum, rounding included, of gradient slices reduced in a fixed order), and the tile's master weights,
