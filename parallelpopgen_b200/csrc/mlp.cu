@@ -1830,6 +1830,7 @@ gf_status run_predict(gf_mlp* m, const double* params, long long rows, const gf_
 // overlapped launches 107; in 23 separate launches it was 230 us of kernels.  At 128: 68 us, at 4,096: 120.
 gf_status run_step(gf_mlp* m, const float* d_inputs, const float* d_targets, const long long* idx, int batch,
                    const AdamArgs* adam, float* d_loss) {
+  std::lock_guard<std::mutex> lock(m->enqueueing);
   cudaError_t err = launch_dependent(encode_inputs_kernel, (batch + 255) / 256, 256, 0, m->stream, d_inputs, idx, batch,
                                      m->x0, m->x0t, m->cap, 1);
   if (err != cudaSuccess) return mlp_fail(m, GF_ERR_CUDA, "encoding the inputs: %s", cudaGetErrorString(err));

@@ -47,3 +47,35 @@ def test_threads_get_their_own_spectra():
         t.join()
     assert not errors and not wrong, (errors, wrong)
     mlp.check()
+
+
+def test_a_training_thread_beside_queries():
+    mlp = sg.Mlp(capacity=1024, lr=0.0)     # steps of size zero: the weights stay, the passes are enqueued
+    mlp.set_params(sg.init_params(3))
+    s = sg.Surrogate(mlp, None)
+    p = sg.draw_parameters(300, 1)
+    want = s.predict(p)
+    g = torch.Generator("cuda").manual_seed(1)
+    x, t = torch.rand((1024, 6), device="cuda", generator=g), torch.rand((1024, 99), device="cuda", generator=g)
+    torch.cuda.synchronize()
+    losses = torch.zeros(200, device="cuda")
+    torch.cuda.synchronize()
+    wrong = []
+
+    def train():
+        for k in range(200):
+            mlp.train_step(x, t, losses.data_ptr() + 4 * k)
+
+    def query():
+        for _ in range(100):
+            if not np.array_equal(s.predict(p), want):
+                wrong.append(1)
+
+    threads = [threading.Thread(target=train), threading.Thread(target=query)]
+    for th in threads:
+        th.start()
+    for th in threads:
+        th.join()
+    torch.cuda.synchronize()
+    mlp.check()
+    assert not wrong and bool((losses == losses[0]).all()) and float(losses[0]) > 0
